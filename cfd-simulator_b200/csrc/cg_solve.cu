@@ -1,18 +1,19 @@
 // cg_solve.cu - the reference's Jacobi-preconditioned conjugate gradient
-// (LinearSystem.cpp:118-210) as a device primitive on one thread-block
-// cluster, for a symmetric five-point system on a structured block given in
-// the reference's LDU layout (LinearSystem.hpp:29-71).
+// (LinearSystem.cpp:118-210) as a device primitive for a symmetric five-point
+// system on a structured block given in the reference's LDU layout
+// (LinearSystem.hpp:29-71): by a wide team of up to 148 CTAs (wide_cg.cuh), or
+// on one thread-block cluster where the block has too few rows to share.
 //
 // The iteration is the reference's, with its L1 stopping rule and its
-// breakdown guards; the dot products are summed in a fixed order (warp
-// trees, then CTA ranks in order), so a solve is deterministic. One cluster
-// barrier per iteration: the single-reduction arrangement described at
-// cgSolveTeam.
+// breakdown guards, arranged with one reduction (described in wide_cg.cuh
+// and at cgSolveTeam); the sums have a fixed order, so a solve is
+// deterministic.
 
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 #include <string>
 
@@ -20,6 +21,8 @@
 #include "common.hpp"
 #include "solver.hpp"
 #include "team.cuh"
+#include "wide_cg.cuh"
+#include "wide_plan.hpp"
 
 namespace cfdb {
 
@@ -182,6 +185,78 @@ __global__ void __launch_bounds__(512, 1) cgSolveKernel(CgView V) {
   t.cl.sync();  // no CTA leaves while a peer may still read its shared memory
 }
 
+// ---- the solve by a wide team ---------------------------------------------------
+
+/// A system in the caller's arrays (reference face order) and a wide team's scratch.
+struct WideCgArgs {
+  int NI, NJ;
+  const double *diag, *upper, *source;
+  const int* across;  // or null
+  double tolerance;
+  int cap;
+  double* x;
+  double* report;  // {iterations, initial, final, converged, bad wake map, fault word}
+  WideScratch mem;
+  double *u, *spill;  // a cell each; what the shared memory does not hold
+  long long spillStride;
+  int smemBytes;
+};
+
+/// The caller's coefficients: boundary faces (other than the wake cut's) are
+/// not part of the system, whatever their entries hold.
+struct ReferenceOrder {
+  const WideCgArgs& A;
+  DEV int wake(int i) const { return (A.across != nullptr && A.across[i] >= 0) ? A.across[i] : -1; }
+  DEV double north(int i, int j) const {
+    if (j == A.NJ || (j == 0 && wake(i) < 0)) return 0.0;
+    return A.upper[j * A.NI + i];
+  }
+  DEV double east(int i, int j) const {
+    return (i > 0 && i < A.NI) ? A.upper[A.NI * (A.NJ + 1) + i * A.NJ + j] : 0.0;
+  }
+  DEV double first(int c, int i, int j) const {
+    const double* x = A.x;
+    double y = A.diag[c] * x[c];
+    if (j > 0) y += north(i, j) * x[c - A.NI];
+    else if (wake(i) >= 0) y += north(i, 0) * x[wake(i)];
+    if (j < A.NJ - 1) y += north(i, j + 1) * x[c + A.NI];
+    if (i > 0) y += east(i, j) * x[c - 1];
+    if (i < A.NI - 1) y += east(i + 1, j) * x[c + 1];
+    return A.source[c] - y;
+  }
+};
+
+__global__ void __launch_bounds__(kWideThreads, 1) wideCgKernel(WideCgArgs A) {
+  __shared__ WideShared sh;
+  int* faultWord = reinterpret_cast<int*>(A.report + 5);
+  const ReferenceOrder load{A};
+  // the wake map: refused when it names no cell of the block
+  bool bad = false, anywhere = false;
+  for (int i = threadIdx.x; i < A.NI; i += blockDim.x) {
+    const int a = load.wake(i);
+    bad |= a >= A.NI * A.NJ;
+    anywhere |= a >= A.NI;
+  }
+  bad = __syncthreads_or(bad);
+  anywhere = __syncthreads_or(anywhere);
+  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+  if (bad) {
+    if (leader) A.report[4] = 1.0;
+    return;
+  }
+  WideTeam t;
+  wideJoin(t, A.mem, faultWord, &sh, blockIdx.x, gridDim.x, A.NI, A.NJ);
+  const WideCgSystem S{A.diag, anywhere, A.x, A.u, A.spill, A.spillStride, A.tolerance, A.cap};
+  const WideCgResult out = wideCg(t, S, load, A.smemBytes);
+  wideLeave(t);
+  if (leader) {
+    A.report[0] = static_cast<double>(out.iterations);
+    A.report[1] = out.initial;
+    A.report[2] = out.final;
+    A.report[3] = out.converged ? 1.0 : 0.0;
+  }
+}
+
 /// Reference-order face coefficients -> device layout; missing wake map -> -1.
 /// A wake-map entry that names no cell of the block (>= cells) would make the
 /// solve read outside x: it is replaced by -1 and flagged in report[4], and the
@@ -228,7 +303,7 @@ Status cgCheck(const cfd_cg_system* s, const double* x, int maxIt, CgView* V) {
 Status cgRun(const cfd_cg_system* s, CgView V, cudaStream_t stream) {
   const int faces = V.NI * (V.NJ + 1) + (V.NI + 1) * V.NJ;
   const int block = 256;
-  cudaError_t e = cudaMemsetAsync(V.report + 4, 0, sizeof(double), stream);
+  cudaError_t e = cudaMemsetAsync(V.report + 4, 0, 2 * sizeof(double), stream);
   if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   cgLayoutKernel<<<(faces + block - 1) / block, block, 0, stream>>>(
       V.NI, V.NJ, s->upper, s->across_j0, const_cast<double*>(V.pN), const_cast<double*>(V.pE),
@@ -261,14 +336,102 @@ Status cgRun(const cfd_cg_system* s, CgView V, cudaStream_t stream) {
   return CFD_OK;
 }
 
+/// Scratch of the calling thread's solves on a device, kept from call to call
+/// up to 64 MB (a larger one is freed when the call ends) and given back when
+/// the thread ends. A call waits for its solve, so the next one may use it.
+struct ThreadScratch {
+  int device{-1};
+  char* base{nullptr};
+  std::size_t bytes{0};
+  static constexpr std::size_t kKept = std::size_t{64} << 20;
+
+  Status take(std::size_t n, char** out) {
+    int current = 0;
+    cudaError_t e = cudaGetDevice(&current);
+    if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+    if (base == nullptr || bytes < n || device != current) {
+      release();
+      e = cudaMalloc(reinterpret_cast<void**>(&base), n);
+      if (e != cudaSuccess) {
+        base = nullptr;
+        return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+      }
+      bytes = n;
+      device = current;
+    }
+    *out = base;
+    return ok();
+  }
+  void done() {
+    if (bytes > kKept) release();
+  }
+  void release() {
+    if (base != nullptr) cudaFree(base);
+    base = nullptr;
+    bytes = 0;
+  }
+  ~ThreadScratch() { release(); }
+};
+
+/// Whether a wide team takes the block: it splits rows over CTAs, so it needs
+/// at least as many rows as the cluster form would use CTAs (a block of a few
+/// very long rows stays with the cluster form, which splits cells). Measured
+/// per iteration: 768x192 on 144 CTAs 3.6 us against 28 on a cluster of 16,
+/// 384x96 2.6 against 8, 192x48 2.2 against 5.5.
+int wideCtasFor(const CgView& V) {
+  const int capacity = wideCapacity();
+  if (capacity < kMaxColumnTiles || V.NJ < chooseClusterSize(V.N)) return 0;
+  return wideChooseCtas(V.NI, V.NJ, capacity);
+}
+WideScratchLayout wideLayoutFor(const CgView& V, int R) {
+  return WideScratchLayout(V.NJ, wideMessages(V.NI, V.NJ, R, kWideThreads));
+}
+
+/// The solve by a wide team of R CTAs (one cooperative launch). `scratch`
+/// holds the messages, which are cleared first.
+Status cgRunWide(const cfd_cg_system* s, const CgView& V, int R, char* messages, double* u, double* spill,
+                 cudaStream_t stream) {
+  const WideScratchLayout layout = wideLayoutFor(V, R);
+  cudaError_t e = cudaMemsetAsync(messages, 0, layout.bytes, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(V.report, 0, 8 * sizeof(double), stream);
+  if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  static PerDeviceOnce configured;
+  if (Status st = configured.run([]() -> Status {
+        const cudaError_t a = cudaFuncSetAttribute(wideCgKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWideSmem);
+        return (a == cudaSuccess) ? ok() : fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(a));
+      });
+      st != CFD_OK) {
+    return st;
+  }
+  const int smem = static_cast<int>(wideCgBytes(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem));
+  const WideCgArgs A{V.NI, V.NJ, s->diag, s->upper, s->source, s->across_j0, V.tol, V.maxIt, V.x, V.report,
+                     layout.at(messages), u, spill, wideCgSpill(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem), smem};
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(R), 1, 1);
+  config.blockDim = dim3(kWideThreads, 1, 1);
+  config.dynamicSmemBytes = static_cast<size_t>(smem);
+  config.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  config.attrs = attr;
+  config.numAttrs = 1;
+  e = cudaLaunchKernelEx(&config, wideCgKernel, A);
+  if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, std::string("CG launch: ") + cudaGetErrorString(e));
+  return CFD_OK;
+}
+
 /// Wait for the solve on `stream`, then copy its report to the host (4
 /// doubles, may be null); a wake map that names a cell outside the block is
 /// an invalid argument (the solve did not run).
 Status cgReport(const CgView& V, cudaStream_t stream, double* report) {
-  double host[5];
+  double host[6];
   cudaError_t e = cudaMemcpyAsync(host, V.report, sizeof(host), cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  int fault = 0;
+  std::memcpy(&fault, host + 5, sizeof(fault));
+  if (fault != 0) return launchFault(fault);
   if (host[4] != 0.0) {
     return fail(CFD_INVALID_ARGUMENT, "across_j0 names a cell outside the block (entries must be < cells_i*cells_j)");
   }
@@ -287,10 +450,31 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
   const std::size_t N = V.N;
   const std::size_t FN = static_cast<std::size_t>(V.NI) * (V.NJ + 1);
   const std::size_t FE = static_cast<std::size_t>(V.NI + 1) * V.NJ;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  V.diag = system->diag;
+  V.b = system->source;
+  V.x = x;
+  V.maxIt = max_iterations;
+  V.tol = tolerance;
+  char* scratch = nullptr;
+  if (const int R = cfdb::wideCtasFor(V); R > 0) {
+    // Scratch for this call: the messages, the report, u, and what the shared
+    // memory does not hold.
+    const cfdb::WideScratchLayout layout = cfdb::wideLayoutFor(V, R);
+    const std::size_t spill = static_cast<std::size_t>(
+        R * cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem));
+    static thread_local cfdb::ThreadScratch kept;
+    if (cfd_status st = kept.take(layout.bytes + (8 + N + spill) * sizeof(double), &scratch); st != CFD_OK) return st;
+    V.report = reinterpret_cast<double*>(scratch + layout.bytes);
+    double* u = V.report + 8;
+    cfd_status st = cfdb::cgRunWide(system, V, R, scratch, u, u + N, s);
+    if (st == CFD_OK) st = cfdb::cgReport(V, s, report);
+    kept.done();
+    return st;
+  }
   // Scratch for this call: both coefficient families, seven CG vectors, the
   // report (8 words) and the wake map.
   const std::size_t doubles = FN + FE + 7 * N + 8;
-  char* scratch = nullptr;
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&scratch), doubles * sizeof(double) + V.NI * sizeof(int));
   if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   double* p = reinterpret_cast<double*>(scratch);
@@ -305,12 +489,6 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
   V.p = p; p += N;
   V.report = p; p += 8;
   V.acrossJ0 = reinterpret_cast<const int*>(p);
-  V.diag = system->diag;
-  V.b = system->source;
-  V.x = x;
-  V.maxIt = max_iterations;
-  V.tol = tolerance;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   cfd_status st = cfdb::cgRun(system, V, s);
   if (st == CFD_OK) st = cfdb::cgReport(V, s, report);
   cudaFree(scratch);
@@ -405,6 +583,27 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
   double* base = nullptr;
   if (cfd_status st = cfdb::noAllocScratch(&base); st != CFD_OK) return st;
   const std::size_t slot = static_cast<std::size_t>(cfdb::kNoAllocMaxNodes);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  V.diag = system->diag;
+  V.b = system->source;
+  V.x = x;
+  V.maxIt = max_iterations;
+  V.tol = tolerance;
+  V.report = base + 9 * slot;
+  // A wide team where everything else stays on chip and its messages fit in
+  // the slots beside u: the array as the cluster form carves it is the limit.
+  if (int R = cfdb::wideCtasFor(V); R > 0) {
+    const std::size_t room = 8 * slot * sizeof(double);
+    while (R > 1 && cfdb::wideLayoutFor(V, R).bytes > room) --R;
+    if (cfdb::wideLayoutFor(V, R).bytes <= room && R >= cfdb::wideCgShape(V.NI, V.NJ, R, cfdb::kWideThreads).columnTiles &&
+        cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem) == 0) {
+      if (cfd_status st = cfdb::cgRunWide(system, V, R, reinterpret_cast<char*>(base), base + 8 * slot, nullptr, s);
+          st != CFD_OK) {
+        return st;
+      }
+      return cfdb::cgReport(V, s, report);
+    }
+  }
   V.pN = base + 0 * slot;
   V.pE = base + 1 * slot;
   V.r = base + 2 * slot;
@@ -414,14 +613,7 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
   V.d1 = base + 6 * slot;
   V.s1 = base + 7 * slot;
   V.p = base + 8 * slot;
-  V.report = base + 9 * slot;
   V.acrossJ0 = reinterpret_cast<const int*>(base + 9 * slot + 8);
-  V.diag = system->diag;
-  V.b = system->source;
-  V.x = x;
-  V.maxIt = max_iterations;
-  V.tol = tolerance;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (cfd_status st = cfdb::cgRun(system, V, s); st != CFD_OK) return st;
   return cfdb::cgReport(V, s, report);
 }

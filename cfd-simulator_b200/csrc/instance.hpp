@@ -19,6 +19,8 @@
 // both rows, which is what its CG inner loop streams.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace cfdb {
@@ -64,12 +66,28 @@ constexpr int kFlagHaloWaitTest = 256;  // tests only: the split CG also waits o
 // Fault codes a launch leaves in iterations[1] (bits, or-ed together).
 constexpr int kFaultChainWait = 1;  // a chained k/omega sweep stage gave up waiting for its neighbour
 constexpr int kFaultHaloWait = 2;   // the pressure CG gave up waiting for a neighbour's halo row
+constexpr int kFaultTeamWait = 4;   // a wide team's barrier or sum gave up waiting for a CTA
 
 // Layout of one monitor record (cfd_monitor), in doubles.
 enum MonitorSlot : int {
   kMonContinuity = 0, kMonMomX, kMonMomY, kMonMassImbalance, kMonMaxDivergence,
   kMonPressureIterations, kMonTurbFirst, kMonTurbSecond, kMonMinK, kMonMaxK, kMonMinW,
   kMonMaxW, kMonMinMut, kMonMaxMut, kMonMaxRatio, kMonMaxYPlus, kMonSlots
+};
+
+// ---- the scratch a wide team of CTAs meets in (wide_team.cuh) --------------------
+
+constexpr int kMaxWideCtas = 160;  // CTAs of one team at most (a B200 has 148 SMs)
+
+/// Zero-filled once; the epoch carries the tags on from launch to launch.
+struct WideScratch {
+  unsigned long long* epoch;
+  unsigned* flags;    // [kMaxWideCtas]
+  double* slots;      // maxima: [2][kMaxWideCtas][8]
+  double* rowSums;    // [2][4][NJ]
+  // the CG's messages, two sets (parity of the exchange) of
+  // wideMessages(...) each
+  ulonglong2* messages;
 };
 
 // ---- mixed form: the pressure-correction multigrid -----------------------------

@@ -43,6 +43,7 @@ Status launchFault(int word) {
   std::string what = "the solver kernel stopped waiting";
   if (word & kFaultChainWait) what += " (a k/omega sweep stage for its neighbour)";
   if (word & kFaultHaloWait) what += " (the pressure CG for a neighbour's halo row)";
+  if (word & kFaultTeamWait) what += " (a CTA for the others of its solve)";
   return fail(CFD_INTERNAL, what + "; the launch's results are not valid");
 }
 

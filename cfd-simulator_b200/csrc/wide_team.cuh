@@ -1,0 +1,318 @@
+// wide_team.cuh - any number of CTAs of one cooperative launch working on one
+// solve: barriers, maxima, row-ordered sums and tagged messages through
+// global memory.
+//
+// Why not a thread-block cluster: a cluster is at most 16 CTAs and must fit
+// in one GPC, so a lone 768x192 solve keeps 132 of the 148 SMs idle and its
+// state (1.2 MB per array) in L2. Spread over ~100 SMs the state of the
+// pressure CG fits on chip, and what a step costs is one exchange through L2
+// (~1.3 us) instead of the streaming of 900 KB per SM.
+//
+// Messages are tagged: every double travels as two 64-bit words, each half of
+// it beside a 32-bit tag, so a reader that sees the tag in both words has the
+// value; no flag, fence or acknowledgement is needed. (Each 64-bit word is a
+// single-copy-atomic access; the two may arrive apart.) Tags come from the
+// team's epoch, which every exchange increments and the solve's scratch keeps
+// between launches, so a stale message never carries the tag waited for.
+//
+// Every CTA of a team must be resident: the launch is cooperative, one CTA
+// per SM. All waits are bounded (kWideSpinLimit polls): one that gives up sets
+// a code in the launch's fault word, after which the CTA waits no more, so a
+// launch always ends and the host reports it.
+//
+// Sums are formed per row of cells (a fixed tree over its columns) and the
+// rows' sums in one fixed order, so their bits do not depend on how many CTAs
+// share the rows.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "instance.hpp"
+#include "team.cuh"
+
+namespace cfdb {
+
+constexpr int kRowBatch = 32;       // rows whose partial sums are held at once
+constexpr int kMaxGroupWarps = 8;   // warps that share a row (256 columns at a time)
+constexpr int kMaxRowSums = 4;
+constexpr int kWideThreads = 512;
+/// Polls before a wait gives up: each is an L2 round trip (~0.7 us), ~3 s in all.
+constexpr int kWideSpinLimit = 1 << 22;
+
+constexpr int kUnitBatch = 8;       // units of the CG whose partial sums are held at once
+constexpr int kUnitWarps = 8;       // warps that share a unit
+constexpr int kSumLine = 8;         // messages from one unit's sums to the next: a 128-byte line
+constexpr int kSumCopies = 4;       // copies of every unit's sums, each polled by its share of the CTAs
+
+struct WideShared {
+  union {
+    double rowPart[kRowBatch][kMaxGroupWarps][kMaxRowSums];
+    double unitPart[kUnitBatch][kUnitWarps][4];
+  };
+  double warpPart[kWideThreads / 32][kRedSlots];
+  double result[kRedSlots];
+  int fault;       // a wait of this CTA gave up
+  unsigned never;  // stays 0: the wait tests' condition
+};
+
+struct WideTeam {
+  int rank, R, tid, T;
+  int NI, NJ;
+  int j0, j1;        // own rows
+  int c0, c1;        // own cells
+  int G, ng;         // threads that share a row, and how many rows at once
+  int g, q;          // this thread's row group and its first column
+  unsigned epoch;
+  WideScratch mem;
+  int* faultWord;
+  WideShared* sh;
+};
+
+/// Threads that share a row: columns in equal passes of at most 256 (and of
+/// at most the block's threads), in whole warps.
+__host__ __device__ inline int wideGroup(int NI, int T) {
+  const int most = (T < 32 * kMaxGroupWarps) ? T : 32 * kMaxGroupWarps;
+  const int passes = (NI + most - 1) / most;
+  const int columns = (NI + passes - 1) / passes;
+  return (columns + 31) / 32 * 32;
+}
+
+DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShared* sh, int rank, int R, int NI,
+                  int NJ) {
+  t.rank = rank;
+  t.R = R;
+  t.tid = static_cast<int>(threadIdx.x);
+  t.T = static_cast<int>(blockDim.x);
+  t.NI = NI;
+  t.NJ = NJ;
+  t.j0 = static_cast<int>((static_cast<long long>(NJ) * rank) / R);
+  t.j1 = static_cast<int>((static_cast<long long>(NJ) * (rank + 1)) / R);
+  t.c0 = t.j0 * NI;
+  t.c1 = t.j1 * NI;
+  t.G = wideGroup(NI, t.T);
+  t.ng = t.T / t.G;
+  t.g = t.tid / t.G;
+  t.q = t.tid - t.g * t.G;
+  t.mem = mem;
+  t.faultWord = faultWord;
+  t.sh = sh;
+  t.epoch = static_cast<unsigned>(*mem.epoch);
+  __syncthreads();
+  if (t.tid == 0) {
+    sh->fault = 0;
+    sh->never = 0u;
+  }
+  __syncthreads();
+}
+
+/// Keep the epoch for the next launch. After a launch that gave up, CTAs can
+/// differ: the largest is kept.
+DEV void wideLeave(WideTeam& t) {
+  if (t.tid == 0) {
+    const unsigned long long was = *t.mem.epoch;
+    const unsigned moved = t.epoch - static_cast<unsigned>(was);
+    if (moved < 0x80000000u) atomicMax(t.mem.epoch, was + moved);
+  }
+}
+
+/// One more unsuccessful poll: true when the wait is over (given up now or before).
+DEV bool wideGiveUp(WideTeam& t, int& polls, int code) {
+  if (*static_cast<volatile int*>(&t.sh->fault) != 0) return true;
+  if (++polls < kWideSpinLimit) return false;
+  t.sh->fault = 1;
+  atomicOr(t.faultWord, code);
+  return true;
+}
+
+// ---- tagged messages ------------------------------------------------------------
+
+DEV void messageStore(ulonglong2* slot, double v, unsigned tag) {
+  const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
+  const unsigned long long t = static_cast<unsigned long long>(tag) << 32;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(slot), "l"(t | (bits & 0xffffffffull)),
+               "l"(t | (bits >> 32))
+               : "memory");
+}
+DEV ulonglong2 messageLoad(const ulonglong2* slot) {
+  ulonglong2 m;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(m.x), "=l"(m.y) : "l"(slot) : "memory");
+  return m;
+}
+DEV bool messageReady(const ulonglong2& m, unsigned tag) {
+  return static_cast<unsigned>(m.x >> 32) == tag && static_cast<unsigned>(m.y >> 32) == tag;
+}
+DEV double messageValue(const ulonglong2& m) {
+  return __longlong_as_double(static_cast<long long>((m.x & 0xffffffffull) | (m.y << 32)));
+}
+/// Wait for the value of `slot` with this tag, given a first look at it.
+DEV double messageWait(WideTeam& t, const ulonglong2* slot, ulonglong2 m, unsigned tag, int code) {
+  int polls = 0;
+  while (!messageReady(m, tag)) {
+    if (wideGiveUp(t, polls, code)) return 0.0;
+    m = messageLoad(slot);
+  }
+  return messageValue(m);
+}
+/// The value of a message; `code` is the fault of a wait that gives up.
+DEV double messageWait(WideTeam& t, const ulonglong2* slot, unsigned tag, int code) {
+  ulonglong2 m = messageLoad(slot);
+  int polls = 0;
+  while (!messageReady(m, tag)) {
+    if (wideGiveUp(t, polls, code)) return 0.0;
+    m = messageLoad(slot);
+  }
+  return messageValue(m);
+}
+/// The values of N messages set[from[k]] (-1: none), waited for together:
+/// every look loads all that are still missing, so the wait ends one L2 round
+/// trip after the last has arrived.
+template <int N>
+DEV void messageWaitAll(WideTeam& t, const ulonglong2* set, const int (&from)[N], unsigned tag, int code,
+                        double (&value)[N]) {
+  unsigned missing = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) missing |= (from[k] >= 0) ? 1u << k : 0u;
+  int polls = 0;
+  while (missing != 0u) {
+    ulonglong2 m[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if (missing & (1u << k)) m[k] = messageLoad(set + from[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if ((missing & (1u << k)) && messageReady(m[k], tag)) {
+        missing &= ~(1u << k);
+        value[k] = messageValue(m[k]);
+      }
+    }
+    if (missing != 0u && wideGiveUp(t, polls, code)) break;
+  }
+}
+
+// ---- barrier ----------------------------------------------------------------------
+
+/// Every CTA's global writes before it are visible to every CTA after it. One
+/// flag per CTA, polled by as many threads; the fences order the block's
+/// writes before its flag and the peers' flags before its reads.
+DEV void wideBarrier(WideTeam& t) {
+  ++t.epoch;
+  __syncthreads();
+  if (t.R == 1) return;
+  if (t.tid == 0) {
+    __threadfence();
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(t.mem.flags + t.rank), "r"(t.epoch) : "memory");
+  }
+  for (int r = t.tid; r < t.R; r += t.T) {
+    int polls = 0;
+    for (;;) {
+      unsigned v;
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.mem.flags + r) : "memory");
+      if (static_cast<int>(v - t.epoch) >= 0) break;
+      if (wideGiveUp(t, polls, kFaultTeamWait)) break;
+    }
+  }
+  if (t.tid < t.R) __threadfence();
+  __syncthreads();
+}
+
+// ---- reductions ---------------------------------------------------------------------
+
+/// Maximum of v[k] over every thread of the team, in every thread. Also a barrier.
+template <int K>
+DEV void wideMax(WideTeam& t, double (&v)[K]) {
+  const int lane = t.tid & 31, warp = t.tid >> 5, warps = t.T >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[k] = smax(v[k], __shfl_down_sync(0xffffffffu, v[k], off));
+    if (lane == 0) t.sh->warpPart[warp][k] = v[k];
+  }
+  __syncthreads();
+  double* slots = t.mem.slots + ((t.epoch + 1u) & 1u) * kMaxWideCtas * kRedSlots;
+  if (t.tid < K) {
+    double a = t.sh->warpPart[0][t.tid];
+    for (int w = 1; w < warps; ++w) a = smax(a, t.sh->warpPart[w][t.tid]);
+    slots[t.rank * kRedSlots + t.tid] = a;
+  }
+  wideBarrier(t);
+  for (int k = warp; k < K; k += warps) {
+    double a = -INFINITY;
+    for (int r = lane; r < t.R; r += 32) a = smax(a, __ldcg(slots + r * kRedSlots + k));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) a = smax(a, __shfl_down_sync(0xffffffffu, a, off));
+    if (lane == 0) t.sh->result[k] = a;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = t.sh->result[k];
+}
+
+/// A row's sums within its warps, into rowPart (slot = the row's place in the batch).
+template <int K>
+DEV void rowPartial(WideTeam& t, int slot, double (&acc)[K]) {
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], off);
+  }
+  if ((t.tid & 31) == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) t.sh->rowPart[slot][t.q >> 5][k] = acc[k];
+  }
+}
+/// The sum of a row over its warps, once they have all been stored.
+DEV double rowTotal(const WideTeam& t, int slot, int k) {
+  const int warps = t.G >> 5;
+  double a[kMaxGroupWarps];
+#pragma unroll
+  for (int w = 0; w < kMaxGroupWarps; ++w) a[w] = (w < warps) ? t.sh->rowPart[slot][w][k] : 0.0;
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
+
+/// The sum of a CG unit over its `warps` warps, once they have all been stored.
+DEV double unitTotal(const WideTeam& t, int slot, int k, int warps) {
+  double a[kUnitWarps];
+#pragma unroll
+  for (int w = 0; w < kUnitWarps; ++w) a[w] = (w < warps) ? t.sh->unitPart[slot][w][k] : 0.0;
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
+
+/// cell(c, i, j, acc) over every own cell, adding to the row's sums; the
+/// team's totals in every thread. Also a barrier.
+template <int K, typename F>
+DEV void wideRowSums(WideTeam& t, double (&out)[K], F&& cell) {
+  const int lane = t.tid & 31, warp = t.tid >> 5, warps = t.T >> 5;
+  const int rows = t.j1 - t.j0;
+  double* sums = t.mem.rowSums + static_cast<std::size_t>((t.epoch + 1u) & 1u) * kMaxRowSums * t.NJ;
+  for (int base = 0; base < rows; base += kRowBatch) {
+    const int n = (rows - base < kRowBatch) ? rows - base : kRowBatch;
+    if (t.g < t.ng) {
+      for (int lr = t.g; lr < n; lr += t.ng) {
+        const int j = t.j0 + base + lr;
+        double acc[K] = {};
+        for (int i = t.q; i < t.NI; i += t.G) cell(j * t.NI + i, i, j, acc);
+        rowPartial(t, lr, acc);
+      }
+    }
+    __syncthreads();
+    for (int m = t.tid; m < n * K; m += t.T) {
+      const int lr = m / K, k = m - lr * K;
+      sums[k * t.NJ + t.j0 + base + lr] = rowTotal(t, lr, k);
+    }
+    if (base + kRowBatch < rows) __syncthreads();
+  }
+  wideBarrier(t);
+  for (int k = warp; k < K; k += warps) {
+    double a = 0.0;
+    for (int j = lane; j < t.NJ; j += 32) a += __ldcg(sums + k * t.NJ + j);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
+    if (lane == 0) t.sh->result[k] = a;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = t.sh->result[k];
+}
+
+}  // namespace cfdb

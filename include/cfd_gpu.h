@@ -264,8 +264,8 @@ typedef struct cfd_cg_system {
  * the device: x (device, cells) is the starting guess in and the solution
  * out; report (host, 4 doubles, may be NULL) = {iterations, initial residual,
  * final residual, converged}; both residuals are L1 norms as in the
- * reference. Allocates its scratch (two coefficient arrays, seven vectors) for
- * the call. stream: a cudaStream_t, or NULL for the legacy default stream.
+ * reference. Its scratch is allocated on the calling thread's first use and
+ * kept for that thread's later calls up to 64 MB. stream: a cudaStream_t, or NULL for the legacy default stream.
  * Returns after the solve has finished. A wake-map entry >= cells_i*cells_j
  * is refused with CFD_INVALID_ARGUMENT, and x is then left unchanged. */
 cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance,
