@@ -245,9 +245,9 @@ __global__ void __launch_bounds__(kWideThreads, 1) wideCgKernel(WideCgArgs A) {
     return;
   }
   WideTeam t;
-  wideJoin(t, A.mem, faultWord, &sh, blockIdx.x, gridDim.x, A.NI, A.NJ);
+  wideJoin(t, A.mem, faultWord, &sh, blockIdx.x, gridDim.x, A.NI, A.NJ, 0);
   const WideCgSystem S{A.diag, anywhere, A.x, A.u, A.spill, A.spillStride, A.tolerance, A.cap};
-  const WideCgResult out = wideCg(t, S, load, A.smemBytes);
+  const WideCgResult out = wideCg(t, S, load, A.smemBytes, false);
   wideLeave(t);
   if (leader) {
     A.report[0] = static_cast<double>(out.iterations);
@@ -384,7 +384,7 @@ int wideCtasFor(const CgView& V) {
   return wideChooseCtas(V.NI, V.NJ, capacity);
 }
 WideScratchLayout wideLayoutFor(const CgView& V, int R) {
-  return WideScratchLayout(V.NJ, wideMessages(V.NI, V.NJ, R, kWideThreads));
+  return WideScratchLayout(V.NI, V.NJ, wideMessages(V.NI, V.NJ, R, kWideThreads));
 }
 
 /// The solve by a wide team of R CTAs (one cooperative launch). `scratch`
@@ -403,9 +403,9 @@ Status cgRunWide(const cfd_cg_system* s, const CgView& V, int R, char* messages,
       st != CFD_OK) {
     return st;
   }
-  const int smem = static_cast<int>(wideCgBytes(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem));
+  const int smem = static_cast<int>(wideCgBytes(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem, true));
   const WideCgArgs A{V.NI, V.NJ, s->diag, s->upper, s->source, s->across_j0, V.tol, V.maxIt, V.x, V.report,
-                     layout.at(messages), u, spill, wideCgSpill(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem), smem};
+                     layout.at(messages), u, spill, wideCgSpill(V.NI, V.NJ, R, kWideThreads, kMaxWideSmem, true), smem};
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(R), 1, 1);
   config.blockDim = dim3(kWideThreads, 1, 1);
@@ -462,7 +462,7 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
     // memory does not hold.
     const cfdb::WideScratchLayout layout = cfdb::wideLayoutFor(V, R);
     const std::size_t spill = static_cast<std::size_t>(
-        R * cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem));
+        R * cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem, true));
     static thread_local cfdb::ThreadScratch kept;
     if (cfd_status st = kept.take(layout.bytes + (8 + N + spill) * sizeof(double), &scratch); st != CFD_OK) return st;
     V.report = reinterpret_cast<double*>(scratch + layout.bytes);
@@ -596,7 +596,7 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
     const std::size_t room = 8 * slot * sizeof(double);
     while (R > 1 && cfdb::wideLayoutFor(V, R).bytes > room) --R;
     if (cfdb::wideLayoutFor(V, R).bytes <= room && R >= cfdb::wideCgShape(V.NI, V.NJ, R, cfdb::kWideThreads).columnTiles &&
-        cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem) == 0) {
+        cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem, true) == 0) {
       if (cfd_status st = cfdb::cgRunWide(system, V, R, reinterpret_cast<char*>(base), base + 8 * slot, nullptr, s);
           st != CFD_OK) {
         return st;

@@ -214,6 +214,8 @@ struct Engine {
   int statusSlots{0};
   Instance* dTable{nullptr};
   int tableSlots{0};
+  char* dPlans{nullptr};  // the wide launches' plans
+  std::size_t planBytes{0};
   std::vector<cudaStream_t> streams;
 
   double now() const {
@@ -225,6 +227,7 @@ struct Engine {
     active.clear();
     if (dStatus) cudaFree(dStatus);
     if (dTable) cudaFree(dTable);
+    if (dPlans) cudaFree(dPlans);
     for (cudaStream_t s : streams) cudaStreamDestroy(s);
   }
 
@@ -298,16 +301,21 @@ struct Engine {
   /// the same bits, whatever else is in the engine. CFD_ENGINE_TUNE=0 keeps the solver's
   /// default shape.
   Status tunedShape(const Pending& q, const Solver& s, std::pair<int, int>* out) {
-    if (!tuned) {
-      // By grid size as a lone solve runs, except that the mixed form takes
-      // clusters of at most 8 CTAs: its cost per iteration falls less than
-      // in proportion to the CTAs (the multigrid's coarse levels and its
-      // barriers do not shrink), so smaller clusters fit more solves per GPU
-      // (a 24-solve polar: 35 s on 8-CTA clusters, 37 s on 16, 43 s on 12),
-      // while the plain form needs 16 for its on-chip CG band (104 s on 16,
-      // 136 s on 12, 146 s on 8).
+    if (!tuned || s.precision() == 0) {
+      // The plain form's launches share the GPU by a plan of their own
+      // (planWide), and its bits do not depend on it. The mixed form runs by
+      // grid size as a lone solve does, except that it takes clusters of at
+      // most 8 CTAs: its cost per iteration falls less than in proportion to
+      // the CTAs (the multigrid's coarse levels and its barriers do not
+      // shrink), so smaller clusters fit more solves per GPU (a 24-solve
+      // polar: 35 s on 8-CTA clusters, 37 s on 16, 43 s on 12).
       int R = s.clusterSize();
       if (s.precision() == 1) R = std::min(R, 8);
+      // A tuned engine reports one of the shapes that it times: for the plain
+      // form, whose launches none of them touch, the largest with a row per CTA.
+      if (tuned) {
+        for (R = 16; R > 4 && R > s.cellsJ();) R /= 2;
+      }
       *out = {R, s.threads()};
       return ok();
     }
@@ -325,7 +333,7 @@ struct Engine {
       int most = 0;
       for (int R : {4, 8, 16}) {
         if (R > s.cellsJ()) continue;
-        const int resident = maxActiveClusters(R, T, s.launchSmemBytes(R));
+        const int resident = maxActiveClusters(R, T, s.launchSmemBytes());
         if (resident <= 0) continue;
         candidates.emplace_back(R, resident);
         most = std::max(most, resident);
@@ -350,7 +358,7 @@ struct Engine {
             cudaSuccess) {
           for (const auto& [R, resident] : candidates) {
             const int n = std::min<int>(resident, static_cast<int>(probes.size()));
-            const int smem = probes[0]->launchSmemBytes(R);
+            const int smem = probes[0]->launchSmemBytes();
             if (launchSimple(table, n, R, T, 2, kStageEnd, -1.0, nullptr, smem) != CFD_OK) continue;
             if (cudaDeviceSynchronize() != cudaSuccess) break;
             const auto t0 = std::chrono::steady_clock::now();
@@ -552,14 +560,21 @@ struct Engine {
   Status launchChunk() {
     const int n = static_cast<int>(active.size());
     if (Status st = reserve(n); st != CFD_OK) return st;
-    // group by launch shape; table rows in slot order within each group
+    // group by launch shape (the plain form's solves in one launch per thread
+    // count, cluster size 0 here); table rows in slot order within each group
+    struct Launch {
+      int offset, count, R, T, smem;
+      WidePlan plan;
+      std::size_t planAt;  // its CTAs, then its list, in the plan area (bytes)
+    };
     std::map<std::pair<int, int>, std::vector<int>> groups;
     for (int k = 0; k < n; ++k) {
       const Solver& s = *active[k]->solver;
-      groups[{s.clusterSize(), s.threads()}].push_back(k);
+      groups[{(s.precision() == 0) ? 0 : s.clusterSize(), s.threads()}].push_back(k);
     }
     std::vector<Instance> table(n);
-    std::vector<std::tuple<int, int, int, int, int>> launches;  // offset, count, R, T, smem
+    std::vector<Launch> launches;
+    std::vector<char> plans;
     const std::size_t per = static_cast<std::size_t>(chunk) * kMonSlots + 1;
     int offset = 0;
     for (const auto& [shape, members] : groups) {
@@ -574,13 +589,36 @@ struct Engine {
         I.stopTol = s.request.tolerance;
         I.iterLimit = std::max(1, std::min(chunk, s.request.max_iterations - s.iterations));
         table[offset + static_cast<int>(m)] = I;
-        smem = std::max(smem, s.solver->launchSmemBytes(shape.first));
+        if (shape.first > 0) smem = std::max(smem, s.solver->launchSmemBytes());
       }
-      launches.emplace_back(offset, static_cast<int>(members.size()), shape.first, shape.second, smem);
+      Launch launch{offset, static_cast<int>(members.size()), shape.first, shape.second, smem, {}, plans.size()};
+      if (shape.first == 0) {
+        std::vector<WideJob> jobs;
+        for (int k : members) jobs.push_back(active[k]->solver->wideJob());
+        launch.plan = planWide(jobs, shape.second);
+        const std::size_t ctas = launch.plan.ctas.size() * sizeof(WideCta);
+        const std::size_t list = launch.plan.list.size() * sizeof(int);
+        plans.resize(plans.size() + ((ctas + list + 15) & ~std::size_t{15}));
+        std::memcpy(plans.data() + launch.planAt, launch.plan.ctas.data(), ctas);
+        std::memcpy(plans.data() + launch.planAt + ctas, launch.plan.list.data(), list);
+      }
+      launches.push_back(std::move(launch));
       offset += static_cast<int>(members.size());
     }
     if (cudaMemcpy(dTable, table.data(), n * sizeof(Instance), cudaMemcpyHostToDevice) != cudaSuccess) {
       return fail(CFD_INITIALIZATION_FAILURE, "engine table upload failed");
+    }
+    if (plans.size() > planBytes) {
+      if (dPlans) cudaFree(dPlans);
+      planBytes = 2 * plans.size();
+      if (cudaMalloc(reinterpret_cast<void**>(&dPlans), planBytes) != cudaSuccess) {
+        dPlans = nullptr;
+        planBytes = 0;
+        return fail(CFD_INITIALIZATION_FAILURE, "engine plan allocation failed");
+      }
+    }
+    if (!plans.empty() && cudaMemcpy(dPlans, plans.data(), plans.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      return fail(CFD_INITIALIZATION_FAILURE, "engine plan upload failed");
     }
     while (streams.size() < launches.size()) {
       cudaStream_t s;
@@ -591,9 +629,13 @@ struct Engine {
     }
     inFlightStreams.clear();
     for (std::size_t g = 0; g < launches.size(); ++g) {
-      const auto [off, count, R, T, smem] = launches[g];
-      if (Status st = launchSimple(dTable + off, count, R, T, chunk, kStageEnd, -1.0, streams[g], smem);
-          st != CFD_OK) {
+      const Launch& l = launches[g];
+      const WideCta* ctas = (l.R == 0) ? reinterpret_cast<const WideCta*>(dPlans + l.planAt) : nullptr;
+      const Status st =
+          (l.R == 0) ? launchPlain(dTable + l.offset, l.plan, ctas, reinterpret_cast<const int*>(ctas + l.plan.ctas.size()),
+                                   l.T, chunk, kStageEnd, -1.0, streams[g])
+                     : launchSimple(dTable + l.offset, l.count, l.R, l.T, chunk, kStageEnd, -1.0, streams[g], l.smem);
+      if (st != CFD_OK) {
         waitForLaunches();
         return st;
       }

@@ -52,16 +52,14 @@ enum Stage : int {
   kStageEnd
 };
 
-// Kernel implementation flags (bit mask).
-constexpr int kFlagGlobalCg = 1;    // the default now; kept so the flag value stays accepted
+// Kernel implementation flags (bit mask; kernelFlags()).
 constexpr int kFlagPlainWavefront = 2;
 constexpr int kFlagSequentialRows = 4;
 constexpr int kFlagTwoReductionCg = 8;
-constexpr int kFlagOnePassCg = 16;
 constexpr int kFlagBarrierSweeps = 32;
-constexpr int kFlagSharedCg = 128;  // the pressure CG's band in shared memory where it fits
-constexpr int kFlagChainWaitTest = 64;  // tests only: a chained stage also waits for a count nothing sets
-constexpr int kFlagHaloWaitTest = 256;  // tests only: the split CG also waits once for a count nothing sets
+constexpr int kFlagChainWaitTest = 64;  // tests only: a sweep also waits for a count nothing sets
+constexpr int kFlagSharedCg = 128;      // the plain CG in its form for any shape
+constexpr int kFlagHaloWaitTest = 256;  // tests only: a wait before the CG for a count nothing sets
 
 // Fault codes a launch leaves in iterations[1] (bits, or-ed together).
 constexpr int kFaultChainWait = 1;  // a chained k/omega sweep stage gave up waiting for its neighbour
@@ -84,10 +82,16 @@ struct WideScratch {
   unsigned long long* epoch;
   unsigned* flags;    // [kMaxWideCtas]
   double* slots;      // maxima: [2][kMaxWideCtas][8]
-  double* rowSums;    // [2][4][NJ]
+  double* chunkSums;  // [2][4][chunks of 256 cells]
   // the CG's messages, two sets (parity of the exchange) of
   // wideMessages(...) each
   ulonglong2* messages;
+};
+
+/// One CTA of a wide launch: the solves it works on (entries begin .. end of the
+/// launch's list), and its place in their teams of R.
+struct WideCta {
+  int begin, end, rank, R;
 };
 
 // ---- mixed form: the pressure-correction multigrid -----------------------------
@@ -159,16 +163,22 @@ struct Instance {
   double *gux, *guy, *gvx, *gvy, *gpx, *gpy;
   // momentum system (shared by u and v), relaxed; aD doubles as momentumDiagonal
   double *aD, *aS, *aN, *aW, *aE, *bU, *bV;
-  // pressure correction; the single-reduction CG double-buffers r in (r, z),
-  // w = A u in (q, d0) and s = A p in (d1, s1), with the direction in cgp
+  // pressure correction; r, z, q, d0, d1 are the two-reduction CG's vectors
   double *pD, *pN, *pE, *pB, *net;
-  double *x, *r, *z, *q, *d0, *d1, *s1, *cgp;
+  double *x, *r, *z, *q, *d0, *d1;
   double* div;
 
   // ---- SST ----
   double *k, *om, *mut, *strain, *f1, *f2, *cd, *prod, *gkx, *gky, *gwx, *gwy;
   double *kD, *kS, *kN, *kW, *kE, *kB;
   double *wD, *wS, *wN, *wW, *wE, *wB;
+
+  // ---- plain form: a wide team's scratch and the k and omega sweeps' layouts ----
+  WideScratch wide;
+  double *kC, *wC;           // packed sweep coefficients (row_sweeps.cuh)
+  ulonglong2 *kV, *wV;       // packed sweep values, as messages
+  double* spill;             // what the CG cannot hold on chip, by CTA
+  int wideMost;              // CTAs at most: one per CG unit, or the CTAs asked for
 
   // ---- outputs ----
   double* history;   // kMonSlots doubles per iteration of the launch

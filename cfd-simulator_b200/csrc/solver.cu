@@ -9,9 +9,13 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <map>
 #include <string>
 
 #include "cfd_gpu.h"
+#include "row_sweeps.cuh"
+#include "wide_cg.cuh"
+#include "wide_plan.hpp"
 
 namespace cfdb {
 
@@ -299,6 +303,23 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
   if (m.nodes != nullptr) nodes_.assign(m.nodes, m.nodes + 2 * static_cast<std::size_t>(ni) * nj);
   const std::size_t S = static_cast<std::size_t>(std::max(wall_.count(), 1));
 
+  // Launch shape: CTAs per solve (the mixed form's cluster, and with
+  // CFD_CLUSTER_SIZE, 1 to 16, the most the plain form's team takes) and threads
+  // per CTA (CFD_THREADS, a multiple of 32, at most 512).
+  clusterSize_ = chooseClusterSize(N_);
+  if (const char* env = std::getenv("CFD_THREADS")) {
+    const int t = std::atoi(env);
+    if (t >= 32 && t <= 512 && t % 32 == 0) threads_ = t;
+  }
+  view_.wideMost = wideMostCtas(NI_, NJ_, threads_);
+  if (const char* env = std::getenv("CFD_CLUSTER_SIZE")) {
+    const int r = std::atoi(env);
+    if (r >= 1 && r <= 16) {
+      clusterSize_ = r;
+      view_.wideMost = std::min(view_.wideMost, std::max(r, wideLeastCtas(NI_, threads_)));
+    }
+  }
+
   // ---- device layout ----
   const std::size_t FN = static_cast<std::size_t>(NI_) * (NJ_ + 1);
   const std::size_t FE = static_cast<std::size_t>(NI_ + 1) * NJ_;
@@ -322,11 +343,27 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
     I.wallMask = a.take<uint8_t>(N);
     double** cellArrays[] = {&I.u, &I.v, &I.p, &I.rho, &I.mu, &I.muMol, &I.gux, &I.guy, &I.gvx,
                              &I.gvy, &I.gpx, &I.gpy, &I.aD, &I.aS, &I.aN, &I.aW, &I.aE, &I.bU,
-                             &I.bV, &I.pD, &I.pB, &I.net, &I.x, &I.r, &I.z, &I.q, &I.d0, &I.d1, &I.s1, &I.cgp,
-                             &I.div, &I.k, &I.om, &I.mut, &I.strain, &I.f1, &I.f2, &I.cd, &I.prod,
-                             &I.gkx, &I.gky, &I.gwx, &I.gwy, &I.kD, &I.kS, &I.kN, &I.kW, &I.kE,
-                             &I.kB, &I.wD, &I.wS, &I.wN, &I.wW, &I.wE, &I.wB};
+                             &I.bV, &I.pD, &I.pB, &I.net, &I.x, &I.r, &I.div, &I.k, &I.om, &I.mut, &I.strain,
+                             &I.f1, &I.f2, &I.cd, &I.prod, &I.gkx, &I.gky, &I.gwx, &I.gwy, &I.kD, &I.kB, &I.wD,
+                             &I.wB};
     for (double** ptr : cellArrays) *ptr = a.take<double>(N);
+    if (settings_.precision == 1) {
+      double** rows[] = {&I.kS, &I.kN, &I.kW, &I.kE, &I.wS, &I.wN, &I.wW, &I.wE};
+      for (double** ptr : rows) *ptr = a.take<double>(N);
+    } else {
+      double** vectors[] = {&I.z, &I.q, &I.d0, &I.d1};
+      for (double** ptr : vectors) *ptr = a.take<double>(N);
+      const std::size_t packed = static_cast<std::size_t>(rowSweepCoefficients(NI_, NJ_));
+      const std::size_t values = static_cast<std::size_t>(rowSweepMessages(NI_, NJ_));
+      I.kC = a.take<double>(packed); I.wC = a.take<double>(packed);
+      I.kV = a.take<ulonglong2>(values); I.wV = a.take<ulonglong2>(values);
+      const std::size_t spill =
+          static_cast<std::size_t>(wideSpillDoubles(NI_, NJ_, I.wideMost, threads_));
+      I.spill = a.take<double>(std::max<std::size_t>(spill, 1));
+      const WideScratchLayout layout(NI_, NJ_, wideMessages(NI_, NJ_, I.wideMost, threads_));
+      char* scratch = a.take<char>(layout.bytes);
+      if (scratch != nullptr) I.wide = layout.at(scratch);
+    }
     I.mfN = a.take<double>(FN); I.mfE = a.take<double>(FE);
     I.pN = a.take<double>(FN); I.pE = a.take<double>(FE);
     I.history = a.take<double>(static_cast<std::size_t>(historyCapacity_) * kMonSlots);
@@ -477,26 +514,16 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
   wallDist_.resize(N);
   CUDA_OR_FAIL(cudaMemcpy(wallDist_.data(), I.wallDist, N * sizeof(double), cudaMemcpyDeviceToHost));
 
-  clusterSize_ = chooseClusterSize(N_);
-  // Launch-shape overrides for tuning sweeps: CTAs per solve (1..16) and
-  // threads per CTA (a multiple of 32, at most 512).
-  if (const char* env = std::getenv("CFD_CLUSTER_SIZE")) {
-    const int r = std::atoi(env);
-    if (r >= 1 && r <= 16) clusterSize_ = r;
-  }
-  if (const char* env = std::getenv("CFD_THREADS")) {
-    const int t = std::atoi(env);
-    if (t >= 32 && t <= 512 && t % 32 == 0) threads_ = t;
-  }
   return uploadSettings();
 }
 
 std::size_t Solver::estimateBytes(int NI, int NJ) {
-  // cell arrays (~60), face arrays of both families (~26), per-face geometry
-  // and conditions; rounded up generously.
+  // cell arrays, face arrays of both families, per-face geometry and
+  // conditions, the sweeps' packed rows and values, messages and spill;
+  // rounded up generously
   const std::size_t N = static_cast<std::size_t>(NI) * NJ;
   const std::size_t F = static_cast<std::size_t>(NI) * (NJ + 1) + static_cast<std::size_t>(NI + 1) * NJ;
-  return (64 * N + 16 * F) * 8 + (1u << 20);
+  return (100 * N + 16 * F) * 8 + (1u << 20);
 }
 
 void Solver::planMultigrid(const std::vector<int>& wake0) {
@@ -551,12 +578,9 @@ Status Solver::setLaunchShape(int clusterSize, int threads) {
   return CFD_OK;
 }
 
-int Solver::launchSmemBytes(int clusterSize) const {
-  if (settings_.precision == 1) {
-    const int scan = chainSweepBytes(NI_, 4);  // the chained k/omega row sweeps, FP32
-    return std::max(mgSmemBytes_, (scan <= kMaxCgSharedBytes) ? scan : 0);
-  }
-  return cgSharedBytes(NI_, NJ_, clusterSize);
+int Solver::launchSmemBytes() const {
+  const int scan = chainSweepBytes(NI_, 4);  // the chained k/omega row sweeps, FP32
+  return std::max(mgSmemBytes_, (scan <= kMaxClusterSmem) ? scan : 0);
 }
 
 Solver::~Solver() {
@@ -809,11 +833,12 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
   int total = 0;
   while (total < n) {
     const int chunk = std::min(n - total, historyCapacity_);
-    if (Status st = launchSimple(dView_, 1, clusterSize_, threads_, chunk, stopStage, tolerance, stream_,
-                                 launchSmemBytes(clusterSize_));
-        st != CFD_OK) {
-      return st;
-    }
+    const Status st =
+        (settings_.precision == 1)
+            ? launchSimple(dView_, 1, clusterSize_, threads_, chunk, stopStage, tolerance, stream_, launchSmemBytes())
+            : launchPlain(dView_, planWide({wideJob()}, threads_), nullptr, nullptr, threads_, chunk, stopStage,
+                          tolerance, stream_);
+    if (st != CFD_OK) return st;
     CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
     int words[2] = {0, 0};
     CUDA_OR_FAIL(cudaMemcpy(words, dIterations_, sizeof(words), cudaMemcpyDeviceToHost));
@@ -1322,12 +1347,18 @@ cfd_status cfd_gpu_destroy(cfd_handle h) {
 
 // ---- batches ------------------------------------------------------------------------------
 
-/// The solves of a batch that share a launch shape: one launch over a
-/// contiguous part of the descriptor table, on a stream of its own.
+/// The solves of a batch that share a launch: the plain form's together, as a
+/// wide plan shares the GPU between them; the mixed form's by cluster size.
+/// One launch over a contiguous part of the descriptor table, on a stream of
+/// its own.
 struct BatchGroup {
+  bool wide{false};
   int offset{0}, count{0};
   int clusterSize{1}, threads{512}, smemBytes{0};
   std::vector<int> members;  // indices into cfd_batch_t::handles
+  cfdb::WidePlan plan;
+  cfdb::WideCta* dPlan{nullptr};
+  int* dList{nullptr};
   cudaStream_t stream{nullptr};
   cudaEvent_t done{nullptr};
 };
@@ -1338,7 +1369,7 @@ struct cfd_batch_t {
   cudaStream_t stream{nullptr};
   cudaEvent_t fork{nullptr};
   std::vector<BatchGroup> groups;  // widest clusters first
-  int clusterSize{1};              // the shape of the largest group (cfd_batch_shape)
+  int clusterSize{1};              // the most frequent shape (cfd_batch_shape)
   int threads{512};
   int lastIterations{0};
   cudaGraphExec_t graph{nullptr};  // the n-iteration launch, captured once
@@ -1354,23 +1385,45 @@ cfd_status refreshTable(cfd_batch b) {
   }
   cudaError_t e = cudaMemcpyAsync(b->dTable, table.data(), table.size() * sizeof(cfdb::Instance),
                                   cudaMemcpyHostToDevice, b->stream);
+  // the wide groups' plans (a solve's model can change between launches)
+  for (BatchGroup& g : b->groups) {
+    if (!g.wide) continue;
+    std::vector<cfdb::WideJob> jobs;
+    for (int k : g.members) jobs.push_back(b->handles[static_cast<std::size_t>(k)]->solver->wideJob());
+    g.plan = cfdb::planWide(jobs, g.threads);
+    if (e == cudaSuccess && g.dPlan == nullptr) {
+      e = cudaMalloc(reinterpret_cast<void**>(&g.dPlan), cfdb::kMaxWideCtas * sizeof(cfdb::WideCta));
+    }
+    if (e == cudaSuccess && g.dList == nullptr) {
+      e = cudaMalloc(reinterpret_cast<void**>(&g.dList), g.members.size() * sizeof(int));
+    }
+    if (e == cudaSuccess) {
+      e = cudaMemcpyAsync(g.dPlan, g.plan.ctas.data(), g.plan.ctas.size() * sizeof(cfdb::WideCta),
+                          cudaMemcpyHostToDevice, b->stream);
+    }
+    if (e == cudaSuccess) {
+      e = cudaMemcpyAsync(g.dList, g.plan.list.data(), g.plan.list.size() * sizeof(int), cudaMemcpyHostToDevice,
+                          b->stream);
+    }
+  }
   if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   return CFD_OK;
 }
 
+cfd_status launchGroup(cfd_batch b, const BatchGroup& g, int n, int stopStage, double tolerance, cudaStream_t s) {
+  const cfdb::Instance* table = b->dTable + g.offset;
+  if (g.wide) return cfdb::launchPlain(table, g.plan, g.dPlan, g.dList, g.threads, n, stopStage, tolerance, s);
+  return cfdb::launchSimple(table, g.count, g.clusterSize, g.threads, n, stopStage, tolerance, s, g.smemBytes);
+}
+
 /// n iterations of every solve of the batch, ordered on `s`: one launch per
 /// group, the groups forked from `s` onto their own streams and joined back,
-/// so solves of different launch shapes run side by side (a group of small
-/// clusters fills the SMs a group of wide ones leaves idle). Used directly
-/// and under stream capture.
+/// so launches of different shapes run side by side where they fit. Used
+/// directly and under stream capture.
 cfd_status launchGroups(cfd_batch b, int n, int stopStage, double tolerance, cudaStream_t s) {
-  if (b->groups.size() == 1) {
-    const BatchGroup& g = b->groups[0];
-    return cfdb::launchSimple(b->dTable + g.offset, g.count, g.clusterSize, g.threads, n, stopStage, tolerance, s,
-                              g.smemBytes);
-  }
+  if (b->groups.size() == 1) return launchGroup(b, b->groups[0], n, stopStage, tolerance, s);
   cudaError_t e = cudaEventRecord(b->fork, s);
   if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   cfd_status st = CFD_OK;
@@ -1378,8 +1431,7 @@ cfd_status launchGroups(cfd_batch b, int n, int stopStage, double tolerance, cud
     e = cudaStreamWaitEvent(g.stream, b->fork, 0);
     if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
     if (st == CFD_OK) {
-      st = cfdb::launchSimple(b->dTable + g.offset, g.count, g.clusterSize, g.threads, n, stopStage, tolerance,
-                              g.stream, g.smemBytes);
+      st = launchGroup(b, g, n, stopStage, tolerance, g.stream);
     }
     e = cudaEventRecord(g.done, g.stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, g.done, 0);
@@ -1403,35 +1455,40 @@ cfd_status cfd_batch_create(const cfd_handle* solvers, int count, cfd_batch* out
     }
     b->handles.push_back(solvers[k]);
   }
-  // One group per launch shape (each solve keeps its own), widest first so
-  // its clusters are placed before the narrower groups fill the gaps.
+  // The plain form's solves in one group per thread count, the mixed form's in
+  // one per launch shape, widest first so its clusters are placed before the
+  // narrower groups fill the gaps.
+  std::map<std::pair<int, int>, int> shapes;  // (CTAs, threads) -> solves
   for (int k = 0; k < count; ++k) {
     const cfdb::Solver& sv = *b->handles[static_cast<std::size_t>(k)]->solver;
+    const bool wide = sv.precision() == 0;
+    shapes[{sv.clusterSize(), sv.threads()}] += 1;
     auto it = std::find_if(b->groups.begin(), b->groups.end(), [&](const BatchGroup& g) {
-      return g.clusterSize == sv.clusterSize() && g.threads == sv.threads();
+      return g.wide == wide && (wide || g.clusterSize == sv.clusterSize()) && g.threads == sv.threads();
     });
     if (it == b->groups.end()) {
       BatchGroup g;
-      g.clusterSize = sv.clusterSize();
+      g.wide = wide;
+      g.clusterSize = wide ? 1 << 16 : sv.clusterSize();
       g.threads = sv.threads();
       b->groups.push_back(g);
       it = b->groups.end() - 1;
     }
     it->members.push_back(k);
-    it->smemBytes = std::max(it->smemBytes, sv.launchSmemBytes(sv.clusterSize()));
+    if (!wide) it->smemBytes = std::max(it->smemBytes, sv.launchSmemBytes());
   }
   std::stable_sort(b->groups.begin(), b->groups.end(),
                    [](const BatchGroup& a, const BatchGroup& c) { return a.clusterSize > c.clusterSize; });
   int offset = 0;
-  std::size_t largest = 0;
-  for (std::size_t g = 0; g < b->groups.size(); ++g) {
-    b->groups[g].offset = offset;
-    b->groups[g].count = static_cast<int>(b->groups[g].members.size());
-    offset += b->groups[g].count;
-    if (b->groups[g].count > b->groups[largest].count) largest = g;
+  for (BatchGroup& g : b->groups) {
+    g.offset = offset;
+    g.count = static_cast<int>(g.members.size());
+    offset += g.count;
   }
-  b->clusterSize = b->groups[largest].clusterSize;
-  b->threads = b->groups[largest].threads;
+  const auto frequent = std::max_element(shapes.begin(), shapes.end(),
+                                         [](const auto& x, const auto& y) { return x.second < y.second; });
+  b->clusterSize = frequent->first.first;
+  b->threads = frequent->first.second;
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&b->dTable), count * sizeof(cfdb::Instance));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
@@ -1470,6 +1527,7 @@ cfd_status cfd_batch_graph_launch(cfd_batch b, int n, void* stream) {
       b->graph = nullptr;
     }
     if (cfd_status st = cfdb::prepareSimpleKernel(); st != CFD_OK) return st;
+    if (cfd_status st = cfdb::preparePlainKernel(); st != CFD_OK) return st;
     cudaError_t e = cudaStreamSynchronize(b->stream);
     if (e == cudaSuccess) e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
@@ -1561,6 +1619,8 @@ cfd_status cfd_batch_destroy(cfd_batch b) {
       cudaStreamDestroy(g.stream);
     }
     if (g.done != nullptr) cudaEventDestroy(g.done);
+    if (g.dPlan != nullptr) cudaFree(g.dPlan);
+    if (g.dList != nullptr) cudaFree(g.dList);
   }
   if (b->graph != nullptr) cudaGraphExecDestroy(b->graph);
   if (b->dTable != nullptr) cudaFree(b->dTable);

@@ -18,6 +18,7 @@
 #include "forces.hpp"
 #include "instance.hpp"
 #include "streamlines.hpp"
+#include "wide_plan.hpp"
 
 namespace cfdb {
 
@@ -132,9 +133,10 @@ class Solver {
   /// Rough device footprint of a solve of NI x NJ cells (the arena's layout).
   static std::size_t estimateBytes(int NI, int NJ);
   const Instance& deviceView() const { return view_; }
-  /// Dynamic shared memory a launch of this solve needs on a cluster of
-  /// `clusterSize` CTAs.
-  int launchSmemBytes(int clusterSize) const;
+  /// Dynamic shared memory a launch of this solve needs on a cluster (mixed form).
+  int launchSmemBytes() const;
+  /// This solve for the planner of wide launches (plain form).
+  WideJob wideJob() const { return WideJob{NI_, NJ_, view_.wideMost, model_ == 2}; }
   int precision() const { return settings_.precision; }
   int wallStations() const { return wall_.count(); }
   /// CTAs per cluster (1..16) and threads per CTA (multiple of 32, <= 512).
@@ -208,11 +210,11 @@ class Solver {
 /// shared memory (eight FP32 arrays per cell: ~130 KB for all of them).
 constexpr int kMgSharedCells = 3072;
 
-/// Launch the SIMPLE kernel over `count` instances (device array), one
-/// cluster of `clusterSize` CTAs each.
 Status launchWallDistance(int n, const double* centroid, int walls, const double* wallCentre,
                           double far, double* out, cudaStream_t stream);
 
+/// Launch the mixed form's kernel over `count` instances (device array), one
+/// cluster of `clusterSize` CTAs each.
 Status launchSimple(const Instance* dInstances, int count, int clusterSize, int threads,
                     int iterations, int stopStage, double tolerance, cudaStream_t stream,
                     int smemBytes);
@@ -226,10 +228,16 @@ Status launchFault(int word);
 /// of `elemBytes` each (two rows, the scan's warp totals and the ring).
 int chainSweepBytes(int NI, int elemBytes);
 
-/// Dynamic shared memory the pressure CG needs to keep a solve's band on
-/// chip (0: it does not fit and the CG runs from global memory).
-int cgSharedBytes(int NI, int NJ, int clusterSize);
-constexpr int kMaxCgSharedBytes = 210 * 1024;
+/// Launch the plain form's kernel as `plan` says; dPlan and dList are its CTAs
+/// and list on the device (null for a plan of the first instance alone).
+Status launchPlain(const Instance* dInstances, const WidePlan& plan, const WideCta* dPlan, const int* dList,
+                   int threads, int iterations, int stopStage, double tolerance, cudaStream_t stream);
+/// The kernel's launch attributes (once per device), before a capture.
+Status preparePlainKernel();
+/// The kernels' implementation flags (kFlag*), from CFD_KERNEL_FLAGS.
+int kernelFlags();
+
+constexpr int kMaxClusterSmem = 210 * 1024;  // dynamic shared memory of the mixed form's kernel at most
 
 /// Cluster size used for a solve of `cells` cells (power of two, 1..16).
 int chooseClusterSize(int cells);

@@ -75,6 +75,14 @@ __host__ __device__ inline WideCgShape wideCgShape(int NI, int NJ, int R, int T)
   return s;
 }
 
+/// The fewest CTAs up to `width` that leave a CTA no more units than `width`
+/// CTAs would (and at least one per column tile).
+__host__ __device__ inline int wideUsefulCtas(int NI, int NJ, int width, int T) {
+  WideCgShape s = wideCgShape(NI, NJ, width, T);
+  if (s.RT < 1) return s.columnTiles;
+  return s.columnTiles * ((s.unitRows + s.units - 1) / s.units);
+}
+
 /// The messages of one exchange: bottom and top rows of every CTA row, left
 /// and right columns of every column tile, the units' three sums.
 __host__ __device__ inline long long wideMessages(int NI, int NJ, int R, int T) {
@@ -91,11 +99,12 @@ __host__ __device__ inline long long wideCgBorder(const WideCgShape& s) {
   return 2LL * s.units * s.B + 2LL * s.width;
 }
 /// Shared memory, in bytes, of the unrolled forms with C cells per thread: u
-/// and the border's r, s, 1/D; where the state is not all in registers the
-/// coefficients, p, x and 1/D.
+/// and the border's r, s, 1/D; p and x above 3 cells, and where they are not
+/// in registers (`all`) the coefficients and 1/D.
 __host__ __device__ inline long long wideCgUnrolledBytes(const WideCgShape& s, int C, int T, bool all) {
   long long n = wideCgPlane(s) + 3 * wideCgBorder(s);
   if (!all) n += 2 * wideCgPlane(s) + 3LL * C * T;
+  else if (C > 3) n += 2LL * C * T;
   return 8 * n;
 }
 /// Doubles of the form for any shape: u, both coefficients, the border, six
@@ -103,16 +112,34 @@ __host__ __device__ inline long long wideCgUnrolledBytes(const WideCgShape& s, i
 __host__ __device__ inline long long wideCgAnyDoubles(const WideCgShape& s, int T) {
   return 3 * wideCgPlane(s) + 3 * wideCgBorder(s) + 6LL * s.rounds * s.K * s.passes * T;
 }
-/// Dynamic shared memory for a team of R CTAs, and doubles of global memory
-/// per CTA for what does not fit there (0: everything does). The form for any
-/// shape must always have room: a wake map that couples to other rows takes it.
-__host__ __device__ inline long long wideCgBytes(int NI, int NJ, int R, int T, long long most) {
-  const WideCgShape s = wideCgShape(NI, NJ, R, T);
-  const long long any = 8 * wideCgAnyDoubles(s, T);
-  return (any < most) ? any : most;
+/// Which form takes the shape in `most` bytes: 8 K + units per team of the
+/// unrolled ones (in the split one, 0 units), or 0 for the form for any shape.
+__host__ __device__ inline int wideCgForm(const WideCgShape& s, int T, long long most) {
+  if (T != kWideThreads || s.passes != 1 || s.RT < 1) return 0;
+  auto fits = [&](int C, bool all) { return wideCgUnrolledBytes(s, C, T, all) <= most; };
+  if (s.units == 1) return (s.K <= 4 && fits(s.K, true)) ? 8 * s.K : 0;
+  if (s.units > kUnitBatch) return 0;
+  const int rounds = (s.rounds == 3) ? 4 : s.rounds;
+  if (s.K == 2 && rounds <= 4 && fits(2 * rounds, rounds == 1)) return 16 + rounds;
+  if (s.K == 4 && rounds <= 2 && fits(4 * rounds, false)) return 32 + rounds;
+  return 0;
 }
-__host__ __device__ inline long long wideCgSpill(int NI, int NJ, int R, int T, long long most) {
+__host__ __device__ inline long long wideCgFormBytes(const WideCgShape& s, int T, int form) {
+  const int K = form / 8, rounds = form % 8;
+  if (form == 0) return 8 * wideCgAnyDoubles(s, T);
+  return wideCgUnrolledBytes(s, K * ((rounds > 0) ? rounds : 1), T, rounds == 0 || K * rounds <= 2);
+}
+/// Dynamic shared memory for a team of R CTAs, and doubles of global memory
+/// per CTA for what does not fit there (0: everything does). `any`: with the
+/// form for any shape (a wake map that couples to other rows needs it).
+__host__ __device__ inline long long wideCgBytes(int NI, int NJ, int R, int T, long long most, bool any) {
   const WideCgShape s = wideCgShape(NI, NJ, R, T);
+  const long long n = wideCgFormBytes(s, T, any ? 0 : wideCgForm(s, T, most));
+  return (n < most) ? n : most;
+}
+__host__ __device__ inline long long wideCgSpill(int NI, int NJ, int R, int T, long long most, bool any) {
+  const WideCgShape s = wideCgShape(NI, NJ, R, T);
+  if (!any && wideCgForm(s, T, most) != 0) return 0;
   return (8 * wideCgAnyDoubles(s, T) <= most) ? 0 : wideCgAnyDoubles(s, T);
 }
 
@@ -353,10 +380,16 @@ DEV void updateBorder(const WideTeam& t, const WideCgSystem& S, const Loader& lo
 /// one unit per CTA, held by the first 256 threads; the others have the border
 /// and the waiting.
 template <int K, int kRounds, bool kSplit, typename Loader>
-DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Loader& load) {
+__device__ __noinline__ WideCgResult wideCgUnrolledTile(WideTeam& team, const WideCgSystem& system, const Loader& load) {
+  // a function of its own, for its registers; copies, because what is read
+  // through a reference is read from the stack again after every message
+  WideTeam t = team;
+  const WideCgSystem S = system;
   extern __shared__ double dyn[];
   constexpr int C = K * kRounds;
-  constexpr bool kAll = kSplit || C <= 2;  // the whole state in registers
+  constexpr bool kAll = kSplit || C <= 2;  // the coefficients and 1/D in registers
+  constexpr bool kPx = kAll && C <= 3;     // p and x too
+  constexpr bool kU = C <= 4;              // a copy of u as well
   const WideCgTile a(t, false);
   const int T = t.T, tid = t.tid, NI = t.NI, SW = a.stride;
   const int plane = static_cast<int>(wideCgPlane(a.z)), border = a.border();
@@ -364,7 +397,8 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
   double* const hr = dyn + plane;
   double* const sN = hr + 3 * wideCgBorder(a.z);
   double* const sE = sN + plane;
-  double* const mine = sE + plane + tid;  // p, x, 1/D of cell k at k*T, (C + k)*T, (2C + k)*T
+  // p, x, 1/D of cell k at k*T, (C + k)*T, (2C + k)*T
+  double* const mine = (kAll ? hr + 3 * wideCgBorder(a.z) : sE + plane) + tid;
   const int teams = kSplit ? 1 : a.z.teams;
   for (int m = tid; m < plane; m += T) U[m] = 0.0;
   if constexpr (!kAll) {
@@ -443,12 +477,13 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
       }
       __syncthreads();  // u
     }
+    team.epoch = t.epoch;
     return WideCgResult{z.iterations, z.initial, z.final, z.converged};
   }
 
   // ---- the thread's cells ----
-  double r[C], w[C], s[C], u[C];
-  double p[kAll ? C : 1], x[kAll ? C : 1], di[kAll ? C : 1];
+  double r[C], w[C], s[C], u[kU ? C : 1];
+  double p[kPx ? C : 1], x[kPx ? C : 1], di[kAll ? C : 1];
   double cS[kAll ? kRounds : 1], cN[kAll ? C : 1], cW[kAll ? C : 1], cE[kAll ? C : 1];
   int first[kRounds];  // the place of the round's first cell; the others follow down the column
   int south = -SW;     // where the very first cell's south neighbour is, from its place
@@ -463,7 +498,8 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
       const int k = m * K + kk;
-      r[k] = w[k] = s[k] = u[k] = 0.0;
+      r[k] = w[k] = s[k] = 0.0;
+      if constexpr (kU) u[k] = 0.0;
       double xk = 0.0, dk = 0.0;
       if constexpr (kAll) cN[k] = cW[k] = cE[k] = 0.0;
       if (kAll && kk == 0) cS[m] = 0.0;
@@ -475,8 +511,9 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
         xk = S.x[c];
         dk = wideCgReciprocal(D);
         if (!isfinite(dk)) oddCells |= 1u << k;
-        u[k] = isfinite(dk) ? r[k] * dk : wideCgPrecondition(r[k], D);
-        U[first[m] + kk * SW] = u[k];
+        const double u0 = isfinite(dk) ? r[k] * dk : wideCgPrecondition(r[k], D);
+        if constexpr (kU) u[k] = u0;
+        U[first[m] + kk * SW] = u0;
         if constexpr (kAll) {
           if (kk == 0) cS[m] = load.north(i, j);
           cN[k] = load.north(i, j + 1);
@@ -493,15 +530,15 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
         }
         if (k == 0) side = a.toSide(t, a.q, lr);
       }
-      if constexpr (kAll) {
+      if constexpr (kPx) {
         p[k] = 0.0;
         x[k] = xk;
-        di[k] = dk;
       } else {
         mine[k * T] = 0.0;
         mine[(C + k) * T] = xk;
-        mine[(2 * C + k) * T] = dk;
       }
+      if constexpr (kAll) di[k] = dk;
+      else mine[(2 * C + k) * T] = dk;
     }
   }
   const bool odd = __syncthreads_or(oddBorder || oddCells != 0);
@@ -515,13 +552,13 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
     for (int m = 0; m < kRounds; ++m) {
       const double* const at = U + first[m];
       double us = (m == 0) ? at[south] : at[-SW], acc[3] = {0.0, 0.0, 0.0};
-      const double uTop = at[K * SW];
+      double uc = at[0];
 #pragma unroll
       for (int kk = 0; kk < K; ++kk) {
         const int k = m * K + kk;
-        const double un = (kk + 1 < K) ? ((have >> (k + 1)) & 1u ? u[(k + 1 < C) ? k + 1 : k] : at[(kk + 1) * SW]) : uTop;
+        const double un = at[(kk + 1) * SW];
         double y = r[k];  // D u is r, unless D has no reciprocal
-        if (odd && (oddCells & (1u << k))) y = S.D[cellOf(k)] * u[k];
+        if (odd && (oddCells & (1u << k))) y = S.D[cellOf(k)] * uc;
         if constexpr (kAll) {
           y = fma((kk == 0) ? cS[m] : cN[k - 1], us, y);
           y = fma(cN[k], un, y);
@@ -535,13 +572,15 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
           y = fma(e[0], at[kk * SW - 1], y);
           y = fma(e[1], at[kk * SW + 1], y);
         }
-        us = u[k];
-        if (!((have >> k) & 1u)) y = 0.0;
+        const bool there = (have >> k) & 1u;
+        if (!there) y = 0.0;
         w[k] = y;
         if (k == top) edge = y;
-        acc[0] = fma(r[k], u[k], acc[0]);
-        acc[1] = fma(y, u[k], acc[1]);
+        acc[0] = fma(r[k], there ? uc : 0.0, acc[0]);
+        acc[1] = fma(y, uc, acc[1]);
         acc[2] += fabs(r[k]);
+        us = uc;
+        uc = un;
       }
       if (unitOf(m) < a.units) unitPartial(t, a, unitOf(m), acc);
     }
@@ -577,11 +616,13 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
     for (int k = 0; k < C; ++k) {
       s[k] = fma(z.beta, s[k], w[k]);
       r[k] = fma(-z.alpha, s[k], r[k]);
-      const double before = u[k];
-      u[k] = r[k] * (kAll ? di[kAll ? k : 0] : mine[(2 * C + k) * T]);
-      if (odd && (oddCells & (1u << k))) u[k] = wideCgPrecondition(r[k], S.D[cellOf(k)]);
-      if ((have >> k) & 1u) U[first[k / K] + (k % K) * SW] = u[k];
-      if constexpr (kAll) {
+      double* const place = U + first[k / K] + (k % K) * SW;
+      const double before = kU ? u[kU ? k : 0] : *place;
+      double next = r[k] * (kAll ? di[kAll ? k : 0] : mine[(2 * C + k) * T]);
+      if (odd && (oddCells & (1u << k))) next = wideCgPrecondition(r[k], S.D[cellOf(k)]);
+      if constexpr (kU) u[k] = next;
+      if ((have >> k) & 1u) *place = next;
+      if constexpr (kPx) {
         p[k] = fma(z.beta, p[k], before);
         x[k] = fma(z.alpha, p[k], x[k]);
       } else {
@@ -594,15 +635,19 @@ DEV WideCgResult wideCgUnrolledTile(WideTeam& t, const WideCgSystem& S, const Lo
   }
 #pragma unroll
   for (int k = 0; k < C; ++k) {
-    if ((have >> k) & 1u) S.x[cellOf(k)] = kAll ? x[kAll ? k : 0] : mine[(C + k) * T];
+    if ((have >> k) & 1u) S.x[cellOf(k)] = kPx ? x[kPx ? k : 0] : mine[(C + k) * T];
   }
+  team.epoch = t.epoch;
   return WideCgResult{z.iterations, z.initial, z.final, z.converged};
 }
 
 /// The form for any shape: every array in memory, on chip as far as
 /// `smemBytes` reach, the rest in the CTA's part of S.spill.
 template <typename Loader>
-DEV WideCgResult wideCgAnyTile(WideTeam& t, const WideCgSystem& S, const Loader& load, int smemBytes) {
+__device__ __noinline__ WideCgResult wideCgAnyTile(WideTeam& team, const WideCgSystem& system, const Loader& load,
+                                                   int smemBytes) {
+  WideTeam t = team;
+  const WideCgSystem S = system;
   extern __shared__ double dyn[];
   const WideCgTile a(t, S.wakeAnywhere);
   const int T = t.T, tid = t.tid, NI = t.NI, SW = a.stride, border = a.border();
@@ -738,31 +783,26 @@ DEV WideCgResult wideCgAnyTile(WideTeam& t, const WideCgSystem& S, const Loader&
   for (int unit = a.team; unit < a.units; unit += a.z.teams) {
     unitCells(unit, [&](int slot, int lr, int q) { S.x[(a.j0 + lr) * NI + a.i0 + q] = x[slot]; });
   }
+  team.epoch = t.epoch;
   return WideCgResult{z.iterations, z.initial, z.final, z.converged};
 }
 
 /// The whole solve by every thread of the team, in the block's dynamic shared
 /// memory of `smemBytes`; on return x is written (no barrier after it). Needs
-/// at least as many CTAs as column tiles.
+/// at least as many CTAs as column tiles. `any`: the form for any shape.
 template <typename Loader>
-DEV WideCgResult wideCg(WideTeam& t, const WideCgSystem& S, const Loader& load, int smemBytes) {
+DEV WideCgResult wideCg(WideTeam& t, const WideCgSystem& S, const Loader& load, int smemBytes, bool any) {
   const WideCgShape z = wideCgShape(t.NI, t.NJ, t.R, t.T);
-  const bool unrolled = t.T == kWideThreads && z.passes == 1 && !S.wakeAnywhere;
-  auto fits = [&](int C) { return wideCgUnrolledBytes(z, C, t.T, z.units == 1 || C <= 2) <= smemBytes; };
-  if (unrolled && z.units == 1) {
-    if (z.K == 2 && fits(2)) return wideCgUnrolledTile<2, 1, true>(t, S, load);
-    if (z.K == 3 && fits(3)) return wideCgUnrolledTile<3, 1, true>(t, S, load);
-    if (z.K == 4 && fits(4)) return wideCgUnrolledTile<4, 1, true>(t, S, load);
-  } else if (unrolled && z.units <= kUnitBatch) {
-    switch (8 * z.K + z.rounds) {
-      case 16 + 1: if (fits(2)) return wideCgUnrolledTile<2, 1, false>(t, S, load); break;
-      case 16 + 2: if (fits(4)) return wideCgUnrolledTile<2, 2, false>(t, S, load); break;
-      case 16 + 3:
-      case 16 + 4: if (fits(8)) return wideCgUnrolledTile<2, 4, false>(t, S, load); break;
-      case 32 + 1: if (fits(4)) return wideCgUnrolledTile<4, 1, false>(t, S, load); break;
-      case 32 + 2: if (fits(8)) return wideCgUnrolledTile<4, 2, false>(t, S, load); break;
-      default: break;
-    }
+  switch ((any || S.wakeAnywhere) ? 0 : wideCgForm(z, t.T, smemBytes)) {
+    case 16: return wideCgUnrolledTile<2, 1, true>(t, S, load);
+    case 24: return wideCgUnrolledTile<3, 1, true>(t, S, load);
+    case 32: return wideCgUnrolledTile<4, 1, true>(t, S, load);
+    case 17: return wideCgUnrolledTile<2, 1, false>(t, S, load);
+    case 18: return wideCgUnrolledTile<2, 2, false>(t, S, load);
+    case 20: return wideCgUnrolledTile<2, 4, false>(t, S, load);
+    case 33: return wideCgUnrolledTile<4, 1, false>(t, S, load);
+    case 34: return wideCgUnrolledTile<4, 2, false>(t, S, load);
+    default: break;
   }
   return wideCgAnyTile(t, S, load, smemBytes);
 }

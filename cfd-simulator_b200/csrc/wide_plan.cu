@@ -1,8 +1,13 @@
-// wide_plan.cu - how many CTAs a wide team gets (host side).
+// wide_plan.cu - how many CTAs a wide team gets, and how a launch shares the
+// GPU between solves (host side).
 
 #include "wide_plan.hpp"
 
+#include <cstdlib>
+#include <numeric>
+
 #include "common.hpp"
+#include "row_sweeps.cuh"
 #include "solver.hpp"
 #include "wide_cg.cuh"
 
@@ -26,16 +31,126 @@ int wideCapacity() {
 
 double wideCgMicroseconds(int NI, int NJ, int R) {
   const WideCgShape s = wideCgShape(NI, NJ, R, kWideThreads);
-  return 1.2 + 0.15 * s.rounds * s.K * s.passes + ((R > 1) ? 0.2 : 0.0);
+  const int cells = s.rounds * s.K * s.passes, form = wideCgForm(s, kWideThreads, kMaxWideSmem);
+  if (form == 0) return 2.0 + 1.3 * cells;
+  return (form % 8 == 0) ? 1.2 + 0.5 * cells : 1.2 + 1.0 * cells;
+}
+
+int wideLeastCtas(int NI, int threads) { return wideCgShape(NI, 1, 1, threads).columnTiles; }
+
+int wideMostCtas(int NI, int NJ, int threads) {
+  const WideCgShape s = wideCgShape(NI, NJ, 1, threads);
+  return std::min(s.columnTiles * s.unitRows, kMaxWideCtas / s.columnTiles * s.columnTiles);
 }
 
 int wideChooseCtas(int NI, int NJ, int capacity) {
-  const int columns = wideCgShape(NI, NJ, 1, kWideThreads).columnTiles;
+  const int columns = wideLeastCtas(NI, kWideThreads);
   int best = columns;
   for (int R = columns; R <= capacity; R += columns) {
     if (wideCgMicroseconds(NI, NJ, R) < wideCgMicroseconds(NI, NJ, best)) best = R;
   }
   return best;
+}
+
+long long wideSpillDoubles(int NI, int NJ, int most, int threads) {
+  long long doubles = 0;
+  const int columns = wideLeastCtas(NI, threads);
+  for (int R = columns; R <= std::max(most, columns); ++R) {
+    doubles = std::max(doubles, R * wideCgSpill(NI, NJ, R, threads, kMaxWideSmem, true));
+  }
+  return doubles;
+}
+
+namespace {
+
+int usefulCtas(const WideJob& job, int width, int threads) {
+  return wideUsefulCtas(job.NI, job.NJ, std::min(width, job.most), threads);
+}
+
+/// Modelled microseconds of one outer iteration: the CG, ~17 barriers, the
+/// other phases' passes (0.54 ms on 16 CTAs at 768x192), the sweeps' rows.
+double outerMicroseconds(const WideJob& job, int R) {
+  const double cells = static_cast<double>(job.NI) * job.NJ;
+  return 200.0 * wideCgMicroseconds(job.NI, job.NJ, R) + 30.0 + cells / R / 512.0 * (job.sst ? 30.0 : 15.0) +
+         (job.sst ? 0.4 * job.NJ : 0.0);
+}
+
+int smemBytes(const WideJob& job, int R, int threads) {
+  const bool any = (kernelFlags() & kFlagSharedCg) != 0;
+  long long bytes = wideCgBytes(job.NI, job.NJ, R, threads, kMaxWideSmem, any);
+  {
+    // whatever the model is now: it can be changed after a batch is planned
+    const RowSweepShape z = rowSweepShape(job.NI);
+    const int warps = threads / 32, perCta = (2 * kSweeps + R - 1) / R;
+    long long sweeps = static_cast<long long>(std::min(perCta, warps)) * rowSweepBytes(z);
+    if (perCta == 1 && warps >= z.chunks && rowSweepRingBytes(z) <= kMaxWideSmem) sweeps = rowSweepRingBytes(z);
+    bytes = std::max(bytes, std::min<long long>(sweeps, kMaxWideSmem));
+  }
+  return static_cast<int>(bytes);
+}
+
+}  // namespace
+
+WidePlan planWide(const std::vector<WideJob>& jobs, int threads) {
+  WidePlan plan;
+  const int capacity = std::max(wideCapacity(), 1), count = static_cast<int>(jobs.size());
+  // side by side, each at its widest
+  std::vector<int> widths(jobs.size());
+  int total = 0;
+  for (int k = 0; k < count; ++k) {
+    widths[k] = usefulCtas(jobs[k], std::min(jobs[k].most, capacity), threads);
+    total += widths[k];
+  }
+  if (total <= capacity) {
+    for (int k = 0; k < count; ++k) {
+      for (int r = 0; r < widths[k]; ++r) plan.ctas.push_back(WideCta{k, k + 1, r, widths[k]});
+      plan.list.push_back(k);
+      plan.smemBytes = std::max(plan.smemBytes, smemBytes(jobs[k], widths[k], threads));
+    }
+    return plan;
+  }
+  // teams of equal width, each with a list of solves: longest first to the
+  // team that is free first. The number of teams that finishes first wins; a
+  // solve's bits do not depend on it.
+  int least = 1;
+  for (const WideJob& job : jobs) least = std::max(least, wideLeastCtas(job.NI, threads));
+  double best = -1.0;
+  int bestTeams = 1;
+  std::vector<std::vector<int>> bestLists;
+  for (int teams = 1; teams <= std::min(count, capacity / least); ++teams) {
+    const int width = capacity / teams;
+    std::vector<double> cost(jobs.size()), load(static_cast<std::size_t>(teams), 0.0);
+    std::vector<int> order(jobs.size());
+    std::iota(order.begin(), order.end(), 0);
+    for (int k = 0; k < count; ++k) cost[k] = outerMicroseconds(jobs[k], usefulCtas(jobs[k], width, threads));
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::vector<std::vector<int>> lists(static_cast<std::size_t>(teams));
+    for (int k : order) {
+      const std::size_t team = std::min_element(load.begin(), load.end()) - load.begin();
+      lists[team].push_back(k);
+      load[team] += cost[k];
+    }
+    const double makespan = *std::max_element(load.begin(), load.end());
+    if (best < 0.0 || makespan < best) {
+      best = makespan;
+      bestTeams = teams;
+      bestLists = std::move(lists);
+    }
+  }
+  const int width = capacity / bestTeams;
+  for (const std::vector<int>& solves : bestLists) {
+    const int begin = static_cast<int>(plan.list.size());
+    int widest = 0;
+    for (int k : solves) {
+      plan.list.push_back(k);
+      const int R = usefulCtas(jobs[k], width, threads);
+      widest = std::max(widest, R);
+      plan.smemBytes = std::max(plan.smemBytes, smemBytes(jobs[k], R, threads));
+    }
+    const int end = static_cast<int>(plan.list.size());
+    for (int r = 0; r < widest; ++r) plan.ctas.push_back(WideCta{begin, end, r, width});
+  }
+  return plan;
 }
 
 }  // namespace cfdb

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <vector>
 
 #include "instance.hpp"
 
@@ -18,8 +19,8 @@ int wideCapacity();
 
 /// The layout of a wide team's scratch, with `messages` messages in a set.
 struct WideScratchLayout {
-  std::size_t epoch, flags, slots, rowSums, set, bytes;
-  WideScratchLayout(int NJ, long long messages) {
+  std::size_t epoch, flags, slots, chunkSums, set, bytes;
+  WideScratchLayout(int NI, int NJ, long long messages) {
     std::size_t at = 0;
     auto take = [&](std::size_t n) {
       const std::size_t here = at;
@@ -29,7 +30,7 @@ struct WideScratchLayout {
     epoch = take(sizeof(unsigned long long));
     flags = take(kMaxWideCtas * sizeof(unsigned));
     slots = take(2 * kMaxWideCtas * 8 * sizeof(double));
-    rowSums = take(2 * 4 * static_cast<std::size_t>(NJ) * sizeof(double));
+    chunkSums = take(2 * 4 * ((static_cast<std::size_t>(NI) * NJ + 255) / 256) * sizeof(double));
     set = take(2 * static_cast<std::size_t>(messages) * sizeof(ulonglong2));
     bytes = at;
   }
@@ -37,7 +38,7 @@ struct WideScratchLayout {
     return WideScratch{reinterpret_cast<unsigned long long*>(base + epoch),
                        reinterpret_cast<unsigned*>(base + flags),
                        reinterpret_cast<double*>(base + slots),
-                       reinterpret_cast<double*>(base + rowSums),
+                       reinterpret_cast<double*>(base + chunkSums),
                        reinterpret_cast<ulonglong2*>(base + set)};
   }
 };
@@ -48,5 +49,28 @@ double wideCgMicroseconds(int NI, int NJ, int R);
 
 /// CTAs for a lone system: the count with the smallest modelled time.
 int wideChooseCtas(int NI, int NJ, int capacity);
+
+/// CTAs a solve can use at most (a CG unit each) and needs at least (a column
+/// tile each), for blocks of `threads`.
+int wideMostCtas(int NI, int NJ, int threads);
+int wideLeastCtas(int NI, int threads);
+
+/// Doubles of spill a solve needs whatever the number of its CTAs up to `most`.
+long long wideSpillDoubles(int NI, int NJ, int most, int threads);
+
+/// A solve as the planner sees it.
+struct WideJob {
+  int NI, NJ;
+  int most;  // CTAs at most
+  bool sst;
+};
+struct WidePlan {
+  std::vector<WideCta> ctas;
+  std::vector<int> list;  // solves in the order the CTAs' ranges name them
+  int smemBytes{0};
+};
+/// How one launch runs these solves: side by side when the GPU holds them all
+/// at their widest, else in teams that take one solve after another.
+WidePlan planWide(const std::vector<WideJob>& jobs, int threads);
 
 }  // namespace cfdb

@@ -20,9 +20,8 @@
 // a code in the launch's fault word, after which the CTA waits no more, so a
 // launch always ends and the host reports it.
 //
-// Sums are formed per row of cells (a fixed tree over its columns) and the
-// rows' sums in one fixed order, so their bits do not depend on how many CTAs
-// share the rows.
+// Sums are formed per chunk of 256 consecutive cells and the chunks' sums in one
+// fixed order, so their bits do not depend on how many CTAs share the cells.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,12 +31,15 @@
 
 namespace cfdb {
 
-constexpr int kRowBatch = 32;       // rows whose partial sums are held at once
-constexpr int kMaxGroupWarps = 8;   // warps that share a row (256 columns at a time)
-constexpr int kMaxRowSums = 4;
+constexpr int kChunkCells = 256;  // cells whose sums are formed together, by as many threads
+constexpr int kChunkBatch = 16;   // chunks of a CTA whose partial sums are held at once
+constexpr int kMaxSums = 4;
 constexpr int kWideThreads = 512;
-/// Polls before a wait gives up: each is an L2 round trip (~0.7 us), ~3 s in all.
-constexpr int kWideSpinLimit = 1 << 22;
+/// Polls before a wait gives up, each an L2 round trip (0.4 us or more): ~1 s,
+/// and ~15 ms more for every iteration of every solve that a CTA may wait for
+/// its team to finish first.
+constexpr int kWideSpinLimit = 1 << 21;
+constexpr int kWideSpinPerIteration = 1 << 15;
 
 constexpr int kUnitBatch = 8;       // units of the CG whose partial sums are held at once
 constexpr int kUnitWarps = 8;       // warps that share a unit
@@ -46,7 +48,8 @@ constexpr int kSumCopies = 4;       // copies of every unit's sums, each polled 
 
 struct WideShared {
   union {
-    double rowPart[kRowBatch][kMaxGroupWarps][kMaxRowSums];
+    double chunkPart[kChunkBatch][kChunkCells / 32][kMaxSums];
+    double groupPart[kMaxSums][256];
     double unitPart[kUnitBatch][kUnitWarps][4];
   };
   double warpPart[kWideThreads / 32][kRedSlots];
@@ -57,42 +60,33 @@ struct WideShared {
 
 struct WideTeam {
   int rank, R, tid, T;
-  int NI, NJ;
-  int j0, j1;        // own rows
-  int c0, c1;        // own cells
-  int G, ng;         // threads that share a row, and how many rows at once
-  int g, q;          // this thread's row group and its first column
+  int NI, NJ, N;
+  int chunks;            // of the block
+  int chunk0, chunk1;    // own ones
+  int c0, c1;            // own cells: whole chunks
   unsigned epoch;
+  int spinLimit;
   WideScratch mem;
   int* faultWord;
   WideShared* sh;
 };
 
-/// Threads that share a row: columns in equal passes of at most 256 (and of
-/// at most the block's threads), in whole warps.
-__host__ __device__ inline int wideGroup(int NI, int T) {
-  const int most = (T < 32 * kMaxGroupWarps) ? T : 32 * kMaxGroupWarps;
-  const int passes = (NI + most - 1) / most;
-  const int columns = (NI + passes - 1) / passes;
-  return (columns + 31) / 32 * 32;
-}
-
 DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShared* sh, int rank, int R, int NI,
-                  int NJ) {
+                  int NJ, int iterationsAhead) {
   t.rank = rank;
   t.R = R;
   t.tid = static_cast<int>(threadIdx.x);
   t.T = static_cast<int>(blockDim.x);
   t.NI = NI;
   t.NJ = NJ;
-  t.j0 = static_cast<int>((static_cast<long long>(NJ) * rank) / R);
-  t.j1 = static_cast<int>((static_cast<long long>(NJ) * (rank + 1)) / R);
-  t.c0 = t.j0 * NI;
-  t.c1 = t.j1 * NI;
-  t.G = wideGroup(NI, t.T);
-  t.ng = t.T / t.G;
-  t.g = t.tid / t.G;
-  t.q = t.tid - t.g * t.G;
+  t.N = NI * NJ;
+  t.chunks = (t.N + kChunkCells - 1) / kChunkCells;
+  t.chunk0 = static_cast<int>(static_cast<long long>(t.chunks) * rank / R);
+  t.chunk1 = static_cast<int>(static_cast<long long>(t.chunks) * (rank + 1) / R);
+  t.c0 = t.chunk0 * kChunkCells;
+  t.c1 = min(t.chunk1 * kChunkCells, t.N);
+  if (t.c0 > t.c1) t.c0 = t.c1;
+  t.spinLimit = kWideSpinLimit + kWideSpinPerIteration * min(iterationsAhead, 32768);
   t.mem = mem;
   t.faultWord = faultWord;
   t.sh = sh;
@@ -118,7 +112,7 @@ DEV void wideLeave(WideTeam& t) {
 /// One more unsuccessful poll: true when the wait is over (given up now or before).
 DEV bool wideGiveUp(WideTeam& t, int& polls, int code) {
   if (*static_cast<volatile int*>(&t.sh->fault) != 0) return true;
-  if (++polls < kWideSpinLimit) return false;
+  if (++polls < t.spinLimit) return false;
   t.sh->fault = 1;
   atomicOr(t.faultWord, code);
   return true;
@@ -248,28 +242,6 @@ DEV void wideMax(WideTeam& t, double (&v)[K]) {
   for (int k = 0; k < K; ++k) v[k] = t.sh->result[k];
 }
 
-/// A row's sums within its warps, into rowPart (slot = the row's place in the batch).
-template <int K>
-DEV void rowPartial(WideTeam& t, int slot, double (&acc)[K]) {
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], off);
-  }
-  if ((t.tid & 31) == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) t.sh->rowPart[slot][t.q >> 5][k] = acc[k];
-  }
-}
-/// The sum of a row over its warps, once they have all been stored.
-DEV double rowTotal(const WideTeam& t, int slot, int k) {
-  const int warps = t.G >> 5;
-  double a[kMaxGroupWarps];
-#pragma unroll
-  for (int w = 0; w < kMaxGroupWarps; ++w) a[w] = (w < warps) ? t.sh->rowPart[slot][w][k] : 0.0;
-  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-}
-
 /// The sum of a CG unit over its `warps` warps, once they have all been stored.
 DEV double unitTotal(const WideTeam& t, int slot, int k, int warps) {
   double a[kUnitWarps];
@@ -278,41 +250,74 @@ DEV double unitTotal(const WideTeam& t, int slot, int k, int warps) {
   return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
 }
 
-/// cell(c, i, j, acc) over every own cell, adding to the row's sums; the
-/// team's totals in every thread. Also a barrier.
+/// f(c, i, j) for every own cell.
+template <typename F>
+DEV void wideCells(const WideTeam& t, F&& f) {
+  for (int c = t.c0 + t.tid; c < t.c1; c += t.T) {
+    const int j = c / t.NI;
+    f(c, c - j * t.NI, j);
+  }
+}
+
+/// cell(c, i, j, acc) over every own cell, adding to its chunk's sums; the
+/// team's totals in every thread. Also a barrier. A chunk's sums are a tree
+/// over its cells, 32 chunks' a tree, and those are added in order.
 template <int K, typename F>
-DEV void wideRowSums(WideTeam& t, double (&out)[K], F&& cell) {
+DEV void wideSums(WideTeam& t, double (&out)[K], F&& cell) {
   const int lane = t.tid & 31, warp = t.tid >> 5, warps = t.T >> 5;
-  const int rows = t.j1 - t.j0;
-  double* sums = t.mem.rowSums + static_cast<std::size_t>((t.epoch + 1u) & 1u) * kMaxRowSums * t.NJ;
-  for (int base = 0; base < rows; base += kRowBatch) {
-    const int n = (rows - base < kRowBatch) ? rows - base : kRowBatch;
-    if (t.g < t.ng) {
-      for (int lr = t.g; lr < n; lr += t.ng) {
-        const int j = t.j0 + base + lr;
+  const int team = min(t.T, kChunkCells), teams = t.T / team, mine = t.tid / team, lt = t.tid - mine * team;
+  double* sums = t.mem.chunkSums + static_cast<std::size_t>((t.epoch + 1u) & 1u) * kMaxSums * t.chunks;
+  for (int base = t.chunk0; base < t.chunk1; base += kChunkBatch) {
+    const int n = min(t.chunk1 - base, kChunkBatch);
+    for (int slot = mine; slot < n && mine < teams; slot += teams) {
+      // the same 32 cells share a warp's part whatever the number of threads
+      for (int first = lt; first < kChunkCells; first += team) {
+        const int c = (base + slot) * kChunkCells + first;
         double acc[K] = {};
-        for (int i = t.q; i < t.NI; i += t.G) cell(j * t.NI + i, i, j, acc);
-        rowPartial(t, lr, acc);
+        if (c < t.N) {
+          const int j = c / t.NI;
+          cell(c, c - j * t.NI, j, acc);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], off);
+          if (lane == 0) t.sh->chunkPart[slot][first >> 5][k] = acc[k];
+        }
       }
     }
     __syncthreads();
     for (int m = t.tid; m < n * K; m += t.T) {
-      const int lr = m / K, k = m - lr * K;
-      sums[k * t.NJ + t.j0 + base + lr] = rowTotal(t, lr, k);
+      const int slot = m / K, k = m - slot * K;
+      double a[kChunkCells / 32];
+#pragma unroll
+      for (int w = 0; w < kChunkCells / 32; ++w) a[w] = t.sh->chunkPart[slot][w][k];
+      sums[k * t.chunks + base + slot] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     }
-    if (base + kRowBatch < rows) __syncthreads();
+    if (base + kChunkBatch < t.chunk1) __syncthreads();
   }
   wideBarrier(t);
-  for (int k = warp; k < K; k += warps) {
-    double a = 0.0;
-    for (int j = lane; j < t.NJ; j += 32) a += __ldcg(sums + k * t.NJ + j);
+  const int groups = (t.chunks + 31) / 32;
+  double total[K] = {};
+  for (int first = 0; first < groups; first += 256) {
+    const int n = min(groups - first, 256);
+    for (int m = warp; m < K * n; m += warps) {
+      const int k = m / n, group = first + m - k * n, at = group * 32 + lane;
+      double a = (at < t.chunks) ? __ldcg(sums + k * t.chunks + at) : 0.0;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
-    if (lane == 0) t.sh->result[k] = a;
+      for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
+      if (lane == 0) t.sh->groupPart[k][group - first] = a;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      for (int g = 0; g < n; ++g) total[k] += t.sh->groupPart[k][g];
+    }
+    __syncthreads();
   }
-  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = t.sh->result[k];
+  for (int k = 0; k < K; ++k) out[k] = total[k];
 }
 
 }  // namespace cfdb
