@@ -80,7 +80,8 @@ constexpr int kMaxWideCtas = 160;  // CTAs of one team at most (a B200 has 148 S
 /// Zero-filled once; the epoch carries the tags on from launch to launch.
 struct WideScratch {
   unsigned long long* epoch;
-  unsigned* flags;    // [kMaxWideCtas]
+  unsigned* arrived;  // the barrier's count, 0 between launches
+  unsigned* left;     // CTAs that have left the launch
   double* slots;      // maxima: [2][kMaxWideCtas][8]
   double* chunkSums;  // [2][4][chunks of 256 cells]
   // the CG's messages, two sets (parity of the exchange) of

@@ -478,6 +478,7 @@ __device__ __noinline__ WideCgResult wideCgUnrolledTile(WideTeam& team, const Wi
       __syncthreads();  // u
     }
     team.epoch = t.epoch;
+    team.barriers = t.barriers;
     return WideCgResult{z.iterations, z.initial, z.final, z.converged};
   }
 
@@ -638,6 +639,7 @@ __device__ __noinline__ WideCgResult wideCgUnrolledTile(WideTeam& team, const Wi
     if ((have >> k) & 1u) S.x[cellOf(k)] = kPx ? x[kPx ? k : 0] : mine[(C + k) * T];
   }
   team.epoch = t.epoch;
+  team.barriers = t.barriers;
   return WideCgResult{z.iterations, z.initial, z.final, z.converged};
 }
 
@@ -784,6 +786,7 @@ __device__ __noinline__ WideCgResult wideCgAnyTile(WideTeam& team, const WideCgS
     unitCells(unit, [&](int slot, int lr, int q) { S.x[(a.j0 + lr) * NI + a.i0 + q] = x[slot]; });
   }
   team.epoch = t.epoch;
+  team.barriers = t.barriers;
   return WideCgResult{z.iterations, z.initial, z.final, z.converged};
 }
 

@@ -19,7 +19,7 @@ int wideCapacity();
 
 /// The layout of a wide team's scratch, with `messages` messages in a set.
 struct WideScratchLayout {
-  std::size_t epoch, flags, slots, chunkSums, set, bytes;
+  std::size_t epoch, arrived, left, slots, chunkSums, set, bytes;
   WideScratchLayout(int NI, int NJ, long long messages) {
     std::size_t at = 0;
     auto take = [&](std::size_t n) {
@@ -28,7 +28,8 @@ struct WideScratchLayout {
       return here;
     };
     epoch = take(sizeof(unsigned long long));
-    flags = take(kMaxWideCtas * sizeof(unsigned));
+    arrived = take(sizeof(unsigned));  // a line each
+    left = take(sizeof(unsigned));
     slots = take(2 * kMaxWideCtas * 8 * sizeof(double));
     chunkSums = take(2 * 4 * ((static_cast<std::size_t>(NI) * NJ + 255) / 256) * sizeof(double));
     set = take(2 * static_cast<std::size_t>(messages) * sizeof(ulonglong2));
@@ -36,7 +37,8 @@ struct WideScratchLayout {
   }
   WideScratch at(char* base) const {
     return WideScratch{reinterpret_cast<unsigned long long*>(base + epoch),
-                       reinterpret_cast<unsigned*>(base + flags),
+                       reinterpret_cast<unsigned*>(base + arrived),
+                       reinterpret_cast<unsigned*>(base + left),
                        reinterpret_cast<double*>(base + slots),
                        reinterpret_cast<double*>(base + chunkSums),
                        reinterpret_cast<ulonglong2*>(base + set)};
