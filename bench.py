@@ -1,7 +1,7 @@
 """Benchmark: the batched polar of steady SIMPLE solves (k-omega SST, plain FP64).
 
 Workload (one "step" = one SIMPLE outer iteration of every solve in it, all
-in one batched launch, one thread-block cluster per solve):
+in one batched launch, a team of CTAs per solve):
   a 21-point NACA 2412 polar, Re 3e6, alpha -4..16 deg step 1, on the fine
   C-grid 768 x 192 cells (surface 256, wake 129, normal 193 points; first
   layer 5e-6 chord), plus NACA 0012 at Re 1e6, alpha 4 deg, on the coarse
@@ -31,7 +31,6 @@ replicas, one per GPU; no collective on the data path (weak scaling).
 from __future__ import annotations
 
 import argparse
-import contextlib
 import json
 import math
 import os
@@ -63,10 +62,7 @@ POLAR = ([("2412", float(a), 3e6, "fine", 5e-6) for a in range(-4, 17)]
             ("0012", 4.0, 1e6, "fine", 5e-6)])
 POLAR_NAME = ("batched polar: NACA2412 k-omega SST Re3e6 C-grid 768x192, alpha -4..16 step 1 "
               "(21 solves) + NACA0012 k-omega SST Re1e6 alpha 4 on 192x48/384x96/768x192, "
-              "24 solves in one batch (one launch per cluster size)")
-# The mixed form runs on clusters of at most 8 CTAs (the engine's default
-# policy for it: smaller clusters fit more of its solves on the GPU).
-MIXED_CLUSTER = 8
+              "24 solves in one batch (one launch)")
 # The former headline pair (384 x 96, alpha 0 and 4), kept as --workload c2.
 C2_ALPHAS = (0.0, 4.0)
 
@@ -155,44 +151,16 @@ def _mesh(cb, designation, level, first_layer, cache):
     return cache[key]
 
 
-@contextlib.contextmanager
-def _cluster_env(cluster: int):
-    """CFD_CLUSTER_SIZE set to `cluster` for the solves created inside."""
-    previous = os.environ.get("CFD_CLUSTER_SIZE")
-    os.environ["CFD_CLUSTER_SIZE"] = str(cluster)
-    try:
-        yield
-    finally:
-        if previous is None:
-            os.environ.pop("CFD_CLUSTER_SIZE", None)
-        else:
-            os.environ["CFD_CLUSTER_SIZE"] = previous
-
-
-def plain_cluster(designation: str, level: str) -> int:
-    """CTAs per solve of the plain form's batched polar. The 21 NACA 2412
-    points take 16-CTA clusters: a B200 holds 7 of those at once, so they fill
-    exactly three waves. The NACA 0012 trio runs beside them on the SMs those
-    clusters leave free, in a launch of its own: 768x192 on 8 CTAs, the two
-    smaller grids on 4. (All 24 on 16 CTAs take a fourth wave for the one
-    768x192 0012 solve: 18.9 against 17.9 ms per step.)"""
-    if designation == "2412":
-        return 16
-    return 8 if level == "fine" else 4
-
-
-def polar_solvers(cb, precision: int = 0, cluster: int | None = None, count: int | None = None):
+def polar_solvers(cb, precision: int = 0, count: int | None = None):
     """The 24 solves of the batched polar (or its first `count`, for a
     profiling capture of a smaller case), created on the device from the
-    uniform start. `cluster` fixes the CTAs per solve (the library's
-    CFD_CLUSTER_SIZE knob), else each solve takes `plain_cluster`'s."""
+    uniform start. The library's plan shares the GPU between them."""
     settings = cb.Settings.defaults(inflow_intensity=INTENSITY, inflow_viscosity_ratio=VISCOSITY_RATIO,
                                     precision=precision)
     meshes, solvers = {}, []
     for des, alpha, re, level, fl in POLAR[:count]:
         mesh = _mesh(cb, des, level, fl, meshes)
-        with _cluster_env(cluster if cluster is not None else plain_cluster(des, level)):
-            s = cb.SimpleSolver.create(mesh, cb.freestream_conditions(mesh, 1.0, alpha), settings)
+        s = cb.SimpleSolver.create(mesh, cb.freestream_conditions(mesh, 1.0, alpha), settings)
         s.set_turbulence_model(cb.MODEL_SST)
         s.initialise(*cb.uniform_field(mesh, 1.0, alpha, 1.0, re))
         solvers.append(s)
@@ -460,8 +428,7 @@ def run_ours(args) -> None:
     if c2:
         solvers = c2_solvers(cb, 1 if mixed_only else 0)
     else:
-        solvers = polar_solvers(cb, 1 if mixed_only else 0, MIXED_CLUSTER if mixed_only else None,
-                                args.solves)
+        solvers = polar_solvers(cb, 1 if mixed_only else 0, args.solves)
     batch = cb.Batch(solvers)
     cells = sum(s.mesh.cells for s in solvers)
     # A stream of our own: events, the L2 flush and the solver launches all go
@@ -490,7 +457,7 @@ def run_ours(args) -> None:
         batch.close()
         for s in solvers:
             s.close()
-        m_solvers = polar_solvers(cb, 1, MIXED_CLUSTER, args.solves)
+        m_solvers = polar_solvers(cb, 1, args.solves)
         m_batch = cb.Batch(m_solvers)
         m_ms, m_clocks = _timed_steps(torch, m_batch, handle, stream, flush, args.steps, args.warmup, dist)
         _, m_mon = m_batch.monitors()
@@ -516,10 +483,8 @@ def run_ours(args) -> None:
         config = c2_config() if c2 else polar_config({"solves": len(solvers), "cells": cells})
         if not c2 and args.solves is not None:
             config["workload"] += f" (only the first {len(solvers)} solves: a profiling case)"
-        config.update({"cluster_shape": shape, "cluster_sizes": sorted(
-                           {plain_cluster(d, lv) for d, _, _, lv, _ in POLAR[:args.solves]}, reverse=True)
-                       if not (c2 or mixed_only) else [shape[0]], "launch": "cuda graph" if args.graph else "direct",
-                       "cg_iterations_per_solve": cg})
+        config.update({"cluster_shape": shape, "launches_per_step": 1,
+                       "launch": "cuda graph" if args.graph else "direct", "cg_iterations_per_solve": cg})
         if mixed_only:
             config["precision"] = "mixed: FP64 assembly/state, FP32 sweeps and multigrid CG"
         line = {
@@ -530,7 +495,7 @@ def run_ours(args) -> None:
             "roofline": roofline,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
-            "gpu_launches": args.steps * len(config["cluster_sizes"]), "clocks": clocks, "finite": finite,
+            "gpu_launches": args.steps * config["launches_per_step"], "clocks": clocks, "finite": finite,
         }
         if mixed is not None:
             m_value = all_cells * args.steps / times[2]
@@ -742,8 +707,7 @@ def run_settled(args) -> None:
 
     out = {"workload": "settled: NACA0012 SST Re1e6 384x96 alpha 0/4, NACA2412 SST Re3e6 768x192 alpha 2/6",
            "rule": f"Cl moves < {cl_move:g} and Cd < {cd_move:g} over {window} iterations", "cap": cap}
-    with _cluster_env(MIXED_CLUSTER):
-        mixed = [make(k, 1) for k in range(len(cases))]
+    mixed = [make(k, 1) for k in range(len(cases))]
     for k, s in enumerate(mixed):
         des, alpha, re, level, fl = cases[k]
         s.initialise(*cb.uniform_field(s.mesh, 1.0, alpha, 1.0, re))

@@ -183,18 +183,12 @@ MeshKey keyOf(const cfd_request& r) {
           r.grid_vertical_chords};
 }
 
-/// Tuned launch shapes per (cells I, cells J, model, precision), shared by
-/// every engine of the process, so a grid runs with one shape (and one
-/// reduction order) whichever engine it is submitted to.
-std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_shapes;
-std::mutex g_shapesMutex;
-
 }  // namespace
 
 struct Engine {
   std::size_t budget{0};
   std::size_t used{0};
-  bool tuned{false};  // launch shapes: by grid size (false) or the occupancy tuner (true)
+  bool tuned{false};  // the launch shapes reported (launchShape)
   int chunk{32};
   int nextId{0};
   std::deque<Pending> queue;
@@ -270,8 +264,7 @@ struct Engine {
   Status start(const Pending& q, std::unique_ptr<Slot>* out) {
     std::unique_ptr<Solver> solver;
     if (Status st = makeSolver(q, &solver, q.warm.get()); st != CFD_OK) return st;
-    std::pair<int, int> shape;
-    if (Status st = tunedShape(q, *solver, &shape); st != CFD_OK) return st;
+    const std::pair<int, int> shape = launchShape(*solver);
     if (Status st = solver->setLaunchShape(shape.first, shape.second); st != CFD_OK) return st;
     auto slot = std::make_unique<Slot>();
     slot->id = q.id;
@@ -289,98 +282,17 @@ struct Engine {
     return ok();
   }
 
-  /// The launch shape of a grid: among clusters of 4, 8 and 16 CTAs of 512
-  /// threads, the one that gives the most solve-iterations per second on a
-  /// full GPU. Each candidate is timed the way the engine runs it when busy:
-  /// as many scratch solves of the grid (same model and precision, from their
-  /// uniform start) as the GPU holds at once for that shape
-  /// (cudaOccupancyMaxActiveClusters), in one launch over a descriptor table,
-  /// so the shared L2 and HBM traffic of that many resident solves is in the
-  /// measurement. Chosen once per (cells I, cells J, model, precision) and
-  /// kept for the process, so a request runs with the same shape, and gives
-  /// the same bits, whatever else is in the engine. CFD_ENGINE_TUNE=0 keeps the solver's
-  /// default shape.
-  Status tunedShape(const Pending& q, const Solver& s, std::pair<int, int>* out) {
-    if (!tuned || s.precision() == 0) {
-      // The plain form's launches share the GPU by a plan of their own
-      // (planWide), and its bits do not depend on it. The mixed form runs by
-      // grid size as a lone solve does, except that it takes clusters of at
-      // most 8 CTAs: its cost per iteration falls less than in proportion to
-      // the CTAs (the multigrid's coarse levels and its barriers do not
-      // shrink), so smaller clusters fit more solves per GPU (a 24-solve
-      // polar: 35 s on 8-CTA clusters, 37 s on 16, 43 s on 12).
-      int R = s.clusterSize();
-      if (s.precision() == 1) R = std::min(R, 8);
-      // A tuned engine reports one of the shapes that it times: for the plain
-      // form, whose launches none of them touch, the largest with a row per CTA.
-      if (tuned) {
-        for (R = 16; R > 4 && R > s.cellsJ();) R /= 2;
-      }
-      *out = {R, s.threads()};
-      return ok();
+  /// The launch shape a solve reports, by its grid alone: its launches share the
+  /// GPU by a plan (planWide), and its bits do not depend on how many CTAs it
+  /// gets. The mixed form reports at most 8 CTAs; a tuned engine the largest of
+  /// 4, 8 and 16 with a row per CTA.
+  std::pair<int, int> launchShape(const Solver& s) const {
+    int R = s.clusterSize();
+    if (s.precision() == 1) R = std::min(R, 8);
+    if (tuned) {
+      for (R = 16; R > 4 && R > s.cellsJ();) R /= 2;
     }
-    const auto key = std::make_tuple(s.cellsI(), s.cellsJ(), q.request.model, s.precision());
-    std::lock_guard<std::mutex> lock(g_shapesMutex);
-    if (auto it = g_shapes.find(key); it != g_shapes.end()) {
-      *out = it->second;
-      return ok();
-    }
-    std::pair<int, int> best{s.clusterSize(), s.threads()};
-    const char* env = std::getenv("CFD_ENGINE_TUNE");
-    if (env == nullptr || std::atoi(env) != 0) {
-      const int T = 512;
-      std::vector<std::pair<int, int>> candidates;  // (R, resident clusters)
-      int most = 0;
-      for (int R : {4, 8, 16}) {
-        if (R > s.cellsJ()) continue;
-        const int resident = maxActiveClusters(R, T, s.launchSmemBytes());
-        if (resident <= 0) continue;
-        candidates.emplace_back(R, resident);
-        most = std::max(most, resident);
-      }
-      // scratch solves, within a quarter of the engine's memory budget
-      const std::size_t each = std::max<std::size_t>(s.deviceBytes(), 1);
-      const int affordable = static_cast<int>(std::max<std::size_t>(1, budget / 4 / each));
-      const int copies = std::min({most, affordable, 40});
-      std::vector<std::unique_ptr<Solver>> probes;
-      for (int k = 0; k < copies; ++k) {
-        std::unique_ptr<Solver> p;
-        if (makeSolver(q, &p) != CFD_OK) break;
-        probes.push_back(std::move(p));
-      }
-      Instance* table = nullptr;
-      if (!probes.empty() &&
-          cudaMalloc(reinterpret_cast<void**>(&table), probes.size() * sizeof(Instance)) == cudaSuccess) {
-        std::vector<Instance> rows;
-        for (const auto& p : probes) rows.push_back(p->deviceView());
-        double bestScore = -1.0;
-        if (cudaMemcpy(table, rows.data(), rows.size() * sizeof(Instance), cudaMemcpyHostToDevice) ==
-            cudaSuccess) {
-          for (const auto& [R, resident] : candidates) {
-            const int n = std::min<int>(resident, static_cast<int>(probes.size()));
-            const int smem = probes[0]->launchSmemBytes();
-            if (launchSimple(table, n, R, T, 2, kStageEnd, -1.0, nullptr, smem) != CFD_OK) continue;
-            if (cudaDeviceSynchronize() != cudaSuccess) break;
-            const auto t0 = std::chrono::steady_clock::now();
-            if (launchSimple(table, n, R, T, 6, kStageEnd, -1.0, nullptr, smem) != CFD_OK) continue;
-            if (cudaDeviceSynchronize() != cudaSuccess) break;
-            const double perIteration =
-                std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() / 6.0;
-            // n solves advance one iteration per perIteration; a full GPU
-            // holds `resident` of them (n < resident only when memory is short)
-            const double score = n / perIteration * (static_cast<double>(resident) / n);
-            if (score > bestScore) {
-              bestScore = score;
-              best = {R, T};
-            }
-          }
-        }
-        cudaFree(table);
-      }
-    }
-    g_shapes[key] = best;
-    *out = best;
-    return ok();
+    return {R, s.threads()};
   }
 
   Status makeSolver(const Pending& q, std::unique_ptr<Solver>* out, const WarmStart* warm = nullptr) {
@@ -560,17 +472,17 @@ struct Engine {
   Status launchChunk() {
     const int n = static_cast<int>(active.size());
     if (Status st = reserve(n); st != CFD_OK) return st;
-    // group by launch shape (the plain form's solves in one launch per thread
-    // count, cluster size 0 here); table rows in slot order within each group
+    // one launch per form and thread count; table rows in slot order within each
     struct Launch {
-      int offset, count, R, T, smem;
+      bool mixed;
+      int offset, T;
       WidePlan plan;
       std::size_t planAt;  // its CTAs, then its list, in the plan area (bytes)
     };
-    std::map<std::pair<int, int>, std::vector<int>> groups;
+    std::map<std::pair<bool, int>, std::vector<int>> groups;
     for (int k = 0; k < n; ++k) {
       const Solver& s = *active[k]->solver;
-      groups[{(s.precision() == 0) ? 0 : s.clusterSize(), s.threads()}].push_back(k);
+      groups[{s.precision() == 1, s.threads()}].push_back(k);
     }
     std::vector<Instance> table(n);
     std::vector<Launch> launches;
@@ -578,7 +490,7 @@ struct Engine {
     const std::size_t per = static_cast<std::size_t>(chunk) * kMonSlots + 1;
     int offset = 0;
     for (const auto& [shape, members] : groups) {
-      int smem = 0;
+      std::vector<WideJob> jobs;
       for (std::size_t m = 0; m < members.size(); ++m) {
         const int k = members[m];
         Slot& s = *active[k];
@@ -589,19 +501,14 @@ struct Engine {
         I.stopTol = s.request.tolerance;
         I.iterLimit = std::max(1, std::min(chunk, s.request.max_iterations - s.iterations));
         table[offset + static_cast<int>(m)] = I;
-        if (shape.first > 0) smem = std::max(smem, s.solver->launchSmemBytes());
+        jobs.push_back(s.solver->wideJob());
       }
-      Launch launch{offset, static_cast<int>(members.size()), shape.first, shape.second, smem, {}, plans.size()};
-      if (shape.first == 0) {
-        std::vector<WideJob> jobs;
-        for (int k : members) jobs.push_back(active[k]->solver->wideJob());
-        launch.plan = planWide(jobs, shape.second);
-        const std::size_t ctas = launch.plan.ctas.size() * sizeof(WideCta);
-        const std::size_t list = launch.plan.list.size() * sizeof(int);
-        plans.resize(plans.size() + ((ctas + list + 15) & ~std::size_t{15}));
-        std::memcpy(plans.data() + launch.planAt, launch.plan.ctas.data(), ctas);
-        std::memcpy(plans.data() + launch.planAt + ctas, launch.plan.list.data(), list);
-      }
+      Launch launch{shape.first, offset, shape.second, planWide(jobs, shape.second), plans.size()};
+      const std::size_t ctas = launch.plan.ctas.size() * sizeof(WideCta);
+      const std::size_t list = launch.plan.list.size() * sizeof(int);
+      plans.resize(plans.size() + ((ctas + list + 15) & ~std::size_t{15}));
+      std::memcpy(plans.data() + launch.planAt, launch.plan.ctas.data(), ctas);
+      std::memcpy(plans.data() + launch.planAt + ctas, launch.plan.list.data(), list);
       launches.push_back(std::move(launch));
       offset += static_cast<int>(members.size());
     }
@@ -630,11 +537,10 @@ struct Engine {
     inFlightStreams.clear();
     for (std::size_t g = 0; g < launches.size(); ++g) {
       const Launch& l = launches[g];
-      const WideCta* ctas = (l.R == 0) ? reinterpret_cast<const WideCta*>(dPlans + l.planAt) : nullptr;
-      const Status st =
-          (l.R == 0) ? launchPlain(dTable + l.offset, l.plan, ctas, reinterpret_cast<const int*>(ctas + l.plan.ctas.size()),
-                                   l.T, chunk, kStageEnd, -1.0, streams[g])
-                     : launchSimple(dTable + l.offset, l.count, l.R, l.T, chunk, kStageEnd, -1.0, streams[g], l.smem);
+      const WideCta* ctas = reinterpret_cast<const WideCta*>(dPlans + l.planAt);
+      const int* list = reinterpret_cast<const int*>(ctas + l.plan.ctas.size());
+      const auto launch = l.mixed ? launchSimple : launchPlain;
+      const Status st = launch(dTable + l.offset, l.plan, ctas, list, l.T, chunk, kStageEnd, -1.0, streams[g]);
       if (st != CFD_OK) {
         waitForLaunches();
         return st;

@@ -59,6 +59,7 @@ constexpr int kFlagTwoReductionCg = 8;
 constexpr int kFlagBarrierSweeps = 32;
 constexpr int kFlagChainWaitTest = 64;  // tests only: a sweep also waits for a count nothing sets
 constexpr int kFlagSharedCg = 128;      // the plain CG in its form for any shape
+constexpr int kFlagPhasedCycle = 512;   // the mixed form's V-cycle with a phase per half sweep
 constexpr int kFlagHaloWaitTest = 256;  // tests only: a wait before the CG for a count nothing sets
 
 // Fault codes a launch leaves in iterations[1] (bits, or-ed together).
@@ -109,20 +110,23 @@ struct MgLevel {
   float *D, *S, *N, *W, *E;  // row coefficients (global memory)
   float* inv;                // 1 / D (0 where D = 0)
   float *x, *b;              // iterate and right-hand side (global memory)
+  float* y;                  // the iterate the way up leaves (global memory)
   const int* wake;           // partner column across j = 0, or -1
-  int smem;                  // byte offset of the level in shared memory when rank 0 runs it alone
+  int smem;                  // byte offset of the level in shared memory when every CTA runs it alike
   int smemWake;              // byte offset of its wake map there
+  unsigned perHalf;          // ceil(2^32 / half its columns, rounded up), for divisions
 };
 
 struct Multigrid {
   int levels;       // >= 1
-  int distributed;  // levels 0 .. distributed-1 are split over the cluster in row bands
-  int warpFrom;     // levels warpFrom .. levels-1 (64 cells or fewer) run on rank 0's warp 0
+  int distributed;  // levels 0 .. distributed-1 are split over the team
+  int warpFrom;     // levels warpFrom .. levels-1 (64 cells or fewer) run on a CTA's warp 0
   int pre, post, coarse;  // Gauss-Seidel sweeps (red-black) per level and on the coarsest
-  int smemBytes;    // shared memory of the levels rank 0 runs alone
+  int coarseBytes;  // the other levels at 32 bytes a cell (mixedRowsFit)
   MgLevel lv[kMaxMgLevels];
   // inner flexible-CG vectors, FP32, fine-grid layout
   float *r, *q, *e, *z0, *z1, *d0, *d1;
+  float* zs;  // the V-cycle's red start r / D
 };
 
 /// FP32 rows of one system in correction form, A delta = r: the mixed form
@@ -131,6 +135,13 @@ struct Rows32 {
   float *D, *S, *N, *W, *E;  // row coefficients
   float *r, *x;              // residual b - A phi (from FP64) and the correction
 };
+
+/// Messages of one k or omega sweep, and 16-byte words of its rows, at most for
+/// any number of threads: the padding of whole warps and of 3 cells to 4. Whole
+/// lines, so that the messages of a sweep are aligned to the pairs they are
+/// loaded in.
+__host__ __device__ inline long long chainSlots(int NI, int NJ) { return (NI + NI / 3 + 195LL) / 16 * 16 * NJ; }
+__host__ __device__ inline long long chainWords(int NI, int NJ) { return 2 * chainSlots(NI, NJ); }
 
 struct Instance {
   int NI, NJ, N;
@@ -174,12 +185,13 @@ struct Instance {
   double *kD, *kS, *kN, *kW, *kE, *kB;
   double *wD, *wS, *wN, *wW, *wE, *wB;
 
-  // ---- plain form: a wide team's scratch and the k and omega sweeps' layouts ----
+  // ---- the solve's team of CTAs: its scratch, and how many at most ----
   WideScratch wide;
+  int wideMost;
+  // ---- plain form: the k and omega sweeps' layouts, the CG's spill ----
   double *kC, *wC;           // packed sweep coefficients (row_sweeps.cuh)
   ulonglong2 *kV, *wV;       // packed sweep values, as messages
   double* spill;             // what the CG cannot hold on chip, by CTA
-  int wideMost;              // CTAs at most: one per CG unit, or the CTAs asked for
 
   // ---- outputs ----
   double* history;   // kMonSlots doubles per iteration of the launch
@@ -191,6 +203,8 @@ struct Instance {
   Rows32 mom;          // momentum rows (shared by u and v); r, x belong to u
   float *momRv, *momXv;  // v's residual and correction
   Rows32 tk, tw;       // k and omega
+  float4 *tkC, *twC;              // their rows for the chained sweeps (mixed_sweeps.cuh)
+  unsigned long long *tkV, *twV;  // the first two sweeps' values, as messages
 
   // ---- per-solve limits of a launch (batches and the engine) ----
   double stopTol;    // convergence tolerance when the launch gives none (< 0: none)

@@ -1,17 +1,15 @@
 // simple_kernel.cu - the SIMPLE outer iteration (laminar and k-omega SST) as
-// one persistent kernel per launch, one thread-block cluster per solve.
+// one persistent cooperative kernel per launch: the mixed FP32/FP64 form.
 //
-// Why a cluster per solve
-// -----------------------
-// A SIMPLE iteration is ~15 dependent phases, and the pressure CG inside it
-// adds two more per CG iteration (up to 200). Each phase is a 5-point stencil
-// or a reduction over 1e4-1e5 cells: far too little work to hide a kernel
-// launch or a grid-wide software barrier. A thread-block cluster gives the
-// CTAs of one solve a hardware barrier (barrier.cluster) with release/acquire
-// semantics, and distributed shared memory to exchange reduction partials,
-// so a phase boundary costs a fraction of a microsecond and no spin loop.
-// Independent solves occupy independent clusters; a batch of uneven solves is
-// a longer grid, one instance descriptor per cluster.
+// A SIMPLE iteration is ~15 dependent phases and a pressure solve of ~16
+// multigrid V-cycles, each a chain of small phases over the levels: 5-point
+// stencils and reductions over 1e4-1e5 cells, far too little work to hide a
+// kernel launch. The launch is cooperative and persistent: a solve has a team of
+// CTAs (wide_team.cuh), one per SM and up to the whole GPU, that meet in
+// barriers through L2, and a batch's solves share the launch by a plan. One
+// thread-block cluster of 16 CTAs per solve has cheaper barriers (0.7 us against
+// ~1.5) but leaves 132 SMs idle beside a lone solve: a phase over 768x192 cells
+// took 6 us there, and an outer iteration 2.6 ms.
 //
 // Arithmetic
 // ----------
@@ -26,10 +24,10 @@
 //     (j-faces before i-faces, ascending index; Mesh.cpp:138-170)
 //   Gauss-Seidel off-diagonal sum:               S, E, N, W
 //     (Mesh::cellFaces order, Mesh.cpp:172-181; LinearSystem.cpp:94-112)
-// Reductions (residual norms, CG dots, maxima) are deterministic: fixed-order
-// warp trees, then rank order across the cluster; every CTA derives the same
-// bits, so control flow that depends on them (CG exit, convergence) is
-// uniform. Gauss-Seidel is red-black instead of lexicographic: exact with the
+// Reductions (residual norms, CG dots, maxima) are deterministic: sums in an
+// order that depends on the grid alone (wide_team.cuh); every CTA derives the
+// same bits, so control flow that depends on them (CG exit, convergence) is
+// uniform, and a solve gives the same bits on any number of CTAs. Gauss-Seidel is red-black instead of lexicographic: exact with the
 // wake cut because cellsI is even on a C-grid, so partners across the cut have
 // opposite colours. It changes the iterate path but not the converged answer.
 
@@ -40,29 +38,26 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include <algorithm>
 #include <string>
 
 #include "common.hpp"
 #include "instance.hpp"
+#include "mixed_sweeps.cuh"
 #include "phases.cuh"
 #include "solver.hpp"
-#include "team.cuh"
+#include "wide_plan.hpp"
+#include "wide_team.cuh"
 
 namespace cfdb {
 namespace {
 
-/// cell(c, i, j) for every cell of the band.
-template <typename F>
-DEV void bandCells(const Instance& I, const Team& t, F&& cell) {
-  for (int c = t.c0 + t.tid; c < t.c1; c += t.T) cell(c, c % I.NI, c / I.NI);
-}
-
-/// Mixed form: one red-black colour pass of the momentum corrections
-/// (A du = ru, A dv = rv in FP32, shared rows). The last pass of the last
-/// sweep also adds both corrections to the FP64 velocities of every own cell:
-/// the other colour's corrections are final by then and no neighbour reads u
-/// or v during the sweeps.
-DEV void gsColourMixed(const Instance& I, Team& t, int colour, bool last) {
+/// One red-black colour pass of the momentum corrections (A du = ru, A dv = rv
+/// in FP32, shared rows). The last pass of the last sweep also adds both
+/// corrections to the FP64 velocities of every own cell: the other colour's
+/// corrections are final by then and no neighbour reads u or v during the
+/// sweeps. Cells in pairs as in the plain form's gsColour.
+DEV void gsColourMixed(const Instance& I, const WideTeam& t, int colour, bool last) {
   const Rows32& m = I.mom;
   const float* __restrict__ D = m.D;
   const float* __restrict__ cS = m.S;
@@ -74,30 +69,30 @@ DEV void gsColourMixed(const Instance& I, Team& t, int colour, bool last) {
   float* __restrict__ xu = m.x;
   float* __restrict__ xv = I.momXv;
   const int NI = I.NI;
-  const int H = (NI + 1) / 2;
-  const int j0 = t.c0 / NI;
-  const int slots = ((t.c1 - t.c0) / NI) * H;
+  const bool paired = (NI & 1) == 0;
+  const int first = paired ? t.c0 / 2 : t.c0, end = paired ? t.c1 / 2 : t.c1;
   constexpr int kPair = 2;
-  // only the colour's cells (i = 2k + ((j + colour) & 1)), two at a time,
-  // every load first; missing neighbours are clamped to the cell and their
-  // terms left out as before, so the sums are unchanged
-  for (int q0 = t.tid; q0 < slots; q0 += kPair * t.T) {
+  for (int q0 = first + t.tid; q0 < end; q0 += kPair * t.T) {
     int cell[kPair], nb[kPair][4];
     bool ok[kPair];
     float d[kPair], a[kPair][4], b1[kPair], b2[kPair], x1[kPair][4], x2[kPair][4];
 #pragma unroll
     for (int e = 0; e < kPair; ++e) {
-      const int q = min(q0 + e * t.T, slots - 1);
-      const int j = j0 + q / H;
-      const int i = 2 * (q % H) + ((j + colour) & 1);
-      ok[e] = (q0 + e * t.T < slots) && i < NI;
-      const int ic = min(i, NI - 1);
-      const int c = j * NI + ic;
+      const int q = min(q0 + e * t.T, end - 1);
+      int c = paired ? 2 * q : q;
+      const int j = c / NI;
+      int i = c - j * NI;
+      const int shift = (i + j + colour) & 1;  // 1: the cell itself has the other colour
+      ok[e] = q0 + e * t.T < end && (paired || shift == 0);
+      if (paired) {
+        c += shift;
+        i += shift;
+      }
       cell[e] = c;
-      nb[e][0] = across(I, c, ic, j, 0);  // S
-      nb[e][1] = across(I, c, ic, j, 3);  // E
-      nb[e][2] = across(I, c, ic, j, 1);  // N
-      nb[e][3] = across(I, c, ic, j, 2);  // W
+      nb[e][0] = across(I, c, i, j, 0);  // S
+      nb[e][1] = across(I, c, i, j, 3);  // E
+      nb[e][2] = across(I, c, i, j, 1);  // N
+      nb[e][3] = across(I, c, i, j, 2);  // W
       d[e] = D[c];
       a[e][0] = cS[c];
       a[e][1] = cE[c];
@@ -128,7 +123,7 @@ DEV void gsColourMixed(const Instance& I, Team& t, int colour, bool last) {
     }
   }
   if (last) {
-    // the corrections of the whole band (this CTA wrote all of them) onto u, v
+    // the corrections of the CTA's cells (it wrote all of them) onto u, v
     __syncthreads();
     for (int c = t.c0 + t.tid; c < t.c1; c += t.T) {
       I.u[c] += static_cast<double>(xu[c]);
@@ -137,560 +132,17 @@ DEV void gsColourMixed(const Instance& I, Team& t, int colour, bool last) {
   }
 }
 
-/// Lexicographic Gauss-Seidel, executed as wavefronts: cells with i + j = d
-/// for d = 0, 1, ... Within a wavefront no cell depends on another; every
-/// cell sees its S and W neighbours already updated and its N and E
-/// neighbours not yet, exactly as in cell-index order. Across the wake cut,
-/// the partner (NI-1-i, 0) of (i, 0) lies on an earlier wavefront exactly when
-/// its cell index is smaller, so that coupling is reproduced too. The result
-/// is the reference's sweep (LinearSystem.cpp:77-116) to the last bit.
-///
-/// One CTA runs one system: rank 0 sweeps x1, rank 1 (or rank 0 again when
-/// the cluster has one CTA) sweeps x2. The caller ends with a cluster barrier.
-DEV void gsWavefrontSweeps(const Instance& I, Team& t, int sweeps, const double* D,
-                           const double* cS, const double* cN, const double* cW,
-                           const double* cE, const double* b1, double* x1, const double* D2,
-                           const double* cS2, const double* cN2, const double* cW2,
-                           const double* cE2, const double* b2, double* x2) {
-  const bool one = (t.R == 1);
-  if (!one && t.rank > 1) return;
-  const int fronts = I.NI + I.NJ - 1;
-  for (int sweep = 0; sweep < sweeps; ++sweep) {
-    for (int d = 0; d < fronts; ++d) {
-      const int jLo = (d - (I.NI - 1) > 0) ? d - (I.NI - 1) : 0;
-      const int jHi = (d < I.NJ - 1) ? d : I.NJ - 1;
-      const int count = jHi - jLo + 1;
-      const int work = one ? 2 * count : count;
-      for (int k = t.tid; k < work; k += t.T) {
-        const bool second = one ? (k >= count) : (t.rank == 1);
-        const int j = jLo + (one ? (k % count) : k);
-        const int i = d - j;
-        const int c = j * I.NI + i;
-        const double* Dv = second ? D2 : D;
-        const double dd = Dv[c];
-        if (!(fabs(dd) > 0.0)) continue;
-        const double* aS = second ? cS2 : cS;
-        const double* aN = second ? cN2 : cN;
-        const double* aW = second ? cW2 : cW;
-        const double* aE = second ? cE2 : cE;
-        double* x = second ? x2 : x1;
-        const double* b = second ? b2 : b1;
-        const int nS = across(I, c, i, j, 0), nE = across(I, c, i, j, 3);
-        const int nN = across(I, c, i, j, 1), nW = across(I, c, i, j, 2);
-        double off = 0.0;
-        if (nS >= 0) off += aS[c] * x[nS];
-        if (nE >= 0) off += aE[c] * x[nE];
-        if (nN >= 0) off += aN[c] * x[nN];
-        if (nW >= 0) off += aW[c] * x[nW];
-        x[c] = (b[c] - off) / dd;
-      }
-      __syncthreads();
-    }
-  }
-}
-
-/// Block-wide exclusive scan of affine maps x -> p + q x composed in thread
-/// order: each thread passes the composition (p, q) of its own elements
-/// (identity (0, 1) if none) and receives the composition of all elements of
-/// lower threads. Uses sc[0 .. 2*warps) of shared memory; two __syncthreads.
-template <typename T>
-DEV void blockAffineExclusiveScan(T& p, T& q, T* sc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nwarps = (blockDim.x + 31) >> 5;
-  // inclusive scan within the warp (later maps applied after earlier ones)
-  T ip = p, iq = q;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const T pp = __shfl_up_sync(0xffffffffu, ip, off);
-    const T qq = __shfl_up_sync(0xffffffffu, iq, off);
-    if (lane >= off) {
-      ip = ip + iq * pp;
-      iq = iq * qq;
-    }
-  }
-  // exclusive within the warp
-  T ep = __shfl_up_sync(0xffffffffu, ip, 1);
-  T eq = __shfl_up_sync(0xffffffffu, iq, 1);
-  if (lane == 0) {
-    ep = T(0);
-    eq = T(1);
-  }
-  if (lane == 31) {
-    sc[2 * warp] = ip;
-    sc[2 * warp + 1] = iq;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    T wp = (lane < nwarps) ? sc[2 * lane] : T(0);
-    T wq = (lane < nwarps) ? sc[2 * lane + 1] : T(1);
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const T pp = __shfl_up_sync(0xffffffffu, wp, off);
-      const T qq = __shfl_up_sync(0xffffffffu, wq, off);
-      if (lane >= off) {
-        wp = wp + wq * pp;
-        wq = wq * qq;
-      }
-    }
-    T xp = __shfl_up_sync(0xffffffffu, wp, 1);
-    T xq = __shfl_up_sync(0xffffffffu, wq, 1);
-    if (lane == 0) {
-      xp = T(0);
-      xq = T(1);
-    }
-    if (lane < nwarps) {
-      sc[2 * lane] = xp;
-      sc[2 * lane + 1] = xq;
-    }
-  }
-  __syncthreads();
-  // earlier warps first, then the earlier lanes of this warp
-  const T wp = sc[2 * warp], wq = sc[2 * warp + 1];
-  p = ep + eq * wp;
-  q = eq * wq;
-}
-
-/// One row of a lexicographic Gauss-Seidel sweep (LinearSystem.cpp:77-116).
-/// With row j-1 already updated and row j+1 and the east neighbours still
-/// holding their old values, the cell-order update of row j is the
-/// first-order recurrence x_i = p_i + q_i x_{i-1},
-///   p_i = (b_i - aS x_S - aE x_E - aN x_N) / a_P,  q_i = -aW / a_P,
-/// solved by a block-wide scan. Row 0 is split in two: the wake-cut partner
-/// (NI-1-i, 0) of (i, 0) comes later in the row for i < NI/2 (old value) and
-/// earlier for i >= NI/2 (new value), so the second half is solved after the
-/// first. A cell with a_P = 0 keeps its value (p = x, q = 0). This is the
-/// reference's sweep map; only the rounding differs from cell-by-cell order.
-///
-/// Run by every thread of one CTA; rowPrev holds row j-1's new values,
-/// oldRow and northRow rows j and j+1 as the previous sweep left them (the
-/// unknowns themselves, or a copy). Needs NI <= 8 * blockDim.x. Leaves row
-/// j's new values in rowNew and ends with a barrier; the caller publishes.
-template <typename T>
-struct SysView {
-  const T *D, *S, *N, *W, *E, *b;
-  T* x;
-};
-
-/// The row solve for any cells per thread (up to 8), loading as it goes.
-template <typename T>
-DEV void gsRowSolveAny(const Instance& I, int j, const SysView<T>& y, const T* oldRow, const T* northRow, T* rowNew,
-                       const T* rowPrev, T* sc) {
-  const T *D = y.D, *cS = y.S, *cN = y.N, *cW = y.W, *cE = y.E, *b = y.b;
-  const int NI = I.NI, NJ = I.NJ;
-  const int nt = blockDim.x;
-  const int per = (NI + nt - 1) / nt;  // contiguous cells per thread
-  const int i0 = threadIdx.x * per;
-  const int segments = (j == 0) ? 2 : 1;
-  T carry = T(0);
-  for (int seg = 0; seg < segments; ++seg) {
-    const int lo = (segments == 1) ? 0 : (seg == 0 ? 0 : NI / 2);
-    const int hi = (segments == 1) ? NI : (seg == 0 ? NI / 2 : NI);
-    T pv[8], qv[8];
-    T P = T(0), Q = T(1);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      pv[e] = T(0);
-      qv[e] = T(1);
-      const int i = i0 + e;
-      if (e >= per || i < lo || i >= hi) continue;
-      const int c = j * NI + i;
-      const T d = D[c];
-      if (!(fabs(d) > T(0))) {
-        pv[e] = oldRow[i];
-        qv[e] = T(0);
-      } else {
-        T off = T(0);
-        if (j > 0) {
-          off += cS[c] * rowPrev[i];
-        } else {
-          const int a = I.acrossJ0[i];
-          if (a >= 0) off += cS[c] * ((a < i) ? rowNew[a] : oldRow[a]);
-        }
-        if (i < NI - 1) off += cE[c] * oldRow[i + 1];
-        if (j < NJ - 1) off += cN[c] * northRow[i];
-        pv[e] = (b[c] - off) / d;
-        qv[e] = (i > 0) ? -cW[c] / d : T(0);
-      }
-      P = pv[e] + qv[e] * P;
-      Q = qv[e] * Q;
-    }
-    blockAffineExclusiveScan(P, Q, sc);
-    T xv = P + Q * carry;  // value entering this thread's chunk
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int i = i0 + e;
-      if (e >= per || i < lo || i >= hi) continue;
-      xv = pv[e] + qv[e] * xv;
-      rowNew[i] = xv;
-    }
-    __syncthreads();
-    if (hi > lo) carry = rowNew[hi - 1];
-  }
-}
-
-/// The row solve for at most MAXPER cells per thread. Every operand of the
-/// thread's cells is loaded before any is used (indices clamped into the row;
-/// values of cells outside it are never used), so the loads overlap instead
-/// of waiting behind the branch on the diagonal.
-template <typename T, int MAXPER>
-DEV void gsRowSolveN(const Instance& I, int j, const SysView<T>& y, const T* oldRow, const T* northRow, T* rowNew,
-                     const T* rowPrev, T* sc) {
-  const T* __restrict__ D = y.D;
-  const T* __restrict__ cS = y.S;
-  const T* __restrict__ cN = y.N;
-  const T* __restrict__ cW = y.W;
-  const T* __restrict__ cE = y.E;
-  const T* __restrict__ b = y.b;
-  const int NI = I.NI, NJ = I.NJ;
-  const int nt = blockDim.x;
-  const int per = (NI + nt - 1) / nt;  // contiguous cells per thread
-  const int i0 = threadIdx.x * per;
-  const bool hasNorth = j < NJ - 1;
-  const long long rowBase = static_cast<long long>(j) * NI;
-  T dv[MAXPER], sv[MAXPER], ev[MAXPER], nv[MAXPER], wv[MAXPER], bv[MAXPER];
-  T oldI[MAXPER], oldE[MAXPER], northI[MAXPER], prevI[MAXPER];
-  int wake[MAXPER];
-#pragma unroll
-  for (int e = 0; e < MAXPER; ++e) {
-    const int i = min(i0 + e, NI - 1);
-    const long long c = rowBase + i;
-    dv[e] = D[c];
-    sv[e] = cS[c];
-    ev[e] = cE[c];
-    nv[e] = cN[c];
-    wv[e] = cW[c];
-    bv[e] = b[c];
-    oldI[e] = oldRow[i];
-    oldE[e] = oldRow[min(i + 1, NI - 1)];
-    northI[e] = hasNorth ? northRow[i] : T(0);
-    prevI[e] = (j > 0) ? rowPrev[i] : T(0);
-    wake[e] = (j == 0) ? I.acrossJ0[i] : -1;
-  }
-  const int segments = (j == 0) ? 2 : 1;
-  T carry = T(0);
-  for (int seg = 0; seg < segments; ++seg) {
-    const int lo = (segments == 1) ? 0 : (seg == 0 ? 0 : NI / 2);
-    const int hi = (segments == 1) ? NI : (seg == 0 ? NI / 2 : NI);
-    T pv[MAXPER], qv[MAXPER];
-    T P = T(0), Q = T(1);
-#pragma unroll
-    for (int e = 0; e < MAXPER; ++e) {
-      pv[e] = T(0);
-      qv[e] = T(1);
-      const int i = i0 + e;
-      if (e >= per || i < lo || i >= hi) continue;
-      const T d = dv[e];
-      if (!(fabs(d) > T(0))) {
-        pv[e] = oldI[e];
-        qv[e] = T(0);
-      } else {
-        T off = T(0);
-        if (j > 0) {
-          off += sv[e] * prevI[e];
-        } else {
-          const int a = wake[e];
-          if (a >= 0) off += sv[e] * ((a < i) ? rowNew[a] : oldRow[a]);
-        }
-        if (i < NI - 1) off += ev[e] * oldE[e];
-        if (hasNorth) off += nv[e] * northI[e];
-        pv[e] = (bv[e] - off) / d;
-        qv[e] = (i > 0) ? -wv[e] / d : T(0);
-      }
-      P = pv[e] + qv[e] * P;
-      Q = qv[e] * Q;
-    }
-    blockAffineExclusiveScan(P, Q, sc);
-    T xv = P + Q * carry;  // value entering this thread's chunk
-#pragma unroll
-    for (int e = 0; e < MAXPER; ++e) {
-      const int i = i0 + e;
-      if (e >= per || i < lo || i >= hi) continue;
-      xv = pv[e] + qv[e] * xv;
-      rowNew[i] = xv;
-    }
-    __syncthreads();
-    if (hi > lo) carry = rowNew[hi - 1];
-  }
-}
-
-template <typename T>
-DEV void gsRowSolve(const Instance& I, int j, const SysView<T>& y, const T* oldRow, const T* northRow, T* rowNew,
-                    const T* rowPrev, T* sc) {
-  if (I.NI <= 2 * static_cast<int>(blockDim.x)) {
-    gsRowSolveN<T, 2>(I, j, y, oldRow, northRow, rowNew, rowPrev, sc);
-  } else {
-    gsRowSolveAny(I, j, y, oldRow, northRow, rowNew, rowPrev, sc);
-  }
-}
-
-/// One row of the sweep on the unknowns in place: solve from the unknowns,
-/// then publish row j to global memory (east/north reads of later rows and
-/// the next sweep) and to rowPrev (the south values of row j + 1). Every
-/// read of this row's old values and of rowPrev happened before the scan's
-/// barriers. Ends without a barrier (the caller synchronises before the
-/// next row).
-template <typename T>
-DEV void gsRow(const Instance& I, int j, const SysView<T>& y, T* rowNew, T* rowPrev, T* sc) {
-  T* x = y.x;
-  const int NI = I.NI;
-  gsRowSolve(I, j, y, x + static_cast<long long>(j) * NI, x + static_cast<long long>(j + 1) * NI, rowNew, rowPrev,
-             sc);
-  for (int i = threadIdx.x; i < NI; i += blockDim.x) {
-    x[j * NI + i] = rowNew[i];
-    rowPrev[i] = rowNew[i];
-  }
-}
-
-/// `sweeps` lexicographic sweeps of one system by one CTA, row after row.
-/// Needs 2 * NI + 2 * warps doubles of shared memory.
-template <typename T>
-DEV void gsRowScanSweeps(const Instance& I, int sweeps, const SysView<T>& y, T* smem) {
-  T* rowNew = smem;          // row j, new values
-  T* rowPrev = smem + I.NI;  // row j - 1, new values
-  T* sc = smem + 2 * I.NI;
-  for (int sweep = 0; sweep < sweeps; ++sweep) {
-    for (int j = 0; j < I.NJ; ++j) {
-      gsRow(I, j, y, rowNew, rowPrev, sc);
-      prefetchRow(I, (j + 1 < I.NJ) ? j + 1 : 0, y);
-      __syncthreads();
-    }
-  }
-}
-
-/// The k and omega sweeps as a software pipeline over 2 * sweeps CTAs: CTA
-/// (eq, s) runs sweep s of equation eq (0: k, 1: omega) and at step t updates
-/// row t - 2s. Sweep s reads row j+1 as left by sweep s-1 (done at step t-1),
-/// row j as left by sweep s-1 (step t-2) and row j-1 from its own previous
-/// step, so every value is the one the sequential order would use, and no row
-/// is written at the step it is read by another sweep (sweep s-1 writes row
-/// j+2, sweep s+1 row j-2). Every CTA of the cluster joins each step's
-/// barrier. Same arithmetic as gsRowScanSweeps, NJ + 2 (sweeps - 1) steps
-/// instead of sweeps * NJ.
-/// Bring row j's coefficients and right-hand side (fixed during the sweeps)
-/// towards this SM's L1 ahead of its scan, one prefetch per 128-byte line,
-/// spread over the CTA's threads. A hint only: it changes no value.
-template <typename T>
-DEV void prefetchRow(const Instance& I, int j, const SysView<T>& y) {
-  if (j < 0 || j >= I.NJ) return;
-  constexpr int perLine = 128 / static_cast<int>(sizeof(T));
-  const int lines = (I.NI + perLine - 1) / perLine;
-  const T* arrays[6] = {y.D, y.S, y.N, y.W, y.E, y.b};
-  for (int q = threadIdx.x; q < 6 * lines; q += blockDim.x) {
-    const T* line = arrays[q / lines] + static_cast<long long>(j) * I.NI + (q % lines) * perLine;
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(line));
-  }
-}
-
-template <typename T>
-DEV void gsRowScanPipelined(const Instance& I, Team& t, int sweeps, const SysView<T>& kSys,
-                            const SysView<T>& wSys, T* smem) {
-  const int role = static_cast<int>(t.rank);
-  const bool active = role < 2 * sweeps;
-  const bool omega = active && role >= sweeps;
-  const int s = active ? role % sweeps : 0;
-  const SysView<T>& y = omega ? wSys : kSys;
-  T* rowNew = smem;
-  T* rowPrev = smem + I.NI;
-  T* sc = smem + 2 * I.NI;
-  const int steps = I.NJ + 2 * (sweeps - 1);
-  if (active) prefetchRow(I, -2 * s, y);
-  for (int step = 0; step < steps; ++step) {
-    const int j = step - 2 * s;
-    if (active && j >= 0 && j < I.NJ) gsRow(I, j, y, rowNew, rowPrev, sc);
-    if (active) prefetchRow(I, j + 1, y);  // the next step's row, over the barrier
-    t.cl.sync();
-  }
-}
-
-// ---- the chained k/omega sweeps: rows pushed to the next stage ------------------
-
-constexpr int kChainSlots = 4;                    // ring rows per stage (Shared::chainBar)
-constexpr long long kChainSpinLimit = 1LL << 24;  // polls before a wait gives up (~0.3 s)
-
-/// Shared memory of gsRowScanChained, in elements of T.
-__host__ __device__ inline long long chainSmemElems(int NI) { return (2LL + kChainSlots) * NI + 64; }
-
-DEV unsigned smemAddr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
-/// The shared::cluster address of this CTA's shared-memory address `a` in CTA `rank`.
-DEV unsigned clusterAddr(unsigned a, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-DEV void mbarInit(unsigned long long* b) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(b)) : "memory");
-}
-/// This CTA's one arrival on the barrier's current phase, expecting `bytes`.
-DEV void mbarArm(unsigned long long* b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddr(b)), "r"(bytes) : "memory");
-}
-/// Whether the phase of parity `parity` has completed (acquire, cluster scope).
-DEV bool mbarDone(const unsigned long long* b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(ok)
-      : "r"(smemAddr(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-/// Store v into another CTA's shared memory; its mbarrier counts the bytes.
-DEV void pushRemote(unsigned dst, float v, unsigned bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(v),
-               "r"(bar)
-               : "memory");
-}
-DEV unsigned loadRelaxedCluster(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.relaxed.cluster.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-DEV void storeRelaxedCluster(unsigned* p, unsigned v) {
-  asm volatile("st.relaxed.cluster.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-/// Kernel start: the ring barriers armed for the first kChainSlots rows (of
-/// `rowBytes` each) and the release count at zero. Made visible to the peers and
-/// the async proxy before the kernel's first cluster barrier.
-DEV void chainSetup(Shared& sh, unsigned rowBytes) {
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < kChainSlots; ++k) {
-      mbarInit(&sh.chainBar[k]);
-      mbarArm(&sh.chainBar[k], rowBytes);
-    }
-    sh.chainAck = 0u;
-    sh.chainNever = 0u;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-}
-
-/// The k and omega sweeps as a chain of 2 * sweeps CTAs, CTA (eq, s) running
-/// sweep s of equation eq (0: k, 1: omega), without cluster-wide barriers.
-/// Row g (counted over the launch: g = base + j, base = calls so far x NJ)
-/// travels through ring slot g % kChainSlots: as a stage finishes a row it
-/// pushes the values into the next stage's slot with st.async, whose bytes
-/// complete that slot's mbarrier; the next stage waits for rows j and j+1
-/// (its old own-row and north values), reads them from its own shared
-/// memory, and when done with row j re-arms the slot for row g + kChainSlots
-/// and writes g + 1 into its producer's release count, which the producer
-/// waits for before pushing into that slot again. The first stage reads the
-/// unknowns, the last writes them, so the values and the arithmetic are
-/// those of gsRowScanSweeps (the same bits). A wait that gives up sets
-/// kFaultChainWait in the launch's fault word and the call waits no more, so
-/// the launch always ends (and reports the fault). With `waitTest` the second
-/// stage also waits once per call for a count nothing sets, which gives up
-/// and reports the fault while the rows still flow as usual.
-template <typename T>
-DEV void gsRowScanChained(const Instance& I, Team& t, Shared& sh, int sweeps, const SysView<T>& kSys,
-                          const SysView<T>& wSys, T* smem, unsigned base, bool waitTest) {
-  const int role = static_cast<int>(t.rank);
-  if (role >= 2 * sweeps) return;
-  const int s = role % sweeps;
-  const bool hasProducer = s > 0, hasConsumer = s < sweeps - 1;
-  const SysView<T>& y = (role >= sweeps) ? wSys : kSys;
-  const int NI = I.NI, NJ = I.NJ;
-  const unsigned rowBytes = static_cast<unsigned>(NI * sizeof(T));
-  T* rowNew = smem;
-  T* rowPrev = smem + NI;
-  T* sc = smem + 2 * NI;
-  T* ring = smem + 2 * NI + 64;
-  const unsigned nextRing = hasConsumer ? clusterAddr(smemAddr(ring), role + 1) : 0u;
-  const unsigned nextBar = hasConsumer ? clusterAddr(smemAddr(&sh.chainBar[0]), role + 1) : 0u;
-  unsigned* producerAck = hasProducer ? t.cl.map_shared_rank(&sh.chainAck, role - 1) : nullptr;
-  T* x = y.x;
-  bool faulted = false;  // a wait of this call gave up: the call waits no more
-  prefetchRow(I, 0, y);
-  for (int j = 0; j < NJ; ++j) {
-    const unsigned g = base + static_cast<unsigned>(j);
-    const unsigned slot = g % kChainSlots, slotN = (g + 1) % kChainSlots;
-    if (threadIdx.x == 0 && waitTest && s == 1 && j == 0) {
-      // test: once per call the second stage waits for a count nothing sets
-      long long spins = 0;
-      while (loadRelaxedCluster(&sh.chainNever) == 0u && ++spins <= kChainSpinLimit) {
-      }
-      if (spins > kChainSpinLimit) atomicOr(I.iterations + 1, kFaultChainWait);
-    }
-    if (threadIdx.x == 0 && !faulted) {
-      long long spins = 0;
-      for (;;) {
-        bool ready = true;
-        if (hasProducer) {
-          ready = mbarDone(&sh.chainBar[slot], (g / kChainSlots) & 1u) &&
-                  (j + 1 >= NJ || mbarDone(&sh.chainBar[slotN], ((g + 1) / kChainSlots) & 1u));
-        }
-        // the next stage has released the row this slot held (g - kChainSlots)
-        if (ready && hasConsumer && g + 1 >= kChainSlots) {
-          ready = loadRelaxedCluster(&sh.chainAck) >= g + 1 - kChainSlots;
-        }
-        if (ready) break;
-        if (++spins > kChainSpinLimit) {
-          atomicOr(I.iterations + 1, kFaultChainWait);
-          faulted = true;
-          break;
-        }
-      }
-    }
-    __syncthreads();
-    const long long row = static_cast<long long>(j) * NI;
-    const T* oldRow = hasProducer ? ring + slot * NI : x + row;
-    const T* northRow = hasProducer ? ring + slotN * NI : x + row + NI;
-    gsRowSolve(I, j, y, oldRow, northRow, rowNew, rowPrev, sc);
-    // every read of ring slot `slot` happened before gsRowSolve's barriers
-    if (threadIdx.x == 0 && hasProducer) {
-      mbarArm(&sh.chainBar[slot], rowBytes);  // for row g + kChainSlots
-      storeRelaxedCluster(producerAck, g + 1);
-    }
-    for (int i = threadIdx.x; i < NI; i += blockDim.x) {
-      const T v = rowNew[i];
-      rowPrev[i] = v;
-      if (hasConsumer) {
-        pushRemote(nextRing + (slot * NI + i) * static_cast<unsigned>(sizeof(T)), v, nextBar + slot * 8u);
-      } else {
-        x[row + i] = v;
-      }
-    }
-    prefetchRow(I, j + 1, y);
-    if (!hasProducer && j + 2 < NJ) {
-      // the first stage's next north row (the unknowns, fixed until the last stage writes them)
-      constexpr int perLine = 128 / static_cast<int>(sizeof(T));
-      for (int q = threadIdx.x; q * perLine < NI; q += blockDim.x) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(x + row + 2 * NI + q * perLine));
-      }
-    }
-    // the next row's wait ends in a barrier, which orders these rowPrev
-    // writes and rowNew reads before the next row's use of them
-  }
-}
-
-DEV SysView<float> correctionSystem(const Rows32& r) { return SysView<float>{r.D, r.S, r.N, r.W, r.E, r.r, r.x}; }
-
 #include "pressure_mg.cuh"
-
-}  // namespace
 
 // ---- the kernel -----------------------------------------------------------------
 
-/// Run `iterations` outer iterations (or fewer: `stopStage` ends the first
-/// iteration early; `tolerance` >= 0 stops at convergence or divergence as
-/// SolverWorker does, SolverWorker.cpp:164-185). One cluster per instance.
-__global__ void __launch_bounds__(512, 1)
-simpleKernel(const Instance* __restrict__ instances, int iterations, int stopStage, double tolerance,
-             int smemBytes, int flags) {
-  __shared__ Shared sh;
-  extern __shared__ double dyn[];
-  Team t{cg::this_cluster(), 0, 0, 0, 0, 0, 0, 0};
-  t.rank = t.cl.block_rank();
-  t.R = t.cl.num_blocks();
-  t.tid = threadIdx.x;
-  t.T = blockDim.x;
-  const Instance& I = instances[blockIdx.x / t.R];
-  // Each CTA owns a band of whole rows; the same split in every phase.
-  t.c0 = I.NI * ((I.NJ * static_cast<int>(t.rank)) / static_cast<int>(t.R));
-  t.c1 = I.NI * ((I.NJ * (static_cast<int>(t.rank) + 1)) / static_cast<int>(t.R));
+/// One solve of a launch, by every thread of its team: `iterations` outer
+/// iterations or fewer (`stopStage` ends the first early; `tolerance` >= 0 stops
+/// at convergence or divergence as SolverWorker does, SolverWorker.cpp:164-185).
+DEV void mixedSolve(const Instance& I, WideTeam& t, int iterations, int stopStage, double tolerance, int smemBytes,
+                    int flags) {
   const bool sst = (I.model == 2);
   const bool leader = (t.rank == 0 && t.tid == 0);
-  // Ordered before any peer's access by the first cluster barrier below.
-  chainSetup(sh, static_cast<unsigned>(I.NI) * 4u);
   if (leader) I.iterations[1] = 0;
 
   int done = 0;
@@ -711,9 +163,8 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
     // 1. face values and gradients; velocity scale.
     {
       double v1[1] = {0.0};
-      const int op[1] = {kMax};
-      bandCells(I, t, [&](int c, int i, int j) { gradientsCell(I, c, i, j, v1[0]); });
-      teamReduce(t, sh, v1, op);
+      wideCells(t, [&](int c, int i, int j) { gradientsCell(I, c, i, j, v1[0]); });
+      wideMax(t, v1);
       double scale = smax(0.0, v1[0]);
       if (!(scale > 0.0)) scale = 1.0;
       momentumX = scale;  // held until the residuals are known
@@ -723,10 +174,10 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
 
     // 2. momentum assembly + relaxation + residuals (u and v together).
     {
-      double v3[3] = {0.0, 0.0, 0.0};
-      const int op[3] = {kSum, kSum, kSum};
-      bandCells(I, t, [&](int c, int i, int j) { momentumCell<true>(I, c, i, j, v3[0], v3[1], v3[2]); });
-      teamReduce(t, sh, v3, op);
+      double v3[3];
+      wideSums(t, v3, [&](int c, int i, int j, double (&acc)[3]) {
+        momentumCell<true>(I, c, i, j, acc[0], acc[1], acc[2]);
+      });
       const double scale = v3[2] * momentumX;
       momentumX = v3[0] / smax(scale, kTinySolver);
       momentumY = v3[1] / smax(scale, kTinySolver);
@@ -739,60 +190,59 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
     for (int sweep = 0; sweep < I.sweeps; ++sweep) {
       for (int colour = 0; colour < 2; ++colour) {
         gsColourMixed(I, t, colour, sweep == I.sweeps - 1 && colour == 1);
-        t.cl.sync();
+        wideBarrier(t);
       }
     }
     if (stopStage == kStageMomentumSolve) { done = it + 1; break; }
 
     // 4. Rhie-Chow face fluxes.
-    bandCells(I, t, [&](int c, int i, int j) { rhieChowCell(I, c, i, j); });
-    t.cl.sync();
+    wideCells(t, [&](int c, int i, int j) { rhieChowCell(I, c, i, j); });
+    wideBarrier(t);
     if (stopStage == kStageRhieChow) { done = it + 1; break; }
 
     bool stopped = false;
     const int passes = (I.nCorr > 1) ? I.nCorr : 1;
     for (int pass = 0; pass < passes && !stopped; ++pass) {
-      // 5. pressure-correction assembly; CG start (x = 0, r = b, d = z = M^-1 r).
-      double v2[2] = {0.0, 0.0};
-      const int op2[2] = {kSum, kSum};
-      bandCells(I, t, [&](int c, int i, int j) { pressureAssemblyCell(I, c, i, j, v2[0], v2[1]); });
-      teamReduce(t, sh, v2, op2);
+      // 5. pressure-correction assembly; the solve starts from x = 0, r = b.
+      double v2[2];
+      wideSums(t, v2, [&](int c, int i, int j, double (&acc)[2]) {
+        pressureAssemblyCell(I, c, i, j, acc[0], acc[1]);
+      });
       if (pass == 0) {
         continuity = v2[0] / I.refMassFlow;
         note(kMonMassImbalance, v2[0]);
         note(kMonContinuity, continuity);
       }
       const double mean = I.hasPRef ? 0.0 : v2[1] / static_cast<double>(I.N);
-      double init[2] = {0.0, 0.0};
-      for (int c = t.c0 + t.tid; c < t.c1; c += t.T) {
+      double init[1];
+      wideSums(t, init, [&](int c, int, int, double (&acc)[1]) {
         double b = I.pB[c];
-        if (!I.hasPRef) { b -= mean; I.pB[c] = b; }
+        if (!I.hasPRef) {
+          b -= mean;
+          I.pB[c] = b;
+        }
         I.x[c] = 0.0;
         I.r[c] = b;
-        init[0] += fabs(b);
-        init[1] += b * precondition(b, I.pD[c]);
-      }
-      teamReduce(t, sh, init, op2);
+        acc[0] += fabs(b);
+      });
       if (stopStage == kStagePressureAssembly) { stopped = true; break; }
 
       // 6. the pressure correction: multigrid CG (pressure_mg.cuh).
       const double initial = init[0];
-      const int cgIters = (initial > 0.0) ? pressureMixed(I, t, sh, dyn, initial) : 0;
+      const int cgIters = (initial > 0.0) ? pressureMixed(I, t, initial, (flags & kFlagPhasedCycle) != 0) : 0;
       if (leader) mon[kMonPressureIterations] += static_cast<double>(cgIters);
       if (!I.hasPRef) {
-        double sx[1] = {0.0};
-        const int opS[1] = {kSum};
-        for (int c = t.c0 + t.tid; c < t.c1; c += t.T) sx[0] += I.x[c];
-        teamReduce(t, sh, sx, opS);
+        double sx[1];
+        wideSums(t, sx, [&](int c, int, int, double (&acc)[1]) { acc[0] += I.x[c]; });
         const double m = sx[0] / static_cast<double>(I.N);
-        for (int c = t.c0 + t.tid; c < t.c1; c += t.T) I.x[c] -= m;
-        t.cl.sync();
+        wideCells(t, [&](int c, int, int) { I.x[c] -= m; });
+        wideBarrier(t);
       }
       if (stopStage == kStagePressureSolve) { stopped = true; break; }
 
       // 7. correct p, u, v and the face fluxes.
-      bandCells(I, t, [&](int c, int i, int j) { correctCell(I, c, i, j); });
-      t.cl.sync();
+      wideCells(t, [&](int c, int i, int j) { correctCell(I, c, i, j); });
+      wideBarrier(t);
       if (stopStage == kStageCorrect) { stopped = true; break; }
     }
     if (stopped) { done = it + 1; break; }
@@ -800,31 +250,38 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
     // 8. divergence (+ SST strain, gradients of k and omega, blending, production).
     if (sst) {
       double v1[1] = {0.0};
-      const int op[1] = {kMax};
-      bandCells(I, t, [&](int c, int i, int j) { sstBlendingCell(I, c, i, j, v1[0]); });
-      teamReduce(t, sh, v1, op);
+      wideCells(t, [&](int c, int i, int j) { sstBlendingCell(I, c, i, j, v1[0]); });
+      wideMax(t, v1);
       note(kMonMaxDivergence, smax(0.0, v1[0]));
       if (stopStage == kStageSstBlending) { done = it + 1; break; }
 
-      double a4[4] = {0.0, 0.0, 0.0, 0.0};
-      const int op4[4] = {kSum, kSum, kSum, kSum};
-      bandCells(I, t, [&](int c, int i, int j) {
-        sstAssemblyCell(I, c, i, j, a4,
+      const unsigned tag = t.epoch;  // of this iteration's sweep messages
+      const bool rowwise = !(flags & kFlagPlainWavefront) && I.NI <= 8 * t.T && mixedRowsFit(I.NI, I.mg.coarseBytes);
+      const bool chained = rowwise && !(flags & (kFlagSequentialRows | kFlagBarrierSweeps)) &&
+                           mixedChained(I, t, smemBytes);
+      const ChainShape z = chainShape(I.NI, t.T);
+      double a4[4];
+      wideSums(t, a4, [&](int c, int i, int j, double (&acc)[4]) {
+        sstAssemblyCell(I, c, i, j, acc,
                         [&](double dK, const double (&oK)[4], double bK, double dW, const double (&oW)[4], double bW,
                             double yk, double yw) {
           I.kD[c] = dK; I.kS[c] = oK[0]; I.kN[c] = oK[1]; I.kW[c] = oK[2]; I.kE[c] = oK[3]; I.kB[c] = bK;
           I.wD[c] = dW; I.wS[c] = oW[0]; I.wN[c] = oW[1]; I.wW[c] = oW[2]; I.wE[c] = oW[3]; I.wB[c] = bW;
-          const Rows32& a = I.tk;
-          a.D[c] = static_cast<float>(dK); a.S[c] = static_cast<float>(oK[0]);
-          a.N[c] = static_cast<float>(oK[1]); a.W[c] = static_cast<float>(oK[2]);
-          a.E[c] = static_cast<float>(oK[3]); a.r[c] = static_cast<float>(bK - yk); a.x[c] = 0.0f;
-          const Rows32& b = I.tw;
-          b.D[c] = static_cast<float>(dW); b.S[c] = static_cast<float>(oW[0]);
-          b.N[c] = static_cast<float>(oW[1]); b.W[c] = static_cast<float>(oW[2]);
-          b.E[c] = static_cast<float>(oW[3]); b.r[c] = static_cast<float>(bW - yw); b.x[c] = 0.0f;
+          const float rk = static_cast<float>(bK - yk), rw = static_cast<float>(bW - yw);
+          auto put = [&](const Rows32& a, float4* rows, double d, const double (&o)[4], float r) {
+            const float D = static_cast<float>(d), S = static_cast<float>(o[0]), N = static_cast<float>(o[1]);
+            const float W = static_cast<float>(o[2]), E = static_cast<float>(o[3]);
+            if (chained) {
+              chainStoreRow(rows, z, i, j, D, S, N, W, E, r);
+            } else {
+              a.D[c] = D; a.S[c] = S; a.N[c] = N; a.W[c] = W; a.E[c] = E; a.r[c] = r;
+            }
+            a.x[c] = 0.0f;
+          };
+          put(I.tk, I.tkC, dK, oK, rk);
+          put(I.tw, I.twC, dW, oW, rw);
         });
       });
-      teamReduce(t, sh, a4, op4);
       note(kMonTurbFirst, a4[0] / smax(a4[1] * smax(I.kIn, kTinySst), kTinySst));
       note(kMonTurbSecond, a4[2] / smax(a4[3] * smax(I.wIn, kTinySst), kTinySst));
       if (stopStage == kStageSstAssembly) { done = it + 1; break; }
@@ -832,31 +289,15 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
       // k and omega sweep in the reference's cell order: their floors and
       // the wall-cell omega override act after the sweeps, so the converged
       // state depends on the order (a colouring would move it by ~1e-3).
-      const bool chained = t.R >= 6 && !(flags & (kFlagSequentialRows | kFlagBarrierSweeps));
-      const unsigned chainBase = static_cast<unsigned>(it) * static_cast<unsigned>(I.NJ);
-      const bool waitTest = (flags & kFlagChainWaitTest) != 0;
-      if (!(flags & kFlagPlainWavefront) && I.NI <= 8 * t.T &&
-          (2 * I.NI + 64) * 8 <= smemBytes) {
-        // the sweep map on the FP32 corrections
-        float* fs = reinterpret_cast<float*>(dyn);
-        const SysView<float> ks = correctionSystem(I.tk), ws = correctionSystem(I.tw);
-        if (chained && chainSmemElems(I.NI) * 4 <= smemBytes) {
-          gsRowScanChained(I, t, sh, 3, ks, ws, fs, chainBase, waitTest);
-        } else if (t.R >= 6 && !(flags & kFlagSequentialRows)) {
-          gsRowScanPipelined(I, t, 3, ks, ws, fs);
-        } else if (t.R == 1) {
-          gsRowScanSweeps(I, 3, ks, fs);
-          gsRowScanSweeps(I, 3, ws, fs);
-        } else if (t.rank == 0) {
-          gsRowScanSweeps(I, 3, ks, fs);
-        } else if (t.rank == 1) {
-          gsRowScanSweeps(I, 3, ws, fs);
-        }
+      if (chained) {
+        chainedSweeps(I, t, tag, (flags & kFlagChainWaitTest) != 0);
+      } else if (rowwise) {
+        sequentialSweeps(I, t);
       } else {
         gsWavefrontSweeps(I, t, 3, I.kD, I.kS, I.kN, I.kW, I.kE, I.kB, I.k, I.wD, I.wS, I.wN,
                           I.wW, I.wE, I.wB, I.om);
       }
-      t.cl.sync();
+      wideBarrier(t);
       if (stopStage == kStageSstSolve) { done = it + 1; break; }
 
       double m8[8];
@@ -864,9 +305,8 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
       for (int s = 0; s < 8; ++s) m8[s] = -INFINITY;
       m8[5] = 0.0;
       m8[7] = 0.0;
-      const int op8[8] = {kMax, kMax, kMax, kMax, kMax, kMax, kMax, kMax};
-      bandCells(I, t, [&](int c, int i, int j) { sstFinishCell<true>(I, c, i, j, m8); });
-      teamReduce(t, sh, m8, op8);
+      wideCells(t, [&](int c, int i, int j) { sstFinishCell<true>(I, c, i, j, m8); });
+      wideMax(t, m8);
       note(kMonMaxK, m8[0]); note(kMonMinK, -m8[1]);
       note(kMonMaxW, m8[2]); note(kMonMinW, -m8[3]);
       note(kMonMaxMut, m8[4]); note(kMonMinMut, -m8[6]);
@@ -874,11 +314,8 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
       note(kMonMaxRatio, m8[7]);
     } else {
       double v1[1] = {0.0};
-      const int op[1] = {kMax};
-      for (int c = t.c0 + t.tid; c < t.c1; c += t.T) {
-        v1[0] = smax(v1[0], fabs(cellDivergence(I, c, c % I.NI, c / I.NI)));
-      }
-      teamReduce(t, sh, v1, op);
+      wideCells(t, [&](int c, int i, int j) { v1[0] = smax(v1[0], fabs(cellDivergence(I, c, i, j))); });
+      wideMax(t, v1);
       note(kMonMaxDivergence, smax(0.0, v1[0]));
     }
 
@@ -890,9 +327,30 @@ simpleKernel(const Instance* __restrict__ instances, int iterations, int stopSta
     }
   }
   if (leader) *I.iterations = done;
-  // No CTA may exit while a peer can still read its shared memory.
-  t.cl.sync();
 }
+
+/// The launch, as plainKernel's (plain_kernel.cu): CTA b runs solves
+/// plan[b].begin .. plan[b].end of `list` one after another; without a plan the
+/// whole grid is the team of instance 0.
+__global__ void __launch_bounds__(kWideThreads, 1)
+simpleKernel(const Instance* __restrict__ instances, const WideCta* __restrict__ plan, const int* __restrict__ list,
+             int iterations, int stopStage, double tolerance, int smemBytes, int flags) {
+  __shared__ WideShared sh;
+  const WideCta me = (plan != nullptr) ? plan[blockIdx.x]
+                                       : WideCta{0, 1, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)};
+  for (int k = me.begin; k < me.end; ++k) {
+    const Instance& I = instances[(list != nullptr) ? list[k] : k];
+    const int R = min(me.R, I.wideMost);
+    if (me.rank >= R) continue;
+    WideTeam t;
+    wideJoin(t, I.wide, I.iterations + 1, &sh, me.rank, R, I.NI, I.NJ, iterations * (me.end - me.begin - 1));
+    mixedSolve(I, t, iterations, stopStage, tolerance, smemBytes, flags);
+    wideLeave(t);
+    __syncthreads();
+  }
+}
+
+}  // namespace
 
 /// Brute-force distance from each cell centroid to the nearest no-slip wall
 /// face centre (TurbulenceModel.cpp:28-65). One thread per cell.
@@ -931,82 +389,57 @@ int chooseClusterSize(int cells) {
 }
 
 int kernelFlags() {
-  // Implementation choices for comparisons and tests. Plain form: bits 2 and 5
-  // run the three k/omega sweeps one after another, bit 7 the pressure CG in
-  // its form for any shape (all in memory), all with the same bits; bit 3 runs
-  // the reference's two-reduction CG (the same to rounding). Mixed form: bit 1
-  // uses the plain wavefront sweeps, bit 2 runs the k/omega row sweeps one after
-  // another instead of pipelined across CTAs, bit 5 pipelines them with a
-  // cluster barrier per row instead of chaining them through DSMEM (identical
-  // results). Bit 6 is for tests: a k/omega sweep also waits for a count that
-  // nothing sets, so that wait gives up and the launch reports its fault word;
-  // bit 8 does the same before the plain form's pressure CG. Other bits are
-  // accepted and have no effect.
+  // Implementation choices for comparisons and tests. Bits 2 and 5 run the
+  // three k/omega sweeps one after another (the same bits). Plain form: bit 7
+  // the pressure CG in its form for any shape (all in memory; the same bits),
+  // bit 3 the reference's two-reduction CG (the same to rounding). Mixed form:
+  // bit 1 the plain wavefront sweeps, bit 9 the V-cycle with a phase per half
+  // sweep (the same bits). Bit 6 is for tests: a k/omega sweep also waits for a
+  // count that nothing sets, so that wait gives up and the launch reports its
+  // fault word; bit 8 does the same before the plain form's pressure CG. Other
+  // bits are accepted and have no effect.
   const char* env = std::getenv("CFD_KERNEL_FLAGS");
   return (env != nullptr) ? std::atoi(env) : 0;
 }
 
-int chainSweepBytes(int NI, int elemBytes) { return static_cast<int>(chainSmemElems(NI) * elemBytes); }
+/// Dynamic shared memory at most: what 227 KB leave beside the static tables
+/// and the multigrid's descriptor.
+constexpr int kMaxMixedSmem = 220928;
 
-namespace {
+int mixedSmemBytes(int NI, int threads, int multigridBytes) {
+  // the coarse levels, the sweeps' copies (a row's two vectors at least)
+  long long bytes = std::max<long long>(multigridBytes, (2LL * NI + 64) * 4);
+  const long long chain = chainBytes(NI, threads);
+  if (chainable(NI, threads) && chain <= kMaxMixedSmem) bytes = std::max(bytes, chain);
+  return static_cast<int>(std::min<long long>(bytes, kMaxMixedSmem));
+}
 
-PerDeviceOnce g_simpleKernelConfigured;
-
-/// The non-portable cluster size (16) and the dynamic shared-memory limit
-/// are attributes of the kernel on each device: set them on every device
-/// this process launches on.
-Status configureSimpleKernel() {
-  return g_simpleKernelConfigured.run([]() -> Status {
-    cudaError_t e = cudaFuncSetAttribute(simpleKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) {
-      e = cudaFuncSetAttribute(simpleKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxClusterSmem);
-    }
-    if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
-    return ok();
+Status prepareSimpleKernel() {
+  static PerDeviceOnce once;
+  return once.run([]() -> Status {
+    const cudaError_t e = cudaFuncSetAttribute(simpleKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxMixedSmem);
+    return (e == cudaSuccess) ? ok() : fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   });
 }
 
-}  // namespace
-
-Status prepareSimpleKernel() { return configureSimpleKernel(); }
-
-int maxActiveClusters(int clusterSize, int threads, int smemBytes) {
-  if (configureSimpleKernel() != CFD_OK) return 0;
+Status launchSimple(const Instance* dInstances, const WidePlan& plan, const WideCta* dPlan, const int* dList,
+                    int threads, int iterations, int stopStage, double tolerance, cudaStream_t stream) {
+  if (Status st = prepareSimpleKernel(); st != CFD_OK) return st;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(static_cast<unsigned>(clusterSize * 64), 1, 1);
+  config.gridDim = dim3(static_cast<unsigned>(plan.ctas.size()), 1, 1);
   config.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
-  config.dynamicSmemBytes = static_cast<size_t>(smemBytes);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(clusterSize);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  config.attrs = attr;
-  config.numAttrs = 1;
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, simpleKernel, &config) != cudaSuccess) return 0;
-  return clusters;
-}
-
-Status launchSimple(const Instance* dInstances, int count, int clusterSize, int threads,
-                    int iterations, int stopStage, double tolerance, cudaStream_t stream,
-                    int smemBytes) {
-  if (Status st = configureSimpleKernel(); st != CFD_OK) return st;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(static_cast<unsigned>(count * clusterSize), 1, 1);
-  config.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
-  config.dynamicSmemBytes = static_cast<size_t>(smemBytes);
+  config.dynamicSmemBytes = static_cast<size_t>(plan.smemBytes);
   config.stream = stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(clusterSize);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
   config.attrs = attr;
   config.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&config, simpleKernel, dInstances, iterations, stopStage, tolerance,
-                                     smemBytes, kernelFlags());
-  if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, std::string("SIMPLE kernel launch: ") + cudaGetErrorString(e));
+  const cudaError_t e = cudaLaunchKernelEx(&config, simpleKernel, dInstances, dPlan, dList, iterations, stopStage,
+                                           tolerance, plan.smemBytes, kernelFlags());
+  if (e != cudaSuccess) {
+    return fail(CFD_INITIALIZATION_FAILURE, std::string("SIMPLE kernel launch: ") + cudaGetErrorString(e));
+  }
   return CFD_OK;
 }
 

@@ -303,20 +303,20 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
   if (m.nodes != nullptr) nodes_.assign(m.nodes, m.nodes + 2 * static_cast<std::size_t>(ni) * nj);
   const std::size_t S = static_cast<std::size_t>(std::max(wall_.count(), 1));
 
-  // Launch shape: CTAs per solve (the mixed form's cluster, and with
-  // CFD_CLUSTER_SIZE, 1 to 16, the most the plain form's team takes) and threads
-  // per CTA (CFD_THREADS, a multiple of 32, at most 512).
+  // Launch shape: CTAs per solve (with CFD_CLUSTER_SIZE, 1 to 16, the most its
+  // team takes) and threads per CTA (CFD_THREADS, a multiple of 32, at most 512).
   clusterSize_ = chooseClusterSize(N_);
   if (const char* env = std::getenv("CFD_THREADS")) {
     const int t = std::atoi(env);
     if (t >= 32 && t <= 512 && t % 32 == 0) threads_ = t;
   }
-  view_.wideMost = wideMostCtas(NI_, NJ_, threads_);
+  const bool mixed = settings_.precision == 1;
+  view_.wideMost = mixed ? mixedMostCtas(NI_, NJ_) : wideMostCtas(NI_, NJ_, threads_);
   if (const char* env = std::getenv("CFD_CLUSTER_SIZE")) {
     const int r = std::atoi(env);
     if (r >= 1 && r <= 16) {
       clusterSize_ = r;
-      view_.wideMost = std::min(view_.wideMost, std::max(r, wideLeastCtas(NI_, threads_)));
+      view_.wideMost = std::min(view_.wideMost, mixed ? r : std::max(r, wideLeastCtas(NI_, threads_)));
     }
   }
 
@@ -350,6 +350,12 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
     if (settings_.precision == 1) {
       double** rows[] = {&I.kS, &I.kN, &I.kW, &I.kE, &I.wS, &I.wN, &I.wW, &I.wE};
       for (double** ptr : rows) *ptr = a.take<double>(N);
+      const std::size_t values = 2 * static_cast<std::size_t>(chainSlots(NI_, NJ_));
+      I.tkV = a.take<unsigned long long>(values);
+      I.twV = a.take<unsigned long long>(values);
+      const std::size_t words = static_cast<std::size_t>(chainWords(NI_, NJ_));
+      I.tkC = a.take<float4>(words);
+      I.twC = a.take<float4>(words);
     } else {
       double** vectors[] = {&I.z, &I.q, &I.d0, &I.d1};
       for (double** ptr : vectors) *ptr = a.take<double>(N);
@@ -360,7 +366,9 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
       const std::size_t spill =
           static_cast<std::size_t>(wideSpillDoubles(NI_, NJ_, I.wideMost, threads_));
       I.spill = a.take<double>(std::max<std::size_t>(spill, 1));
-      const WideScratchLayout layout(NI_, NJ_, wideMessages(NI_, NJ_, I.wideMost, threads_));
+    }
+    {
+      const WideScratchLayout layout(NI_, NJ_, mixed ? 0 : wideMessages(NI_, NJ_, I.wideMost, threads_));
       char* scratch = a.take<char>(layout.bytes);
       if (scratch != nullptr) I.wide = layout.at(scratch);
     }
@@ -393,7 +401,7 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
           break;
         }
       }
-      G.smemBytes = mgSmemBytes_;
+      G.coarseBytes = mgCoarseBytes_;
       // Red-black sweeps before and after the coarse correction, and on the
       // coarsest level; CFD_MG="pre,post,coarse" overrides for tuning runs.
       G.pre = 1;
@@ -416,12 +424,14 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
         L.NJ = sh.NJ;
         L.smem = sh.smem;
         L.smemWake = sh.smemWake;
+        const unsigned half = static_cast<unsigned>((sh.NI + 1) / 2);
+        L.perHalf = (half > 1) ? static_cast<unsigned>(((1ull << 32) + half - 1) / half) : 0u;
         L.D = a.take<float>(n); L.S = a.take<float>(n); L.N = a.take<float>(n);
         L.W = a.take<float>(n); L.E = a.take<float>(n); L.inv = a.take<float>(n);
-        L.x = a.take<float>(n); L.b = a.take<float>(n);
+        L.x = a.take<float>(n); L.b = a.take<float>(n); L.y = a.take<float>(n);
         L.wake = (l == 0) ? I.acrossJ0 : a.take<int>(sh.NI);
       }
-      float** vectors[] = {&G.r, &G.q, &G.e, &G.z0, &G.z1, &G.d0, &G.d1};
+      float** vectors[] = {&G.r, &G.q, &G.e, &G.z0, &G.z1, &G.d0, &G.d1, &G.zs};
       for (float** ptr : vectors) *ptr = a.take<float>(N);
       for (Rows32* rows : {&I.mom, &I.tk, &I.tw}) {
         float** arrays[] = {&rows->D, &rows->S, &rows->N, &rows->W, &rows->E, &rows->r, &rows->x};
@@ -560,11 +570,14 @@ void Solver::planMultigrid(const std::vector<int>& wake0) {
     }
   }
   int bytes = 0;
+  mgCoarseBytes_ = 0;
   for (int l = mgDistributed_; l < levels; ++l) {
     mgShape_[l].smem = bytes;
-    bytes += 8 * ((mgShape_[l].NI * mgShape_[l].NJ + 3) & ~3) * static_cast<int>(sizeof(float));
+    bytes += 32 * (((mgShape_[l].NI + 1) / 2 * 2 * mgShape_[l].NJ + 3) & ~3);  // apart by colour
     mgShape_[l].smemWake = bytes;
-    bytes += ((mgShape_[l].NI + 3) & ~3) * static_cast<int>(sizeof(int));
+    const int wake = ((mgShape_[l].NI + 3) & ~3) * static_cast<int>(sizeof(int));
+    bytes += wake;
+    mgCoarseBytes_ += 32 * ((mgShape_[l].NI * mgShape_[l].NJ + 3) & ~3) + wake;
   }
   mgSmemBytes_ = bytes;
 }
@@ -578,9 +591,9 @@ Status Solver::setLaunchShape(int clusterSize, int threads) {
   return CFD_OK;
 }
 
-int Solver::launchSmemBytes() const {
-  const int scan = chainSweepBytes(NI_, 4);  // the chained k/omega row sweeps, FP32
-  return std::max(mgSmemBytes_, (scan <= kMaxClusterSmem) ? scan : 0);
+WideJob Solver::wideJob() const {
+  return WideJob{NI_, NJ_, view_.wideMost, model_ == 2,
+                 (settings_.precision == 1) ? mixedSmemBytes(NI_, threads_, mgSmemBytes_) : 0};
 }
 
 Solver::~Solver() {
@@ -833,11 +846,9 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
   int total = 0;
   while (total < n) {
     const int chunk = std::min(n - total, historyCapacity_);
-    const Status st =
-        (settings_.precision == 1)
-            ? launchSimple(dView_, 1, clusterSize_, threads_, chunk, stopStage, tolerance, stream_, launchSmemBytes())
-            : launchPlain(dView_, planWide({wideJob()}, threads_), nullptr, nullptr, threads_, chunk, stopStage,
-                          tolerance, stream_);
+    const auto launch = (settings_.precision == 1) ? launchSimple : launchPlain;
+    const Status st = launch(dView_, planWide({wideJob()}, threads_), nullptr, nullptr, threads_, chunk, stopStage,
+                             tolerance, stream_);
     if (st != CFD_OK) return st;
     CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
     int words[2] = {0, 0};
@@ -1347,14 +1358,13 @@ cfd_status cfd_gpu_destroy(cfd_handle h) {
 
 // ---- batches ------------------------------------------------------------------------------
 
-/// The solves of a batch that share a launch: the plain form's together, as a
-/// wide plan shares the GPU between them; the mixed form's by cluster size.
-/// One launch over a contiguous part of the descriptor table, on a stream of
-/// its own.
+/// The solves of a batch that share a launch, as a plan shares the GPU between
+/// them: those of one form and thread count. One launch over a contiguous part
+/// of the descriptor table, on a stream of its own.
 struct BatchGroup {
-  bool wide{false};
+  bool mixed{false};
   int offset{0}, count{0};
-  int clusterSize{1}, threads{512}, smemBytes{0};
+  int threads{512};
   std::vector<int> members;  // indices into cfd_batch_t::handles
   cfdb::WidePlan plan;
   cfdb::WideCta* dPlan{nullptr};
@@ -1368,7 +1378,7 @@ struct cfd_batch_t {
   cfdb::Instance* dTable{nullptr};
   cudaStream_t stream{nullptr};
   cudaEvent_t fork{nullptr};
-  std::vector<BatchGroup> groups;  // widest clusters first
+  std::vector<BatchGroup> groups;
   int clusterSize{1};              // the most frequent shape (cfd_batch_shape)
   int threads{512};
   int lastIterations{0};
@@ -1385,9 +1395,8 @@ cfd_status refreshTable(cfd_batch b) {
   }
   cudaError_t e = cudaMemcpyAsync(b->dTable, table.data(), table.size() * sizeof(cfdb::Instance),
                                   cudaMemcpyHostToDevice, b->stream);
-  // the wide groups' plans (a solve's model can change between launches)
+  // the groups' plans (a solve's model can change between launches)
   for (BatchGroup& g : b->groups) {
-    if (!g.wide) continue;
     std::vector<cfdb::WideJob> jobs;
     for (int k : g.members) jobs.push_back(b->handles[static_cast<std::size_t>(k)]->solver->wideJob());
     g.plan = cfdb::planWide(jobs, g.threads);
@@ -1414,8 +1423,8 @@ cfd_status refreshTable(cfd_batch b) {
 
 cfd_status launchGroup(cfd_batch b, const BatchGroup& g, int n, int stopStage, double tolerance, cudaStream_t s) {
   const cfdb::Instance* table = b->dTable + g.offset;
-  if (g.wide) return cfdb::launchPlain(table, g.plan, g.dPlan, g.dList, g.threads, n, stopStage, tolerance, s);
-  return cfdb::launchSimple(table, g.count, g.clusterSize, g.threads, n, stopStage, tolerance, s, g.smemBytes);
+  const auto launch = g.mixed ? cfdb::launchSimple : cfdb::launchPlain;
+  return launch(table, g.plan, g.dPlan, g.dList, g.threads, n, stopStage, tolerance, s);
 }
 
 /// n iterations of every solve of the batch, ordered on `s`: one launch per
@@ -1455,30 +1464,24 @@ cfd_status cfd_batch_create(const cfd_handle* solvers, int count, cfd_batch* out
     }
     b->handles.push_back(solvers[k]);
   }
-  // The plain form's solves in one group per thread count, the mixed form's in
-  // one per launch shape, widest first so its clusters are placed before the
-  // narrower groups fill the gaps.
+  // One group per form and thread count.
   std::map<std::pair<int, int>, int> shapes;  // (CTAs, threads) -> solves
   for (int k = 0; k < count; ++k) {
     const cfdb::Solver& sv = *b->handles[static_cast<std::size_t>(k)]->solver;
-    const bool wide = sv.precision() == 0;
+    const bool mixed = sv.precision() == 1;
     shapes[{sv.clusterSize(), sv.threads()}] += 1;
     auto it = std::find_if(b->groups.begin(), b->groups.end(), [&](const BatchGroup& g) {
-      return g.wide == wide && (wide || g.clusterSize == sv.clusterSize()) && g.threads == sv.threads();
+      return g.mixed == mixed && g.threads == sv.threads();
     });
     if (it == b->groups.end()) {
       BatchGroup g;
-      g.wide = wide;
-      g.clusterSize = wide ? 1 << 16 : sv.clusterSize();
+      g.mixed = mixed;
       g.threads = sv.threads();
       b->groups.push_back(g);
       it = b->groups.end() - 1;
     }
     it->members.push_back(k);
-    if (!wide) it->smemBytes = std::max(it->smemBytes, sv.launchSmemBytes());
   }
-  std::stable_sort(b->groups.begin(), b->groups.end(),
-                   [](const BatchGroup& a, const BatchGroup& c) { return a.clusterSize > c.clusterSize; });
   int offset = 0;
   for (BatchGroup& g : b->groups) {
     g.offset = offset;

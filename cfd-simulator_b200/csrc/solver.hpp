@@ -133,13 +133,11 @@ class Solver {
   /// Rough device footprint of a solve of NI x NJ cells (the arena's layout).
   static std::size_t estimateBytes(int NI, int NJ);
   const Instance& deviceView() const { return view_; }
-  /// Dynamic shared memory a launch of this solve needs on a cluster (mixed form).
-  int launchSmemBytes() const;
-  /// This solve for the planner of wide launches (plain form).
-  WideJob wideJob() const { return WideJob{NI_, NJ_, view_.wideMost, model_ == 2}; }
+  /// This solve for the planner of launches.
+  WideJob wideJob() const;
   int precision() const { return settings_.precision; }
   int wallStations() const { return wall_.count(); }
-  /// CTAs per cluster (1..16) and threads per CTA (multiple of 32, <= 512).
+  /// The CTAs reported (1..16) and threads per CTA (multiple of 32, <= 512).
   Status setLaunchShape(int clusterSize, int threads);
   int multigridLevels() const { return static_cast<int>(mgShape_.size()); }
   cudaStream_t stream() const { return stream_; }
@@ -203,30 +201,28 @@ class Solver {
   };
   std::vector<MgShape> mgShape_;
   int mgDistributed_{0};
-  int mgSmemBytes_{0};
+  int mgSmemBytes_{0}, mgCoarseBytes_{0};
 };
 
-/// Levels of the multigrid with at most this many cells run on one CTA from
+/// Levels of the multigrid with at most this many cells run on every CTA from
 /// shared memory (eight FP32 arrays per cell: ~130 KB for all of them).
 constexpr int kMgSharedCells = 3072;
 
 Status launchWallDistance(int n, const double* centroid, int walls, const double* wallCentre,
                           double far, double* out, cudaStream_t stream);
 
-/// Launch the mixed form's kernel over `count` instances (device array), one
-/// cluster of `clusterSize` CTAs each.
-Status launchSimple(const Instance* dInstances, int count, int clusterSize, int threads,
-                    int iterations, int stopStage, double tolerance, cudaStream_t stream,
-                    int smemBytes);
+/// Launch the mixed form's kernel as `plan` says; dPlan and dList are its CTAs
+/// and list on the device (null for a plan of the first instance alone).
+Status launchSimple(const Instance* dInstances, const WidePlan& plan, const WideCta* dPlan, const int* dList,
+                    int threads, int iterations, int stopStage, double tolerance, cudaStream_t stream);
+/// Its dynamic shared memory on blocks of `threads`, with that of the
+/// multigrid's coarse levels.
+int mixedSmemBytes(int NI, int threads, int multigridBytes);
 
 /// The error for a launch whose fault word (Instance::iterations[1]) is
 /// nonzero: a bounded wait inside the kernel gave up, so its results are not
 /// to be used.
 Status launchFault(int word);
-
-/// Dynamic shared memory of the chained k/omega sweeps on rows of NI cells
-/// of `elemBytes` each (two rows, the scan's warp totals and the ring).
-int chainSweepBytes(int NI, int elemBytes);
 
 /// Launch the plain form's kernel as `plan` says; dPlan and dList are its CTAs
 /// and list on the device (null for a plan of the first instance alone).
@@ -237,16 +233,11 @@ Status preparePlainKernel();
 /// The kernels' implementation flags (kFlag*), from CFD_KERNEL_FLAGS.
 int kernelFlags();
 
-constexpr int kMaxClusterSmem = 210 * 1024;  // dynamic shared memory of the mixed form's kernel at most
-
-/// Cluster size used for a solve of `cells` cells (power of two, 1..16).
+/// The CTAs reported for a solve of `cells` cells (power of two, 1..16).
 int chooseClusterSize(int cells);
 
 /// Set the kernel's launch attributes (once per process); must run before a
 /// launch is captured into a CUDA graph.
 Status prepareSimpleKernel();
-
-/// Clusters of this shape the GPU holds at once (cudaOccupancyMaxActiveClusters).
-int maxActiveClusters(int clusterSize, int threads, int smemBytes);
 
 }  // namespace cfdb

@@ -43,6 +43,12 @@ int wideMostCtas(int NI, int NJ, int threads) {
   return std::min(s.columnTiles * s.unitRows, kMaxWideCtas / s.columnTiles * s.columnTiles);
 }
 
+int mixedMostCtas(int NI, int NJ) {
+  // 256 cells a CTA (half its threads): below that the barriers are all there is
+  const int chunks = static_cast<int>((static_cast<long long>(NI) * NJ + 255) / 256);
+  return std::min(std::max(chunks, 6), kMaxWideCtas);
+}
+
 int wideChooseCtas(int NI, int NJ, int capacity) {
   const int columns = wideLeastCtas(NI, kWideThreads);
   int best = columns;
@@ -64,6 +70,7 @@ long long wideSpillDoubles(int NI, int NJ, int most, int threads) {
 namespace {
 
 int usefulCtas(const WideJob& job, int width, int threads) {
+  if (job.mixedSmem > 0) return std::min(width, job.most);
   return wideUsefulCtas(job.NI, job.NJ, std::min(width, job.most), threads);
 }
 
@@ -71,11 +78,17 @@ int usefulCtas(const WideJob& job, int width, int threads) {
 /// other phases' passes (0.54 ms on 16 CTAs at 768x192), the sweeps' rows.
 double outerMicroseconds(const WideJob& job, int R) {
   const double cells = static_cast<double>(job.NI) * job.NJ;
+  if (job.mixedSmem > 0) {
+    // 16 V-cycles of ~8 barriers and a coarse cycle each
+    return 16.0 * (30.0 + 3.3 * cells / R / 512.0) + 30.0 + cells / R / 512.0 * (job.sst ? 30.0 : 15.0) +
+           (job.sst ? 0.4 * job.NJ : 0.0);
+  }
   return 200.0 * wideCgMicroseconds(job.NI, job.NJ, R) + 30.0 + cells / R / 512.0 * (job.sst ? 30.0 : 15.0) +
          (job.sst ? 0.4 * job.NJ : 0.0);
 }
 
 int smemBytes(const WideJob& job, int R, int threads) {
+  if (job.mixedSmem > 0) return job.mixedSmem;
   const bool any = (kernelFlags() & kFlagSharedCg) != 0;
   long long bytes = wideCgBytes(job.NI, job.NJ, R, threads, kMaxWideSmem, any);
   {
@@ -113,7 +126,9 @@ WidePlan planWide(const std::vector<WideJob>& jobs, int threads) {
   // team that is free first. The number of teams that finishes first wins; a
   // solve's bits do not depend on it.
   int least = 1;
-  for (const WideJob& job : jobs) least = std::max(least, wideLeastCtas(job.NI, threads));
+  for (const WideJob& job : jobs) {
+    if (job.mixedSmem == 0) least = std::max(least, wideLeastCtas(job.NI, threads));
+  }
   double best = -1.0;
   int bestTeams = 1;
   std::vector<std::vector<int>> bestLists;

@@ -60,18 +60,22 @@ int wideLeastCtas(int NI, int threads);
 /// Doubles of spill a solve needs whatever the number of its CTAs up to `most`.
 long long wideSpillDoubles(int NI, int NJ, int most, int threads);
 
+/// CTAs a solve of the mixed form can use at most.
+int mixedMostCtas(int NI, int NJ);
+
 /// A solve as the planner sees it.
 struct WideJob {
   int NI, NJ;
   int most;  // CTAs at most
   bool sst;
+  int mixedSmem;  // mixed form: its dynamic shared memory; 0: plain form
 };
 struct WidePlan {
   std::vector<WideCta> ctas;
   std::vector<int> list;  // solves in the order the CTAs' ranges name them
   int smemBytes{0};
 };
-/// How one launch runs these solves: side by side when the GPU holds them all
+/// How one launch runs these solves (of one form): side by side when the GPU holds them all
 /// at their widest, else in teams that take one solve after another.
 WidePlan planWide(const std::vector<WideJob>& jobs, int threads);
 

@@ -270,25 +270,39 @@ DEV void wideCells(const WideTeam& t, F&& f) {
   }
 }
 
-/// cell(c, i, j, acc) over every own cell, adding to its chunk's sums; the
-/// team's totals in every thread. Also a barrier. A chunk's sums are a tree
-/// over its cells, 32 chunks' a tree, and those are added in order.
+/// Items 0 .. count-1 in chunks of 256, and this CTA's share of the chunks.
+struct WideRange {
+  int count, chunks, chunk0, chunk1;
+};
+DEV WideRange wideRange(const WideTeam& t, int count) {
+  const int chunks = (count + kChunkCells - 1) / kChunkCells;
+  return WideRange{count, chunks, static_cast<int>(static_cast<long long>(chunks) * t.rank / t.R),
+                   static_cast<int>(static_cast<long long>(chunks) * (t.rank + 1) / t.R)};
+}
+/// f(m) for every own item.
+template <typename F>
+DEV void wideItems(const WideTeam& t, const WideRange& range, F&& f) {
+  const int end = min(range.chunk1 * kChunkCells, range.count);
+  for (int m = range.chunk0 * kChunkCells + t.tid; m < end; m += t.T) f(m);
+}
+
+/// item(m, acc) over every own item, adding to its chunk's sums; the team's
+/// totals in every thread. Also a barrier. A chunk's sums are a tree over its
+/// items, 32 chunks' a tree, and those are added in order. At most as many
+/// items as the block has cells.
 template <int K, typename F>
-DEV void wideSums(WideTeam& t, double (&out)[K], F&& cell) {
+DEV void wideItemSums(WideTeam& t, const WideRange& range, double (&out)[K], F&& item) {
   const int lane = t.tid & 31, warp = t.tid >> 5, warps = t.T >> 5;
   const int team = min(t.T, kChunkCells), teams = t.T / team, mine = t.tid / team, lt = t.tid - mine * team;
   double* sums = t.mem.chunkSums + static_cast<std::size_t>((t.epoch + 1u) & 1u) * kMaxSums * t.chunks;
-  for (int base = t.chunk0; base < t.chunk1; base += kChunkBatch) {
-    const int n = min(t.chunk1 - base, kChunkBatch);
+  for (int base = range.chunk0; base < range.chunk1; base += kChunkBatch) {
+    const int n = min(range.chunk1 - base, kChunkBatch);
     for (int slot = mine; slot < n && mine < teams; slot += teams) {
-      // the same 32 cells share a warp's part whatever the number of threads
+      // the same 32 items share a warp's part whatever the number of threads
       for (int first = lt; first < kChunkCells; first += team) {
-        const int c = (base + slot) * kChunkCells + first;
+        const int m = (base + slot) * kChunkCells + first;
         double acc[K] = {};
-        if (c < t.N) {
-          const int j = c / t.NI;
-          cell(c, c - j * t.NI, j, acc);
-        }
+        if (m < range.count) item(m, acc);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -304,18 +318,18 @@ DEV void wideSums(WideTeam& t, double (&out)[K], F&& cell) {
       double a[kChunkCells / 32];
 #pragma unroll
       for (int w = 0; w < kChunkCells / 32; ++w) a[w] = t.sh->chunkPart[slot][w][k];
-      sums[k * t.chunks + base + slot] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+      sums[k * range.chunks + base + slot] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     }
-    if (base + kChunkBatch < t.chunk1) __syncthreads();
+    if (base + kChunkBatch < range.chunk1) __syncthreads();
   }
   wideBarrier(t);
-  const int groups = (t.chunks + 31) / 32;
+  const int groups = (range.chunks + 31) / 32;
   double total[K] = {};
   for (int first = 0; first < groups; first += 256) {
     const int n = min(groups - first, 256);
     for (int m = warp; m < K * n; m += warps) {
       const int k = m / n, group = first + m - k * n, at = group * 32 + lane;
-      double a = (at < t.chunks) ? __ldcg(sums + k * t.chunks + at) : 0.0;
+      double a = (at < range.chunks) ? __ldcg(sums + k * range.chunks + at) : 0.0;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
       if (lane == 0) t.sh->groupPart[k][group - first] = a;
@@ -329,6 +343,15 @@ DEV void wideSums(WideTeam& t, double (&out)[K], F&& cell) {
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) out[k] = total[k];
+}
+
+/// The sums over every cell of the block, cell(c, i, j, acc).
+template <int K, typename F>
+DEV void wideSums(WideTeam& t, double (&out)[K], F&& cell) {
+  wideItemSums(t, WideRange{t.N, t.chunks, t.chunk0, t.chunk1}, out, [&](int c, double (&acc)[K]) {
+    const int j = c / t.NI;
+    cell(c, c - j * t.NI, j, acc);
+  });
 }
 
 }  // namespace cfdb
