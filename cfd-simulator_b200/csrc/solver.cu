@@ -316,7 +316,7 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
     const int r = std::atoi(env);
     if (r >= 1 && r <= 16) {
       clusterSize_ = r;
-      view_.wideMost = std::min(view_.wideMost, mixed ? r : std::max(r, wideLeastCtas(NI_, threads_)));
+      view_.wideMost = std::min(view_.wideMost, mixed ? r : std::max(r, wideLeastCtas(NI_, NJ_, threads_)));
     }
   }
 

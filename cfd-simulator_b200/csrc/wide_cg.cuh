@@ -50,15 +50,14 @@ constexpr int kMaxColumnTiles = 64;
 constexpr int kMaxUnits = 160;  // of a block: 144 as tiled below
 constexpr int kUnitThreads = 32 * kUnitWarps;
 
-__host__ __device__ inline WideCgShape wideCgShape(int NI, int NJ, int R, int T) {
+/// The tiling of the block in `columnTiles` column tiles (rows of a unit and
+/// units included), for teams of `team` threads.
+__host__ __device__ inline WideCgShape wideCgTiles(int NI, int NJ, int columnTiles, int team) {
   WideCgShape s;
-  const int team = (T < kUnitThreads) ? T : kUnitThreads;
-  s.columnTiles = (NI + team - 1) / team;
-  if (s.columnTiles > kMaxColumnTiles) s.columnTiles = kMaxColumnTiles;  // then several columns a thread
+  s.columnTiles = columnTiles;
   s.width = (NI + s.columnTiles - 1) / s.columnTiles;
   s.passes = (s.width + team - 1) / team;
   s.G = ((s.width + s.passes - 1) / s.passes + 31) / 32 * 32;
-  s.teams = T / team;
   s.groups = team / s.G;
   // units: as many as fit the SMs (144 of 148 leave a column-tile remainder),
   // and two rows a thread at least, below which the exchange is all there is
@@ -68,6 +67,33 @@ __host__ __device__ inline WideCgShape wideCgShape(int NI, int NJ, int R, int T)
   if (s.K < 2) s.K = 2;
   s.B = s.K * s.groups;
   s.unitRows = (NJ + s.B - 1) / s.B;
+  return s;
+}
+/// The block's tiling is a rule of the block and the threads alone: column tiles
+/// as wide as a team, half or a quarter of it, whichever leaves a thread the
+/// fewest rows; above two rows a thread, of those the shortest border. 768x192 in
+/// 144 units of 64x16 cells has 160 border cells a unit, in units of 256x4 it has
+/// 520: 1,000 iterations 4.7 against 5.2 ms; 642x151 gets 3 rows a thread instead
+/// of 4. With two rows a thread wide tiles stay: a side's messages are stored a
+/// row at a time, 16 bytes each, and cost more than the shorter border saves
+/// (384x96, 200 iterations and the rest of an SST iteration: 0.93 ms in tiles
+/// of 192x2, 1.01 in tiles of 64x8).
+__host__ __device__ inline WideCgShape wideCgShape(int NI, int NJ, int R, int T) {
+  const int team = (T < kUnitThreads) ? T : kUnitThreads;
+  WideCgShape s;
+  int best = 0;
+  for (int w = team; w >= 32 && w >= team / 4; w /= 2) {
+    int tiles = (NI + w - 1) / w;
+    if (w < team && (w % 32 != 0 || tiles > 144)) break;
+    if (tiles > kMaxColumnTiles) tiles = kMaxColumnTiles;  // then several columns a thread
+    const WideCgShape z = wideCgTiles(NI, NJ, tiles, team);
+    const int cost = 4096 * z.K * z.passes + ((z.K > 2) ? 2 * (z.width + z.B) : 0);
+    if (w == team || cost < best) {
+      s = z;
+      best = cost;
+    }
+  }
+  s.teams = T / team;
   s.RT = R / s.columnTiles;
   if (s.RT > s.unitRows) s.RT = s.unitRows;
   s.units = (s.RT > 0) ? (s.unitRows + s.RT - 1) / s.RT : s.unitRows;

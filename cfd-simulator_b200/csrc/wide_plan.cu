@@ -36,7 +36,7 @@ double wideCgMicroseconds(int NI, int NJ, int R) {
   return (form % 8 == 0) ? 1.2 + 0.5 * cells : 1.2 + 1.0 * cells;
 }
 
-int wideLeastCtas(int NI, int threads) { return wideCgShape(NI, 1, 1, threads).columnTiles; }
+int wideLeastCtas(int NI, int NJ, int threads) { return wideCgShape(NI, NJ, 1, threads).columnTiles; }
 
 int wideMostCtas(int NI, int NJ, int threads) {
   const WideCgShape s = wideCgShape(NI, NJ, 1, threads);
@@ -50,7 +50,7 @@ int mixedMostCtas(int NI, int NJ) {
 }
 
 int wideChooseCtas(int NI, int NJ, int capacity) {
-  const int columns = wideLeastCtas(NI, kWideThreads);
+  const int columns = wideLeastCtas(NI, NJ, kWideThreads);
   int best = columns;
   for (int R = columns; R <= capacity; R += columns) {
     if (wideCgMicroseconds(NI, NJ, R) < wideCgMicroseconds(NI, NJ, best)) best = R;
@@ -60,7 +60,7 @@ int wideChooseCtas(int NI, int NJ, int capacity) {
 
 long long wideSpillDoubles(int NI, int NJ, int most, int threads) {
   long long doubles = 0;
-  const int columns = wideLeastCtas(NI, threads);
+  const int columns = wideLeastCtas(NI, NJ, threads);
   for (int R = columns; R <= std::max(most, columns); ++R) {
     doubles = std::max(doubles, R * wideCgSpill(NI, NJ, R, threads, kMaxWideSmem, true));
   }
@@ -127,7 +127,7 @@ WidePlan planWide(const std::vector<WideJob>& jobs, int threads) {
   // solve's bits do not depend on it.
   int least = 1;
   for (const WideJob& job : jobs) {
-    if (job.mixedSmem == 0) least = std::max(least, wideLeastCtas(job.NI, threads));
+    if (job.mixedSmem == 0) least = std::max(least, wideLeastCtas(job.NI, job.NJ, threads));
   }
   double best = -1.0;
   int bestTeams = 1;

@@ -55,7 +55,7 @@ int wideChooseCtas(int NI, int NJ, int capacity);
 /// CTAs a solve can use at most (a CG unit each) and needs at least (a column
 /// tile each), for blocks of `threads`.
 int wideMostCtas(int NI, int NJ, int threads);
-int wideLeastCtas(int NI, int threads);
+int wideLeastCtas(int NI, int NJ, int threads);
 
 /// Doubles of spill a solve needs whatever the number of its CTAs up to `most`.
 long long wideSpillDoubles(int NI, int NJ, int most, int threads);
