@@ -44,8 +44,11 @@ int wideMostCtas(int NI, int NJ, int threads) {
 }
 
 int mixedMostCtas(int NI, int NJ) {
-  // 256 cells a CTA (half its threads): below that the barriers are all there is
-  const int chunks = static_cast<int>((static_cast<long long>(NI) * NJ + 255) / 256);
+  // 512 cells a CTA, one a thread: more CTAs gain nothing (two iterations at
+  // 384x96 on 72 CTAs 1.66 ms, on 144 1.67; at 192x48 on 18 1.22, on 36 1.22),
+  // fewer do lose (1.75 on 36, 1.25 on 9), and a batch holds more solves side by
+  // side. Six, for the sweeps.
+  const int chunks = static_cast<int>((static_cast<long long>(NI) * NJ + 511) / 512);
   return std::min(std::max(chunks, 6), kMaxWideCtas);
 }
 
