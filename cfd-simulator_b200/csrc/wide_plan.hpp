@@ -11,7 +11,7 @@ namespace cfdb {
 
 /// Dynamic shared memory of a wide kernel: what 227 KB leave beside its
 /// static tables.
-constexpr int kMaxWideSmem = 223120;
+constexpr int kMaxWideSmem = 222032;
 
 /// CTAs the current device runs at once with one wide CTA per SM (at most
 /// kMaxWideCtas); 0 with an error set when the device cannot be asked.
