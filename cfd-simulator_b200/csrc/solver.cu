@@ -449,13 +449,26 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
   dIterations_ = view_.iterations;
   CUDA_OR_FAIL(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
 
-  // Scatter per-face data into the two device families.
-  std::vector<double> hN(FN), hE(FE);
+  // Per-face data into the two device families: the j-faces are in the device's
+  // order already, the i-faces go from columns to rows, in tiles that stay in the
+  // cache (the index of every face by a division took half of a solve's creation).
+  std::vector<double> hE(FE);
+  auto rowsOfIFaces = [&](const auto* columns, auto* rows) {
+    constexpr int kTile = 16;
+    for (int i0 = 0; i0 <= NI_; i0 += kTile) {
+      for (int j0 = 0; j0 < NJ_; j0 += kTile) {
+        const int iEnd = std::min(i0 + kTile, NI_ + 1), jEnd = std::min(j0 + kTile, NJ_);
+        for (int j = j0; j < jEnd; ++j) {
+          for (int i = i0; i < iEnd; ++i) {
+            rows[static_cast<std::size_t>(j) * (NI_ + 1) + i] = columns[static_cast<std::size_t>(i) * NJ_ + j];
+          }
+        }
+      }
+    }
+  };
   auto put = [&](const std::vector<double>& src, const double* dN, const double* dE) -> Status {
-    std::fill(hN.begin(), hN.end(), 0.0);
-    std::fill(hE.begin(), hE.end(), 0.0);
-    for (int f = 0; f < F_; ++f) (famOf(f) ? hE : hN)[idxOf(f)] = src[f];
-    CUDA_OR_FAIL(cudaMemcpy(const_cast<double*>(dN), hN.data(), FN * sizeof(double), cudaMemcpyHostToDevice));
+    rowsOfIFaces(src.data() + jFaces_, hE.data());
+    CUDA_OR_FAIL(cudaMemcpy(const_cast<double*>(dN), src.data(), FN * sizeof(double), cudaMemcpyHostToDevice));
     CUDA_OR_FAIL(cudaMemcpy(const_cast<double*>(dE), hE.data(), FE * sizeof(double), cudaMemcpyHostToDevice));
     return CFD_OK;
   };
@@ -476,9 +489,9 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
       (st = put(bv, I.bcvN, I.bcvE)) || (st = put(bcP_, I.bcpN, I.bcpE))) {
     return st;
   }
-  std::vector<int8_t> kN(FN, 0), kE(FE, 0);
-  for (int f = 0; f < F_; ++f) (famOf(f) ? kE : kN)[idxOf(f)] = static_cast<int8_t>(kind_[f]);
-  CUDA_OR_FAIL(cudaMemcpy(const_cast<int8_t*>(I.kindN), kN.data(), FN, cudaMemcpyHostToDevice));
+  std::vector<int8_t> kinds(kind_.begin(), kind_.end()), kE(FE);
+  rowsOfIFaces(kinds.data() + jFaces_, kE.data());
+  CUDA_OR_FAIL(cudaMemcpy(const_cast<int8_t*>(I.kindN), kinds.data(), FN, cudaMemcpyHostToDevice));
   CUDA_OR_FAIL(cudaMemcpy(const_cast<int8_t*>(I.kindE), kE.data(), FE, cudaMemcpyHostToDevice));
   CUDA_OR_FAIL(cudaMemcpy(const_cast<int*>(I.acrossJ0), acrossJ0.data(), NI_ * sizeof(int), cudaMemcpyHostToDevice));
   for (std::size_t l = 1; l < mgShape_.size(); ++l) {
