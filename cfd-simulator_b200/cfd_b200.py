@@ -528,7 +528,7 @@ def set_device(device: int) -> None:
 
 
 class Batch:
-    """Many solves in one launch, one thread-block cluster each (cfd_batch_*)."""
+    """Many solves in one launch, a team of CTAs each (cfd_batch_*)."""
 
     def __init__(self, solvers: list[SimpleSolver]):
         self.solvers = list(solvers)

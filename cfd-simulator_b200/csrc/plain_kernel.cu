@@ -8,7 +8,7 @@
 // fluxes; pressure-correction assembly; the pressure CG (wide_cg.cuh);
 // correction; SST blending, assembly, the k and omega sweeps (row_sweeps.cuh),
 // floors and eddy viscosity. A phase is a grid-stride pass over the team's
-// cells between two barriers (~1.5 us each); the CG, 200 exchanges an
+// cells between two barriers (1.0 us each); the CG, 200 exchanges an
 // iteration, is most of the time.
 //
 // Every sum is formed in an order that depends on the grid alone, so a solve

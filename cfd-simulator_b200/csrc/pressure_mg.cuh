@@ -19,7 +19,7 @@
 //                  then red coming up, so the cycle is symmetric).
 //
 // What bounds it is the number of steps that need the whole team, each a
-// barrier through L2 (~1.5 us) around well under a microsecond of work. So:
+// barrier through L2 (1.0 us) around a microsecond or two of work. So:
 //   * the red half sweep of a level from a zero start is x = b / D and is
 //     written by whatever phase produced b;
 //   * a level's way down is one phase, its way up another. A thread has a 2x2
@@ -315,8 +315,8 @@ DEV Blacks blacksOf(const Lv& L, int I, int J, Value&& value) {
 /// A level's way down with one sweep: the black half sweep and the restriction
 /// of its residual, from the red start. The black values are used and not kept
 /// (the way up starts with that half sweep). kStart: begin the coarse level, red
-/// cells b / D, black 0. 768x192 on 148 CTAs, and the half sweep and the
-/// restriction it replaces, see the top.
+/// cells b / D, black 0. 768x192 on 148 CTAs: 2.8 us and a barrier; as two
+/// phases on 16 CTAs it took 6.4 and 6.7.
 template <bool kStart>
 DEV void levelDown(const Lv& F, const Lv& C, const Span& s) {
   float* __restrict__ bw = C.b;
@@ -441,8 +441,9 @@ DEV CoarseValues sharedValues(const SharedLv& C) { return CoarseValues{C.x, C.NI
 
 /// The V-cycle of the shared-memory levels, by every CTA alike: their
 /// right-hand side is where the team restricted it (global memory); the result
-/// stays in shared memory. 96x24 cells and the four levels below: 5.2 us; by
-/// cell, with a division and eight loads of separate arrays a cell, 15.5 us.
+/// stays in shared memory. 96x24 cells and the four levels below: 10 us; by
+/// cell, with a division and eight loads of separate arrays a cell, 15.5 us. One
+/// phase a level as above is slower here (384x96: 1.80 -> 1.97 ms a call).
 DEV void sharedCycle(const Multigrid& G) {
   const int L = G.levels, m = G.distributed, w = G.warpFrom;
   const int tid = static_cast<int>(threadIdx.x);

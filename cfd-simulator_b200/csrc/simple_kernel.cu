@@ -8,7 +8,7 @@
 // CTAs (wide_team.cuh), one per SM and up to the whole GPU, that meet in
 // barriers through L2, and a batch's solves share the launch by a plan. One
 // thread-block cluster of 16 CTAs per solve has cheaper barriers (0.7 us against
-// ~1.5) but leaves 132 SMs idle beside a lone solve: a phase over 768x192 cells
+// 1.0) but leaves 132 SMs idle beside a lone solve: a phase over 768x192 cells
 // took 6 us there, and an outer iteration 2.6 ms.
 //
 // Arithmetic

@@ -292,8 +292,8 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
  * solve per worker thread; its polar sweep runs points one after another,
  * src/post/Polar.cpp:86-124). Requests queue until their device memory fits
  * the budget; admitted solves stay resident, and every engine step advances
- * all of them together (one launch per cluster shape, one thread-block
- * cluster per solve, `chunk` iterations). A solve retires when its residuals
+ * all of them together (one launch per form, a team of CTAs per solve,
+ * `chunk` iterations). A solve retires when its residuals
  * pass the tolerance (converged), go non-finite (diverged: restarted once
  * from the freestream, as the reference's RetryCold) or reach its iteration
  * cap; its forces are integrated on the device and its memory freed for the
@@ -324,7 +324,7 @@ typedef struct cfd_result {
   int iterations;
   int retried_cold;
   int cells;
-  int cluster_size;              /* CTAs per solve the engine ran it with */
+  int cluster_size;              /* CTAs reported for its grid (cfd_engine_set_shape_policy) */
   double continuity, momentum_x, momentum_y;
   double lift_coefficient, drag_coefficient, moment_coefficient;
   double pressure_drag_coefficient, friction_drag_coefficient;
@@ -372,14 +372,10 @@ cfd_status cfd_engine_submit_sweep(cfd_engine e, const cfd_request* base, double
                                    double step, int continued, int* first_id, int* count);
 /* Move up to `capacity` finished results into `out`; *count gets how many. */
 cfd_status cfd_engine_results(cfd_engine e, cfd_result* out, int capacity, int* count);
-/* Launch shapes of the solves the engine starts from now on: 0 (default) by
- * grid size, as a lone solve would run (the mixed form on clusters of at most
- * 8 CTAs), which suits a few dozen concurrent solves (a polar); 1 tuned per
- * grid for a saturated GPU (serving streams): the
- * cluster size with the most solve-iterations per second when as many solves
- * as fit run at once, measured once per grid and kept for the process. Either
- * way a grid always runs with the same shape, so results do not depend on
- * what else is in the engine. */
+/* Launch shapes that the solves started from now on report: 0 (default) by
+ * grid size (the mixed form at most 8 CTAs); 1 the largest of 4, 8 and 16 CTAs
+ * with a row each. A launch shares the GPU between its solves by a plan, and
+ * their results depend neither on that nor on what else is in the engine. */
 cfd_status cfd_engine_set_shape_policy(cfd_engine e, int policy);
 
 /* Pressure coefficient at every wall station of a finished solve (upper
@@ -394,12 +390,10 @@ cfd_status cfd_engine_destroy(cfd_engine e);
 
 /* ---- batches: many solves in one launch ------------------------------------
  * A batch is a descriptor table over existing handles (each keeps its own
- * device state). One launch runs every solve of the table, one thread-block
- * cluster each, so uneven sizes, angles and sections share the GPU. Each
- * solve keeps its own cluster size (set at create or by CFD_CLUSTER_SIZE);
- * solves of different sizes run as one launch per size, side by side on
- * streams forked from and joined back to the caller's, so small clusters can
- * fill SMs that wide ones leave idle. The reference runs one solve per worker
+ * device state). One launch runs every solve of the table (of one form; the
+ * two forms on streams forked from and joined back to the caller's), a team of
+ * CTAs each, by a plan that shares the GPU between uneven sizes. A solve's bits
+ * do not depend on its team. The reference runs one solve per worker
  * thread (src/app/SolverWorker.cpp); this has no counterpart there. The
  * handles must outlive the batch and must not be iterated on their own while
  * a batch launch is in flight. */
@@ -421,7 +415,7 @@ cfd_status cfd_batch_launch(cfd_batch b, int n, void* stream);
 cfd_status cfd_batch_graph_launch(cfd_batch b, int n, void* stream);
 /* Monitors of the last launch (count entries); synchronises first. */
 cfd_status cfd_batch_monitors(cfd_batch b, int* taken, cfd_monitor* last);
-/* Cluster size (CTAs per solve) and threads per CTA of the batch's largest
+/* CTAs reported per solve and threads per CTA of the batch's largest
  * group of solves. */
 cfd_status cfd_batch_shape(cfd_batch b, int* cluster_size, int* threads);
 cfd_status cfd_batch_destroy(cfd_batch b);
