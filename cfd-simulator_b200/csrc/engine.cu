@@ -503,7 +503,7 @@ struct Engine {
         table[offset + static_cast<int>(m)] = I;
         jobs.push_back(s.solver->wideJob());
       }
-      Launch launch{shape.first, offset, shape.second, planWide(jobs, shape.second), plans.size()};
+      Launch launch{shape.first, offset, shape.second, planWide(jobs, shape.second, wideCapacity()), plans.size()};
       const std::size_t ctas = launch.plan.ctas.size() * sizeof(WideCta);
       const std::size_t list = launch.plan.list.size() * sizeof(int);
       plans.resize(plans.size() + ((ctas + list + 15) & ~std::size_t{15}));

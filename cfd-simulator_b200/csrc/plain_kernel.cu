@@ -263,7 +263,7 @@ DEV void plainSolve(const Instance& I, WideTeam& t, int iterations, int stopStag
         const PressureSystem load{I};
         const bool any = (flags & kFlagSharedCg) != 0;
         const WideCgSystem S{I.pD, false, I.x, nullptr, I.spill,
-                             wideCgSpill(I.NI, I.NJ, t.R, t.T, kMaxWideSmem, any), I.cgTol, I.cgMax};
+                             wideCgSpill(I.NI, I.NJ, t.R, t.T, smemBytes, any), I.cgTol, I.cgMax};
         if (flags & kFlagHaloWaitTest) {
           // test: a wait for a count nothing sets, which gives up and reports it
           if (t.tid == 0) {

@@ -860,8 +860,8 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
   while (total < n) {
     const int chunk = std::min(n - total, historyCapacity_);
     const auto launch = (settings_.precision == 1) ? launchSimple : launchPlain;
-    const Status st = launch(dView_, planWide({wideJob()}, threads_), nullptr, nullptr, threads_, chunk, stopStage,
-                             tolerance, stream_);
+    const Status st = launch(dView_, planWide({wideJob()}, threads_, wideCapacity()), nullptr, nullptr, threads_, chunk,
+                             stopStage, tolerance, stream_);
     if (st != CFD_OK) return st;
     CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
     int words[2] = {0, 0};
@@ -1395,7 +1395,7 @@ struct cfd_batch_t {
   int clusterSize{1};              // the most frequent shape (cfd_batch_shape)
   int threads{512};
   int lastIterations{0};
-  cudaGraphExec_t graph{nullptr};  // the n-iteration launch, captured once
+  cudaGraphExec_t graph{nullptr};  // the n-iteration launch, captured once for the groups' plans
   int graphIterations{0};
 };
 
@@ -1408,11 +1408,20 @@ cfd_status refreshTable(cfd_batch b) {
   }
   cudaError_t e = cudaMemcpyAsync(b->dTable, table.data(), table.size() * sizeof(cfdb::Instance),
                                   cudaMemcpyHostToDevice, b->stream);
-  // the groups' plans (a solve's model can change between launches)
+  // the groups' plans (a solve's model can change between launches). A graph has
+  // the grid and the shared memory of the plan it was captured with: with another
+  // plan in its place teams would wait for CTAs that it does not launch, so it is
+  // captured again.
   for (BatchGroup& g : b->groups) {
     std::vector<cfdb::WideJob> jobs;
     for (int k : g.members) jobs.push_back(b->handles[static_cast<std::size_t>(k)]->solver->wideJob());
-    g.plan = cfdb::planWide(jobs, g.threads);
+    cfdb::WidePlan plan = cfdb::planWide(jobs, g.threads, cfdb::wideCapacity());
+    if (g.dList != nullptr && plan == g.plan) continue;
+    if (b->graph != nullptr) {
+      cudaGraphExecDestroy(b->graph);
+      b->graph = nullptr;
+    }
+    g.plan = std::move(plan);
     if (e == cudaSuccess && g.dPlan == nullptr) {
       e = cudaMalloc(reinterpret_cast<void**>(&g.dPlan), cfdb::kMaxWideCtas * sizeof(cfdb::WideCta));
     }
@@ -1428,9 +1437,11 @@ cfd_status refreshTable(cfd_batch b) {
                           b->stream);
     }
   }
-  if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
-  e = cudaStreamSynchronize(b->stream);
-  if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  if (e != cudaSuccess) {
+    for (BatchGroup& g : b->groups) g.plan = cfdb::WidePlan{};  // what the device holds is not known
+    return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  }
   return CFD_OK;
 }
 

@@ -107,9 +107,10 @@ int smemBytes(const WideJob& job, int R, int threads) {
 
 }  // namespace
 
-WidePlan planWide(const std::vector<WideJob>& jobs, int threads) {
+WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity) {
   WidePlan plan;
-  const int capacity = std::max(wideCapacity(), 1), count = static_cast<int>(jobs.size());
+  const int count = static_cast<int>(jobs.size());
+  capacity = std::max(capacity, 1);
   // side by side, each at its widest
   std::vector<int> widths(jobs.size());
   int total = 0;

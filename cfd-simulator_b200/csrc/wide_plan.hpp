@@ -74,9 +74,17 @@ struct WidePlan {
   std::vector<WideCta> ctas;
   std::vector<int> list;  // solves in the order the CTAs' ranges name them
   int smemBytes{0};
+  bool operator==(const WidePlan& o) const {
+    auto same = [](const WideCta& a, const WideCta& b) {
+      return a.begin == b.begin && a.end == b.end && a.rank == b.rank && a.R == b.R;
+    };
+    return smemBytes == o.smemBytes && list == o.list &&
+           std::equal(ctas.begin(), ctas.end(), o.ctas.begin(), o.ctas.end(), same);
+  }
 };
-/// How one launch runs these solves (of one form): side by side when the GPU holds them all
-/// at their widest, else in teams that take one solve after another.
-WidePlan planWide(const std::vector<WideJob>& jobs, int threads);
+/// How one launch runs these solves (of one form) on `capacity` CTAs (wideCapacity()):
+/// side by side when the GPU holds them all at their widest, else in teams that take
+/// one solve after another.
+WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity);
 
 }  // namespace cfdb

@@ -1,0 +1,48 @@
+"""Batches whose plan matters: a captured graph beside changes of plan."""
+import numpy as np
+import pytest
+
+import cfd_b200 as cb
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("U", "V", "P", "MASS_FLUX", "K", "OMEGA", "MUT")
+# (surface, wake, normal): 2 * (surface + wake) - 2 by normal - 1 cells, the grids
+# of test_plans.SIX
+GRIDS = [(168, 84, 56), (109, 54, 56), (237, 118, 133), (107, 53, 61), (102, 50, 186), (55, 27, 153)]
+
+
+def _solver(grid, alpha, **settings):
+    surface, wake, normal = grid
+    mesh = cb.cgrid("0012", surface_points=surface, wake_points=wake, normal_points=normal, first_layer_height=1e-4)
+    s = cb.SimpleSolver.create(mesh, cb.freestream_conditions(mesh, 1.0, alpha),
+                               cb.Settings.defaults(inflow_viscosity_ratio=10.0, **settings))
+    s.set_turbulence_model(cb.MODEL_SST)
+    s.initialise(*cb.uniform_field(mesh, 1.0, alpha, 1.0, 1e6))
+    return s
+
+
+def test_a_graph_is_captured_again_when_the_plan_changes():
+    # SST members that become laminar need another plan (other CTAs, other shared
+    # memory); the graph's next replay must give what direct launches give
+    laminar = (0, 4, 5)
+    make = lambda: [_solver(g, 0.5 * k) for k, g in enumerate(GRIDS)]  # noqa: E731
+    solvers = make()
+    batch = cb.Batch(solvers)
+    batch.graph_launch(1)
+    batch.monitors()
+    for k in laminar:
+        solvers[k].set_turbulence_model(cb.MODEL_LAMINAR)
+    batch.iterate(1)
+    batch.graph_launch(1)
+    taken, _ = batch.monitors()
+    assert taken == [1] * len(solvers)
+    alone = make()
+    for k, s in enumerate(alone):
+        s.iterate(1)
+        if k in laminar:
+            s.set_turbulence_model(cb.MODEL_LAMINAR)
+        s.iterate(2)
+        for f in FIELDS:
+            assert np.array_equal(solvers[k].read(f), s.read(f)), (k, f)
+    batch.close()

@@ -1,0 +1,48 @@
+"""How launches share the GPU, asked of the library's own host code (no GPU):
+plan_check.cu is built against the library and answers queries."""
+import os
+import random
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "cfd-simulator_b200")
+# six SST solves whose plan needs other CTAs, and other shared memory, once the
+# first, fifth and sixth are laminar
+SIX = [(502, 55), (324, 55), (708, 132), (318, 60), (302, 185), (162, 152)]
+
+
+@pytest.fixture(scope="module")
+def ask(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("plan") / "plan_check")
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-fmad=false",
+                    "-I" + os.path.join(PKG, "csrc"), "-I" + os.path.join(ROOT, "include"), "-o", exe,
+                    os.path.join(ROOT, "tests", "plan_check.cu"), os.path.join(PKG, "libcfd_b200.so"),
+                    "-Xlinker", "-rpath", "-Xlinker", PKG], check=True)
+
+    def run(queries):
+        out = subprocess.run([exe], input="\n".join(queries) + "\n", text=True, capture_output=True, check=True).stdout
+        return [[int(v) for v in row.split()] for row in out.splitlines()]
+    return run
+
+
+def plan(jobs, threads=512, capacity=148):
+    return f"plan {capacity} {threads} " + " ".join(f"{ni} {nj} {sst}" for ni, nj, sst in jobs)
+
+
+def test_a_plan_changes_with_a_members_model(ask):
+    before, after = ask([plan([(i, j, 1) for i, j in SIX]),
+                         plan([(i, j, 0 if k in (0, 4, 5) else 1) for k, (i, j) in enumerate(SIX)])])
+    assert before[3] == after[3] == 1
+    assert before[:2] != after[:2]  # so a graph of the one must not replay against the other
+
+
+def test_plans_of_any_batch_are_sound(ask):
+    rng = random.Random(4)
+    queries = []
+    for _ in range(300):
+        jobs = [(2 * rng.randint(10, 400), rng.randint(5, 200), rng.randint(0, 1)) for _ in range(rng.randint(1, 40))]
+        queries.append(plan(jobs, threads=rng.choice([64, 128, 256, 512])))
+    for query, (ctas, smem, teams, ok) in zip(queries, ask(queries)):
+        assert ok == 1 and 1 <= ctas <= 148 and teams >= 1 and 0 < smem <= 222032, query
