@@ -515,6 +515,10 @@ struct Engine {
     if (cudaMemcpy(dTable, table.data(), n * sizeof(Instance), cudaMemcpyHostToDevice) != cudaSuccess) {
       return fail(CFD_INITIALIZATION_FAILURE, "engine table upload failed");
     }
+    // monitors, counts and fault words of the chunk
+    if (cudaMemset(dStatus, 0, n * per * sizeof(double)) != cudaSuccess) {
+      return fail(CFD_INITIALIZATION_FAILURE, "engine status reset failed");
+    }
     if (plans.size() > planBytes) {
       if (dPlans) cudaFree(dPlans);
       planBytes = 2 * plans.size();

@@ -195,8 +195,10 @@ struct Instance {
 
   // ---- outputs ----
   double* history;   // kMonSlots doubles per iteration of the launch
-  int* iterations;   // iterations completed by the launch, then the launch's fault
-                     // word (iterations[1]: nonzero when a bounded wait gave up)
+  int* iterations;   // iterations completed by the launch, then the fault word
+                     // (iterations[1]: nonzero once a bounded wait gave up). Launches
+                     // only add to it and the host clears it once it has read it: a CTA
+                     // can give up before the others of its solve have begun
 
   // ---- mixed form ----
   Multigrid mg;

@@ -181,7 +181,6 @@ DEV void plainSolve(const Instance& I, WideTeam& t, int iterations, int stopStag
   extern __shared__ double dyn[];
   const bool sst = I.model == 2;
   const bool leader = t.rank == 0 && t.tid == 0;
-  if (leader) I.iterations[1] = 0;
   int done = 0;
   const int limit = min(I.iterLimit, iterations);
   const double stopTol = (tolerance >= 0.0) ? tolerance : I.stopTol;

@@ -143,7 +143,6 @@ DEV void mixedSolve(const Instance& I, WideTeam& t, int iterations, int stopStag
                     int flags) {
   const bool sst = (I.model == 2);
   const bool leader = (t.rank == 0 && t.tid == 0);
-  if (leader) I.iterations[1] = 0;
 
   int done = 0;
   const int limit = (I.iterLimit < iterations) ? I.iterLimit : iterations;

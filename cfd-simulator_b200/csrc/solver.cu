@@ -4,6 +4,7 @@
 #include "solver.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -750,6 +751,8 @@ Status Solver::initialise(const double* u, const double* v, const double* p, con
       return st;
     }
   }
+  // a fault of an earlier launch that nobody has read goes with its values
+  CUDA_OR_FAIL(cudaMemset(dIterations_ + 1, 0, sizeof(int)));
   initialised_ = true;
   if (model_ == 2) {
     if ((st = sstInitialise()) != CFD_OK) return st;
@@ -866,7 +869,10 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
     CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
     int words[2] = {0, 0};
     CUDA_OR_FAIL(cudaMemcpy(words, dIterations_, sizeof(words), cudaMemcpyDeviceToHost));
-    if (words[1] != 0) return launchFault(words[1]);
+    if (words[1] != 0) {
+      CUDA_OR_FAIL(cudaMemset(dIterations_ + 1, 0, sizeof(int)));
+      return launchFault(words[1]);
+    }
     const int ran = words[0];
     if (history != nullptr && ran > 0) {
       const std::size_t old = history->size();
@@ -1584,13 +1590,19 @@ cfd_status cfd_batch_monitors(cfd_batch b, int* taken, cfd_monitor* last) {
   if (b == nullptr) return cfdb::fail(CFD_INVALID_ARGUMENT, "null batch");
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  std::vector<std::array<int, 2>> words(b->handles.size());  // iterations, fault word
+  int fault = 0;
+  for (std::size_t k = 0; k < b->handles.size(); ++k) {
+    int* const source = b->handles[k]->solver->deviceView().iterations;
+    e = cudaMemcpy(words[k].data(), source, sizeof(words[k]), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && words[k][1] != 0) e = cudaMemset(source + 1, 0, sizeof(int));
+    if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+    fault |= words[k][1];
+  }
+  if (fault != 0) return cfdb::launchFault(fault);
   for (std::size_t k = 0; k < b->handles.size(); ++k) {
     const cfdb::Instance& I = b->handles[k]->solver->deviceView();
-    int words[2] = {0, 0};
-    e = cudaMemcpy(words, I.iterations, sizeof(words), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
-    if (words[1] != 0) return cfdb::launchFault(words[1]);
-    const int ran = words[0];
+    const int ran = words[k][0];
     if (taken != nullptr) taken[k] = ran;
     if (last != nullptr && ran > 0) {
       double h[cfdb::kMonSlots];

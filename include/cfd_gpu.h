@@ -413,7 +413,8 @@ cfd_status cfd_batch_launch(cfd_batch b, int n, void* stream);
  * and then launched as a graph on `stream` (NULL: the batch's stream). The
  * results are those of cfd_batch_launch. */
 cfd_status cfd_batch_graph_launch(cfd_batch b, int n, void* stream);
-/* Monitors of the last launch (count entries); synchronises first. */
+/* Monitors of the last launch (count entries); synchronises first. Fails with
+ * CFD_INTERNAL when a wait inside any launch since the last call gave up. */
 cfd_status cfd_batch_monitors(cfd_batch b, int* taken, cfd_monitor* last);
 /* CTAs reported per solve and threads per CTA of the batch's largest
  * group of solves. */

@@ -46,3 +46,36 @@ def test_a_graph_is_captured_again_when_the_plan_changes():
         for f in FIELDS:
             assert np.array_equal(solvers[k].read(f), s.read(f)), (k, f)
     batch.close()
+
+
+@pytest.mark.parametrize("precision,flag", [(0, 256), (1, 64)])  # waits that give up, for tests
+def test_a_fault_is_kept_until_it_is_read(precision, flag, monkeypatch):
+    # a later launch must not erase what an earlier one reported: a CTA may give up
+    # before the first CTA of its solve has begun
+    solvers = [_solver((55, 27, 20), 1.0, precision=precision) for _ in range(2)]
+    batch = cb.Batch(solvers)
+    monkeypatch.setenv("CFD_KERNEL_FLAGS", str(flag))
+    batch.launch(1)
+    monkeypatch.delenv("CFD_KERNEL_FLAGS")
+    batch.launch(1)
+    with pytest.raises(cb.CfdError) as err:
+        batch.monitors()
+    assert err.value.code == 8  # CFD_INTERNAL
+    # read once, for every solve of the batch
+    taken, last = batch.iterate(1)
+    assert taken == [1, 1] and all(np.isfinite(m.continuity) for m in last)
+    assert np.isfinite(solvers[1].iterate(1).continuity)
+    batch.close()
+
+
+def test_a_new_start_drops_an_unread_fault(monkeypatch):
+    s = _solver((55, 27, 20), 1.0)
+    batch = cb.Batch([s])
+    monkeypatch.setenv("CFD_KERNEL_FLAGS", "256")
+    batch.launch(1)
+    monkeypatch.delenv("CFD_KERNEL_FLAGS")
+    import torch
+    torch.cuda.synchronize()
+    s.initialise(*cb.uniform_field(s.mesh, 1.0, 1.0, 1.0, 1e6))
+    assert np.isfinite(s.iterate(1).continuity)
+    batch.close()
