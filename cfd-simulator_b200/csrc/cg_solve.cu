@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(kWideThreads, 1) wideCgKernel(WideCgArgs A) {
     return;
   }
   WideTeam t;
-  wideJoin(t, A.mem, faultWord, &sh, blockIdx.x, gridDim.x, A.NI, A.NJ, 0);
+  if (threadIdx.x == 0) sh.ahead = 0.0;
+  wideJoin(t, A.mem, faultWord, &sh, blockIdx.x, gridDim.x, A.NI, A.NJ, 0,
+           outerBound(A.NI, A.NJ, static_cast<int>(gridDim.x), static_cast<int>(blockDim.x), WideEffort{1.0, 0.0, 0}));
   const WideCgSystem S{A.diag, anywhere, A.x, A.u, A.spill, A.spillStride, A.tolerance, A.cap};
   const WideCgResult out = wideCg(t, S, load, A.smemBytes, false);
   wideLeave(t);

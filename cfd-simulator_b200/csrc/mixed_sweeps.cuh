@@ -434,7 +434,7 @@ DEV bool chainReady(unsigned long long word, unsigned tag) { return static_cast<
 DEV float chainValue(unsigned long long word) { return __uint_as_float(static_cast<unsigned>(word)); }
 /// The value of a message.
 DEV float chainWait(WideTeam& t, const unsigned long long* from, unsigned long long word, unsigned tag) {
-  int polls = 0;
+  long long polls = 0;
   while (!chainReady(word, tag)) {
     if (wideGiveUp(t, polls, kFaultChainWait)) return 0.0f;
     word = chainLoad(from);
@@ -497,7 +497,7 @@ __device__ __noinline__ void rowChain(const Instance& I, WideTeam& team, const f
 #pragma unroll
     for (int e = 0; e < CELLS; ++e) value[e] = 0.0f;
     if (hasOld && j < NJ) {
-      int polls = 0;
+      long long polls = 0;
       for (;;) {
         bool ready = true;
 #pragma unroll

@@ -107,7 +107,8 @@ DEV double edgeWait(WideTeam& t, volatile unsigned long long* slot, unsigned tag
       return __longlong_as_double(static_cast<long long>((a & 0xffffffffull) | (b << 32)));
     }
     if (*static_cast<volatile int*>(&t.sh->fault) != 0) return 0.0;
-    if (spins > (1LL << 24)) {
+    // looks on chip, eight and more to an L2 round trip
+    if (spins > 8LL * kWideSpinLimit && spins > 8 * t.sh->spinLimit) {
       t.sh->fault = 1;
       atomicOr(t.faultWord, kFaultChainWait);
       return 0.0;
@@ -119,7 +120,8 @@ DEV double edgeWait(WideTeam& t, volatile unsigned long long* slot, unsigned tag
 DEV void edgeRoom(WideTeam& t, volatile int* progress, int rows) {
   for (long long spins = 0; *progress < rows; ++spins) {
     if (*static_cast<volatile int*>(&t.sh->fault) != 0) return;
-    if (spins > (1LL << 24)) {
+    // looks on chip, eight and more to an L2 round trip
+    if (spins > 8LL * kWideSpinLimit && spins > 8 * t.sh->spinLimit) {
       t.sh->fault = 1;
       atomicOr(t.faultWord, kFaultChainWait);
       return;
@@ -201,7 +203,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
     if (!exists) return 0.0;
     const ulonglong2* slot = in + static_cast<long long>(j) * z.padded + place;
     ulonglong2 m = first;
-    int polls = 0;
+    long long polls = 0;
     while (!messageReady(m, tag)) {
       if (wideGiveUp(t, polls, kFaultChainWait)) return 0.0;
       m = messageLoad(slot);
@@ -310,7 +312,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
           const int place = rowSweepPlace(z, a);
           const ulonglong2* slot = ((a < i) ? out : in) + place;
           ulonglong2 m = messageLoad(slot);
-          int polls = 0;
+          long long polls = 0;
           while (!messageReady(m, tag) && !wideGiveUp(t, polls, kFaultChainWait)) m = messageLoad(slot);
           partner = messageValue(m);
         }
@@ -405,7 +407,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
             // this lane's own value of the row before
             const ulonglong2* slot = out + static_cast<long long>(j - 1) * z.padded + at;
             ulonglong2 m = messageLoad(slot);
-            int polls = 0;
+            long long polls = 0;
             while (!messageReady(m, tag) && !wideGiveUp(t, polls, kFaultChainWait)) m = messageLoad(slot);
             south[e] = messageValue(m);
           }

@@ -337,14 +337,22 @@ simpleKernel(const Instance* __restrict__ instances, const WideCta* __restrict__
   __shared__ WideShared sh;
   const WideCta me = (plan != nullptr) ? plan[blockIdx.x]
                                        : WideCta{0, 1, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)};
+  if (threadIdx.x == 0) sh.ahead = 0.0;
   for (int k = me.begin; k < me.end; ++k) {
     const Instance& I = instances[(list != nullptr) ? list[k] : k];
     const int R = min(me.R, I.wideMost);
-    if (me.rank >= R) continue;
+    const double outer = outerBound(I.NI, I.NJ, R, static_cast<int>(blockDim.x),
+                                    wideEffort(true, I.nCorr, I.cgMax, I.mgCap, I.sweeps));
+    if (me.rank >= R) {
+      // the rest of the team is at work on it: a wait of the next one is behind that
+      if (threadIdx.x == 0) sh.ahead += outer;
+      continue;
+    }
     WideTeam t;
-    wideJoin(t, I.wide, I.iterations + 1, &sh, me.rank, R, I.NI, I.NJ, iterations * (me.end - me.begin - 1));
+    wideJoin(t, I.wide, I.iterations + 1, &sh, me.rank, R, I.NI, I.NJ, iterations, outer);
     mixedSolve(I, t, iterations, stopStage, tolerance, smemBytes, flags);
     wideLeave(t);
+    if (t.tid == 0) sh.ahead += outer;
     __syncthreads();
   }
 }

@@ -35,11 +35,41 @@ constexpr int kChunkCells = 256;  // cells whose sums are formed together, by as
 constexpr int kChunkBatch = 16;   // chunks of a CTA whose partial sums are held at once
 constexpr int kMaxSums = 4;
 constexpr int kWideThreads = 512;
-/// Polls before a wait gives up, each an L2 round trip (0.4 us or more): ~1 s,
-/// and ~15 ms more for every iteration of every solve that a CTA may wait for
-/// its team to finish first.
+/// Polls before a wait gives up, each an L2 round trip (0.4 us or more): ~1 s, and
+/// four times the bound below for what a CTA may have to wait for: its own solve's
+/// phases, and the earlier solves of its team that it has no part in.
 constexpr int kWideSpinLimit = 1 << 21;
-constexpr int kWideSpinPerIteration = 1 << 15;
+constexpr double kWidePollsPerMicrosecond = 4.0 / 0.4;
+
+/// What a solve's settings let one outer iteration do.
+struct WideEffort {
+  double exchanges;  // of the CG (plain form)
+  double cycles;     // of the multigrid (mixed form)
+  int sweeps;        // of the momentum system
+};
+__host__ __device__ inline WideEffort wideEffort(bool mixed, int corrections, int cgMax, int mgCap, int sweeps) {
+  const double passes = (corrections > 1) ? corrections : 1;
+  return WideEffort{mixed ? 0.0 : passes * (cgMax + 1.0), mixed ? passes * (mgCap + 3.0) : 0.0, sweeps};
+}
+/// Microseconds that one outer iteration of a solve takes at most on R CTAs of T
+/// threads, per cell of a thread where it streams. Measured at 768x192: a CG
+/// exchange 5.9 us on 148 CTAs (2 cells a thread), 12 on 37, 30 on 24 and 88 on 12
+/// (24 cells), bounded by 5 + 5 a cell; a V-cycle 38 us, by 200 + 20; the rows of
+/// the sweeps 1.1 to 3.5 us each, by 5 + 5 a cell of the row for each of the six.
+__host__ __device__ inline double outerBound(int NI, int NJ, int R, int T, const WideEffort& e) {
+  const double cells = static_cast<double>(NI) * NJ / (static_cast<double>(R) * T) + 1.0;
+  double us = 1000.0 + e.exchanges * (5.0 + 5.0 * cells) + e.cycles * (200.0 + 20.0 * cells);
+  us += (50.0 + 2.0 * e.sweeps) * (2.0 + 2.0 * cells) + 6.0 * NJ * (10.0 + 5.0 * NI / T);
+  if (e.cycles > 0.0) {  // as wavefronts of diagonals
+    us += 6.0 * (static_cast<double>(NI) + NJ) * (2.0 + 2.0 * ((NI < NJ) ? NI : NJ) / T);
+  }
+  return us;
+}
+/// Polls of a wait behind `microseconds` of other work.
+__host__ __device__ inline long long wideSpinLimit(double microseconds) {
+  const double polls = kWideSpinLimit + kWidePollsPerMicrosecond * microseconds;
+  return (polls < 1e18) ? static_cast<long long>(polls) : 1000000000000000000LL;
+}
 
 constexpr int kUnitBatch = 8;       // units of the CG whose partial sums are held at once
 constexpr int kUnitWarps = 8;       // warps that share a unit
@@ -54,6 +84,8 @@ struct WideShared {
   };
   double warpPart[kWideThreads / 32][kRedSlots];
   double result[kRedSlots];
+  double ahead;    // microseconds an iteration of the earlier solves of the CTA's list, at most
+  long long spinLimit;
   int fault;       // a wait of this CTA gave up
   unsigned never;  // stays 0: the wait tests' condition
 };
@@ -66,14 +98,15 @@ struct WideTeam {
   int c0, c1;            // own cells: whole chunks
   unsigned epoch;
   unsigned barriers;  // of this launch so far
-  int spinLimit;
   WideScratch mem;
   int* faultWord;
   WideShared* sh;
 };
 
+/// `iterations` of this solve, each of `outer` microseconds at most, behind as many
+/// of the solves before it (sh->ahead).
 DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShared* sh, int rank, int R, int NI,
-                  int NJ, int iterationsAhead) {
+                  int NJ, int iterations, double outer) {
   t.rank = rank;
   t.R = R;
   t.tid = static_cast<int>(threadIdx.x);
@@ -87,7 +120,6 @@ DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShare
   t.c0 = t.chunk0 * kChunkCells;
   t.c1 = min(t.chunk1 * kChunkCells, t.N);
   if (t.c0 > t.c1) t.c0 = t.c1;
-  t.spinLimit = kWideSpinLimit + kWideSpinPerIteration * min(iterationsAhead, 32768);
   t.mem = mem;
   t.faultWord = faultWord;
   t.sh = sh;
@@ -95,6 +127,7 @@ DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShare
   t.barriers = 0u;
   __syncthreads();
   if (t.tid == 0) {
+    sh->spinLimit = wideSpinLimit(outer + iterations * sh->ahead);
     sh->fault = 0;
     sh->never = 0u;
   }
@@ -119,9 +152,9 @@ DEV void wideLeave(WideTeam& t) {
 }
 
 /// One more unsuccessful poll: true when the wait is over (given up now or before).
-DEV bool wideGiveUp(WideTeam& t, int& polls, int code) {
+DEV bool wideGiveUp(WideTeam& t, long long& polls, int code) {
   if (*static_cast<volatile int*>(&t.sh->fault) != 0) return true;
-  if (++polls < t.spinLimit) return false;
+  if (++polls < *static_cast<volatile long long*>(&t.sh->spinLimit)) return false;
   t.sh->fault = 1;
   atomicOr(t.faultWord, code);
   return true;
@@ -149,7 +182,7 @@ DEV double messageValue(const ulonglong2& m) {
 }
 /// Wait for the value of `slot` with this tag, given a first look at it.
 DEV double messageWait(WideTeam& t, const ulonglong2* slot, ulonglong2 m, unsigned tag, int code) {
-  int polls = 0;
+  long long polls = 0;
   while (!messageReady(m, tag)) {
     if (wideGiveUp(t, polls, code)) return 0.0;
     m = messageLoad(slot);
@@ -159,7 +192,7 @@ DEV double messageWait(WideTeam& t, const ulonglong2* slot, ulonglong2 m, unsign
 /// The value of a message; `code` is the fault of a wait that gives up.
 DEV double messageWait(WideTeam& t, const ulonglong2* slot, unsigned tag, int code) {
   ulonglong2 m = messageLoad(slot);
-  int polls = 0;
+  long long polls = 0;
   while (!messageReady(m, tag)) {
     if (wideGiveUp(t, polls, code)) return 0.0;
     m = messageLoad(slot);
@@ -175,7 +208,7 @@ DEV void messageWaitAll(WideTeam& t, const ulonglong2* set, const int (&from)[N]
   unsigned missing = 0;
 #pragma unroll
   for (int k = 0; k < N; ++k) missing |= (from[k] >= 0) ? 1u << k : 0u;
-  int polls = 0;
+  long long polls = 0;
   while (missing != 0u) {
     ulonglong2 m[N];
 #pragma unroll
@@ -210,7 +243,7 @@ DEV void wideBarrier(WideTeam& t) {
   if (t.tid == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.mem.arrived) : "memory");
     const unsigned all = t.barriers * static_cast<unsigned>(t.R);
-    int polls = 0;
+    long long polls = 0;
     for (;;) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.mem.arrived) : "memory");

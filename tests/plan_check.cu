@@ -3,11 +3,17 @@
 //
 //   plan CAPACITY THREADS {NI NJ SST}...   CTAs, shared memory, teams of the plain
 //                                          form's plan; 1 if the plan is sound
+//   teams CAPACITY THREADS {NI NJ SST}...  its teams: the solves in order as solve
+//                                          CTAs pairs, -1 after each team
+//   waits CAPACITY THREADS ITERATIONS CAP {NI NJ SST}...  of any CTA's longest wait
+//                                          for the solves before its own, as
+//                                          modelled, the permille of its limit
 #include <cstdio>
 #include <iostream>
 #include <sstream>
 #include <string>
 
+#include "wide_cg.cuh"
 #include "wide_plan.hpp"
 
 using namespace cfdb;
@@ -37,6 +43,32 @@ bool sound(const WidePlan& plan, const std::vector<WideJob>& jobs) {
   return plan.list.size() == jobs.size();
 }
 
+int ctasOf(const WideJob& job, int width, int threads) {
+  return wideUsefulCtas(job.NI, job.NJ, std::min(width, job.most), threads);
+}
+
+/// Modelled milliseconds of `iterations` of a solve with `cap` CG iterations each.
+double milliseconds(const WideJob& job, int R, int iterations, int cap) {
+  return 1e-3 * iterations * (cap * wideCgMicroseconds(job.NI, job.NJ, R) + (job.sst ? 1.5 * job.NJ : 0.0));
+}
+
+double waits(const WidePlan& plan, const std::vector<WideJob>& jobs, int threads, int iterations, int cap) {
+  double worst = 0.0;
+  for (const WideCta& c : plan.ctas) {
+    double behind = 0.0, ahead = 0.0;
+    for (int k = c.begin; k < c.end; ++k) {
+      const WideJob& job = jobs[static_cast<std::size_t>(plan.list[static_cast<std::size_t>(k)])];
+      const int R = ctasOf(job, c.R, threads);
+      const double outer = outerBound(job.NI, job.NJ, R, threads, wideEffort(false, 1, cap, 16, 3));
+      // a poll is 0.4 us at least
+      worst = std::max(worst, behind / (wideSpinLimit(outer + iterations * ahead) * 0.4e-3));
+      behind += milliseconds(job, R, iterations, cap);
+      ahead += outer;
+    }
+  }
+  return worst;
+}
+
 }  // namespace
 
 int main() {
@@ -45,14 +77,31 @@ int main() {
     std::istringstream in(line);
     std::string what;
     in >> what;
-    if (what == "plan") {
-      int capacity = 0, threads = 0;
+    if (what == "plan" || what == "teams" || what == "waits") {
+      int capacity = 0, threads = 0, iterations = 0, cap = 0;
       in >> capacity >> threads;
+      if (what == "waits") in >> iterations >> cap;
       std::vector<WideJob> jobs;
       for (int NI, NJ, sst; in >> NI >> NJ >> sst;) {
         jobs.push_back(WideJob{NI, NJ, wideMostCtas(NI, NJ, threads), sst != 0, 0});
       }
       const WidePlan plan = planWide(jobs, threads, capacity);
+      if (what == "waits") {
+        std::printf("%d\n", static_cast<int>(1000.0 * waits(plan, jobs, threads, iterations, cap)));
+        continue;
+      }
+      if (what == "teams") {
+        for (const WideCta& c : plan.ctas) {
+          if (c.rank != 0) continue;
+          for (int k = c.begin; k < c.end; ++k) {
+            const int job = plan.list[static_cast<std::size_t>(k)];
+            std::printf("%d %d ", job, ctasOf(jobs[static_cast<std::size_t>(job)], c.R, threads));
+          }
+          std::printf("-1 ");
+        }
+        std::printf("\n");
+        continue;
+      }
       int teams = 0;
       for (const WideCta& c : plan.ctas) teams += (c.rank == 0) ? 1 : 0;
       std::printf("%zu %d %d %d\n", plan.ctas.size(), plan.smemBytes, teams, sound(plan, jobs) ? 1 : 0);

@@ -79,3 +79,29 @@ def test_a_new_start_drops_an_unread_fault(monkeypatch):
     s.initialise(*cb.uniform_field(s.mesh, 1.0, 1.0, 1.0, 1e6))
     assert np.isfinite(s.iterate(1).continuity)
     batch.close()
+
+
+def test_a_wide_solve_waits_behind_a_long_narrow_one():
+    # the plan gives solve 2 (490x73) to the 74 CTAs of which 12 first run solve 0
+    # (50x94): the others wait in solve 2's first barrier for all of that, here
+    # seconds, and must not give up
+    import time
+    narrow = dict(pressure_iterations=300, pressure_tolerance=0.0, non_orthogonal_correctors=120,
+                  pressure_relaxation=0.01)
+    make = lambda: ([_solver((17, 9, 95), float(k), **narrow) for k in range(2)] +  # noqa: E731
+                    [_solver((164, 82, 74), float(k)) for k in range(2)])
+    iterations = 32
+    together, alone = make(), make()
+    for s in together[2:] + alone[2:]:
+        s.set_turbulence_model(cb.MODEL_LAMINAR)
+    batch = cb.Batch(together)
+    start = time.perf_counter()
+    taken, _ = batch.iterate(iterations)
+    assert time.perf_counter() - start > 2.0  # longer than any fixed second
+    assert taken == [iterations] * 4
+    for k in (0, 2, 3):
+        s = alone[k]
+        s.iterate(iterations)
+        for f in FIELDS[:4]:
+            assert np.array_equal(together[k].read(f), s.read(f)), (k, f)
+    batch.close()

@@ -46,3 +46,19 @@ def test_plans_of_any_batch_are_sound(ask):
         queries.append(plan(jobs, threads=rng.choice([64, 128, 256, 512])))
     for query, (ctas, smem, teams, ok) in zip(queries, ask(queries)):
         assert ok == 1 and 1 <= ctas <= 148 and teams >= 1 and 0 < smem <= 222032, query
+
+
+def test_a_wait_behind_other_solves_stays_within_its_limit(ask):
+    # a CTA that has no part in a solve waits for it in the next one
+    cases = [(32, 200, [(1500, 700, 1)] * 8 + [(1600, 400, 1)] * 8),
+             (32, 200, [(1400, 380, 1)] * 12 + [(2400, 600, 1)] * 12),
+             (256, 200, [(768, 192, 1)] * 21 + [(192, 48, 1), (384, 96, 1), (768, 192, 1)]),
+             (256, 2000, [(768, 192, 1)] * 21 + [(192, 48, 1), (384, 96, 1), (768, 192, 1)]),
+             (8, 100000, [(768, 192, 1)] * 4 + [(384, 96, 0)] * 9)]
+    rng = random.Random(7)
+    for _ in range(100):
+        jobs = [(2 * rng.randint(10, 1500), rng.randint(5, 900), rng.randint(0, 1)) for _ in range(rng.randint(2, 30))]
+        cases.append((rng.choice([1, 32, 256]), rng.choice([50, 200, 2000, 50000]), jobs))
+    queries = [plan(jobs).replace("plan 148 512", f"waits 148 512 {n} {cap}") for n, cap, jobs in cases]
+    for query, (permille,) in zip(queries, ask(queries)):
+        assert permille <= 500, query
