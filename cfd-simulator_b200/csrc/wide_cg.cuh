@@ -54,8 +54,8 @@ constexpr int kUnitThreads = 32 * kUnitWarps;
 /// units included), for teams of `team` threads.
 __host__ __device__ inline WideCgShape wideCgTiles(int NI, int NJ, int columnTiles, int team) {
   WideCgShape s;
-  s.columnTiles = columnTiles;
-  s.width = (NI + s.columnTiles - 1) / s.columnTiles;
+  s.width = (NI + columnTiles - 1) / columnTiles;
+  s.columnTiles = (NI + s.width - 1) / s.width;  // as many as hold a column at that width
   s.passes = (s.width + team - 1) / team;
   s.G = ((s.width + s.passes - 1) / s.passes + 31) / 32 * 32;
   s.groups = team / s.G;

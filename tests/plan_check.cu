@@ -5,6 +5,9 @@
 //                                          form's plan; 1 if the plan is sound
 //   teams CAPACITY THREADS {NI NJ SST}...  its teams: the solves in order as solve
 //                                          CTAs pairs, -1 after each team
+//   tiles THREADS NJ NI0 NI1               blocks of NI0 .. NI1 columns with a column
+//                                          tile that holds no column, or more units
+//                                          than sums are kept of; the first of them
 //   waits CAPACITY THREADS ITERATIONS CAP {NI NJ SST}...  of any CTA's longest wait
 //                                          for the solves before its own, as
 //                                          modelled, the permille of its limit
@@ -77,7 +80,18 @@ int main() {
     std::istringstream in(line);
     std::string what;
     in >> what;
-    if (what == "plan" || what == "teams" || what == "waits") {
+    if (what == "tiles") {
+      int threads = 0, NJ = 0, first = 0, last = 0, bad = 0, where = 0;
+      in >> threads >> NJ >> first >> last;
+      for (int NI = first; NI <= last; ++NI) {
+        const WideCgShape s = wideCgShape(NI, NJ, kMaxWideCtas, threads);
+        const bool ok = s.columnTiles >= 1 && s.columnTiles <= kMaxColumnTiles && (s.columnTiles - 1) * s.width < NI &&
+                        s.columnTiles * s.width >= NI && s.columnTiles * s.unitRows <= kMaxUnits &&
+                        s.unitRows * s.B >= NJ && (s.unitRows - 1) * s.B < NJ;
+        if (!ok && bad++ == 0) where = NI;
+      }
+      std::printf("%d %d\n", bad, where);
+    } else if (what == "plan" || what == "teams" || what == "waits") {
       int capacity = 0, threads = 0, iterations = 0, cap = 0;
       in >> capacity >> threads;
       if (what == "waits") in >> iterations >> cap;

@@ -62,3 +62,10 @@ def test_a_wait_behind_other_solves_stays_within_its_limit(ask):
     queries = [plan(jobs).replace("plan 148 512", f"waits 148 512 {n} {cap}") for n, cap, jobs in cases]
     for query, (permille,) in zip(queries, ask(queries)):
         assert permille <= 500, query
+
+
+def test_every_column_tile_holds_columns(ask):
+    # the plain CG's tiling, for every block size up to 5,000 columns and any threads
+    queries = [f"tiles {threads} {nj} 1 5000" for threads in range(32, 513, 32) for nj in (1, 6, 48, 192, 400, 3000)]
+    for query, (bad, where) in zip(queries, ask(queries)):
+        assert bad == 0, (query, bad, where)
