@@ -434,9 +434,9 @@ DEV bool chainReady(unsigned long long word, unsigned tag) { return static_cast<
 DEV float chainValue(unsigned long long word) { return __uint_as_float(static_cast<unsigned>(word)); }
 /// The value of a message.
 DEV float chainWait(WideTeam& t, const unsigned long long* from, unsigned long long word, unsigned tag) {
-  long long polls = 0;
+  int polls = 0;
   while (!chainReady(word, tag)) {
-    if (wideGiveUp(t, polls, kFaultChainWait)) return 0.0f;
+    if (wideGiveUpFar(t, polls, kFaultChainWait)) return 0.0f;
     word = chainLoad(from);
   }
   return chainValue(word);
@@ -497,12 +497,12 @@ __device__ __noinline__ void rowChain(const Instance& I, WideTeam& team, const f
 #pragma unroll
     for (int e = 0; e < CELLS; ++e) value[e] = 0.0f;
     if (hasOld && j < NJ) {
-      long long polls = 0;
+      int polls = 0;
       for (;;) {
         bool ready = true;
 #pragma unroll
         for (int e = 0; e < CELLS; ++e) ready = ready && (e >= exists || chainReady(raw[e], tag));
-        if (ready || wideGiveUp(t, polls, kFaultChainWait)) break;
+        if (ready || wideGiveUpFar(t, polls, kFaultChainWait)) break;
         chainLoad<CELLS>(slot(j), raw);
       }
 #pragma unroll

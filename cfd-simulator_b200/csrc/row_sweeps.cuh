@@ -93,6 +93,9 @@ DEV void rowSweepStoreRow(const RowSweepSystem& y, const RowSweepShape& z, int N
   messageStore(y.values + static_cast<long long>(j) * z.padded + place, x, tag);
 }
 
+/// Polls of shared memory after which a wait is overdue: eight and more to one of L2.
+constexpr unsigned kEdgePolls = 1u << 24;
+
 /// A chunk's last value of a row, tagged j + 1, in shared memory.
 DEV void edgeStore(volatile unsigned long long* slot, double v, unsigned tag) {
   const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
@@ -101,31 +104,21 @@ DEV void edgeStore(volatile unsigned long long* slot, double v, unsigned tag) {
   slot[1] = t | (bits >> 32);
 }
 DEV double edgeWait(WideTeam& t, volatile unsigned long long* slot, unsigned tag) {
-  for (long long spins = 0;; ++spins) {
+  int polls = 0;
+  for (;;) {
     const unsigned long long a = slot[0], b = slot[1];
     if (static_cast<unsigned>(a >> 32) == tag && static_cast<unsigned>(b >> 32) == tag) {
       return __longlong_as_double(static_cast<long long>((a & 0xffffffffull) | (b << 32)));
     }
-    if (*static_cast<volatile int*>(&t.sh->fault) != 0) return 0.0;
-    // looks on chip, eight and more to an L2 round trip
-    if (spins > 8LL * kWideSpinLimit && spins > 8 * t.sh->spinLimit) {
-      t.sh->fault = 1;
-      atomicOr(t.faultWord, kFaultChainWait);
-      return 0.0;
-    }
+    if (wideGiveUp<kEdgePolls>(t, polls, kFaultChainWait)) return 0.0;
   }
 }
 
 /// Wait until the next chunk has taken the edges of `rows` rows.
 DEV void edgeRoom(WideTeam& t, volatile int* progress, int rows) {
-  for (long long spins = 0; *progress < rows; ++spins) {
-    if (*static_cast<volatile int*>(&t.sh->fault) != 0) return;
-    // looks on chip, eight and more to an L2 round trip
-    if (spins > 8LL * kWideSpinLimit && spins > 8 * t.sh->spinLimit) {
-      t.sh->fault = 1;
-      atomicOr(t.faultWord, kFaultChainWait);
-      return;
-    }
+  int polls = 0;
+  while (*progress < rows) {
+    if (wideGiveUp<kEdgePolls>(t, polls, kFaultChainWait)) return;
   }
 }
 
@@ -203,7 +196,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
     if (!exists) return 0.0;
     const ulonglong2* slot = in + static_cast<long long>(j) * z.padded + place;
     ulonglong2 m = first;
-    long long polls = 0;
+    int polls = 0;
     while (!messageReady(m, tag)) {
       if (wideGiveUp(t, polls, kFaultChainWait)) return 0.0;
       m = messageLoad(slot);
@@ -312,7 +305,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
           const int place = rowSweepPlace(z, a);
           const ulonglong2* slot = ((a < i) ? out : in) + place;
           ulonglong2 m = messageLoad(slot);
-          long long polls = 0;
+          int polls = 0;
           while (!messageReady(m, tag) && !wideGiveUp(t, polls, kFaultChainWait)) m = messageLoad(slot);
           partner = messageValue(m);
         }
@@ -407,7 +400,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
             // this lane's own value of the row before
             const ulonglong2* slot = out + static_cast<long long>(j - 1) * z.padded + at;
             ulonglong2 m = messageLoad(slot);
-            long long polls = 0;
+            int polls = 0;
             while (!messageReady(m, tag) && !wideGiveUp(t, polls, kFaultChainWait)) m = messageLoad(slot);
             south[e] = messageValue(m);
           }

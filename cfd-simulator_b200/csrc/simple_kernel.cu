@@ -352,7 +352,6 @@ simpleKernel(const Instance* __restrict__ instances, const WideCta* __restrict__
     wideJoin(t, I.wide, I.iterations + 1, &sh, me.rank, R, I.NI, I.NJ, iterations, outer);
     mixedSolve(I, t, iterations, stopStage, tolerance, smemBytes, flags);
     wideLeave(t);
-    if (t.tid == 0) sh.ahead += outer;
     __syncthreads();
   }
 }

@@ -35,11 +35,9 @@ constexpr int kChunkCells = 256;  // cells whose sums are formed together, by as
 constexpr int kChunkBatch = 16;   // chunks of a CTA whose partial sums are held at once
 constexpr int kMaxSums = 4;
 constexpr int kWideThreads = 512;
-/// Polls before a wait gives up, each an L2 round trip (0.4 us or more): ~1 s, and
-/// four times the bound below for what a CTA may have to wait for: its own solve's
-/// phases, and the earlier solves of its team that it has no part in.
+/// Polls after which a wait is overdue, each an L2 round trip (0.4 us or more): ~1 s.
+/// From there on it goes by the clock (wideWaitLimit).
 constexpr int kWideSpinLimit = 1 << 21;
-constexpr double kWidePollsPerMicrosecond = 4.0 / 0.4;
 
 /// What a solve's settings let one outer iteration do.
 struct WideEffort {
@@ -65,10 +63,12 @@ __host__ __device__ inline double outerBound(int NI, int NJ, int R, int T, const
   }
   return us;
 }
-/// Polls of a wait behind `microseconds` of other work.
-__host__ __device__ inline long long wideSpinLimit(double microseconds) {
-  const double polls = kWideSpinLimit + kWidePollsPerMicrosecond * microseconds;
-  return (polls < 1e18) ? static_cast<long long>(polls) : 1000000000000000000LL;
+/// How long an overdue wait still waits behind `microseconds` of other work (its own
+/// solve's phases, and the earlier solves of its team that it has no part in): two
+/// seconds and four times that, in 2^20 ns.
+__host__ __device__ inline int wideWaitLimit(double microseconds) {
+  const double limit = 2000.0 + 4.0e-3 * microseconds;
+  return (limit < 5e8) ? static_cast<int>(limit) : 500000000;
 }
 
 constexpr int kUnitBatch = 8;       // units of the CG whose partial sums are held at once
@@ -85,7 +85,7 @@ struct WideShared {
   double warpPart[kWideThreads / 32][kRedSlots];
   double result[kRedSlots];
   double ahead;    // microseconds an iteration of the earlier solves of the CTA's list, at most
-  long long spinLimit;
+  int waitLimit;
   int fault;       // a wait of this CTA gave up
   unsigned never;  // stays 0: the wait tests' condition
 };
@@ -127,7 +127,8 @@ DEV void wideJoin(WideTeam& t, const WideScratch& mem, int* faultWord, WideShare
   t.barriers = 0u;
   __syncthreads();
   if (t.tid == 0) {
-    sh->spinLimit = wideSpinLimit(outer + iterations * sh->ahead);
+    sh->waitLimit = wideWaitLimit(outer + iterations * sh->ahead);
+    sh->ahead += outer;
     sh->fault = 0;
     sh->never = 0u;
   }
@@ -151,14 +152,34 @@ DEV void wideLeave(WideTeam& t) {
   }
 }
 
-/// One more unsuccessful poll: true when the wait is over (given up now or before).
-DEV bool wideGiveUp(WideTeam& t, long long& polls, int code) {
-  if (*static_cast<volatile int*>(&t.sh->fault) != 0) return true;
-  if (++polls < *static_cast<volatile long long*>(&t.sh->spinLimit)) return false;
-  t.sh->fault = 1;
-  atomicOr(t.faultWord, code);
-  return true;
+/// An overdue wait: `polls` counted up to its number, from then on it holds the time
+/// that was, below 0. The next `polls`, or 0 when the wait is given up.
+DEV int wideOverdue(WideShared* sh, int* faultWord, int polls, int code) {
+  constexpr int kLowest = -2147483647 - 1, kTime = (1 << 30) - 1;
+  unsigned long long ns;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(ns));
+  const int now = static_cast<int>(ns >> 20) & kTime;
+  if (polls > 0) return kLowest + now;
+  if (((now - (polls - 1 - kLowest)) & kTime) < *static_cast<volatile int*>(&sh->waitLimit)) return polls - 1;
+  *static_cast<volatile int*>(&sh->fault) = 1;
+  atomicOr(faultWord, code);
+  return 0;
 }
+static __device__ __noinline__ int wideOverdueFar(WideShared* sh, int* faultWord, int polls, int code) {
+  return wideOverdue(sh, faultWord, polls, code);
+}
+/// One more unsuccessful poll: true when the wait is over (given up now or before).
+/// kFar: what an overdue wait does lies in a function of its own. The mixed form's
+/// waits and the barrier are 1 % of an iteration faster so, the CG's 8 % slower
+/// (192x48), whose registers a call would spill.
+template <unsigned kPolls = static_cast<unsigned>(kWideSpinLimit), bool kFar = false>
+DEV bool wideGiveUp(WideTeam& t, int& polls, int code) {
+  if (*static_cast<volatile int*>(&t.sh->fault) != 0) return true;
+  if (static_cast<unsigned>(++polls) < kPolls) return false;
+  polls = kFar ? wideOverdueFar(t.sh, t.faultWord, polls, code) : wideOverdue(t.sh, t.faultWord, polls, code);
+  return polls == 0;
+}
+DEV bool wideGiveUpFar(WideTeam& t, int& polls, int code) { return wideGiveUp<kWideSpinLimit, true>(t, polls, code); }
 
 // ---- tagged messages ------------------------------------------------------------
 
@@ -182,7 +203,7 @@ DEV double messageValue(const ulonglong2& m) {
 }
 /// Wait for the value of `slot` with this tag, given a first look at it.
 DEV double messageWait(WideTeam& t, const ulonglong2* slot, ulonglong2 m, unsigned tag, int code) {
-  long long polls = 0;
+  int polls = 0;
   while (!messageReady(m, tag)) {
     if (wideGiveUp(t, polls, code)) return 0.0;
     m = messageLoad(slot);
@@ -192,7 +213,7 @@ DEV double messageWait(WideTeam& t, const ulonglong2* slot, ulonglong2 m, unsign
 /// The value of a message; `code` is the fault of a wait that gives up.
 DEV double messageWait(WideTeam& t, const ulonglong2* slot, unsigned tag, int code) {
   ulonglong2 m = messageLoad(slot);
-  long long polls = 0;
+  int polls = 0;
   while (!messageReady(m, tag)) {
     if (wideGiveUp(t, polls, code)) return 0.0;
     m = messageLoad(slot);
@@ -208,7 +229,7 @@ DEV void messageWaitAll(WideTeam& t, const ulonglong2* set, const int (&from)[N]
   unsigned missing = 0;
 #pragma unroll
   for (int k = 0; k < N; ++k) missing |= (from[k] >= 0) ? 1u << k : 0u;
-  long long polls = 0;
+  int polls = 0;
   while (missing != 0u) {
     ulonglong2 m[N];
 #pragma unroll
@@ -243,12 +264,12 @@ DEV void wideBarrier(WideTeam& t) {
   if (t.tid == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.mem.arrived) : "memory");
     const unsigned all = t.barriers * static_cast<unsigned>(t.R);
-    long long polls = 0;
+    int polls = 0;
     for (;;) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.mem.arrived) : "memory");
       if (static_cast<int>(v - all) >= 0) break;
-      if (wideGiveUp(t, polls, kFaultTeamWait)) break;
+      if (wideGiveUpFar(t, polls, kFaultTeamWait)) break;
     }
   }
   __syncthreads();

@@ -8,6 +8,7 @@
 //   tiles THREADS NJ NI0 NI1               blocks of NI0 .. NI1 columns with a column
 //                                          tile that holds no column, or more units
 //                                          than sums are kept of; the first of them
+//   sweeps NI                              shared memory of one k or omega sweep
 //   waits CAPACITY THREADS ITERATIONS CAP {NI NJ SST}...  of any CTA's longest wait
 //                                          for the solves before its own, as
 //                                          modelled, the permille of its limit
@@ -16,6 +17,7 @@
 #include <sstream>
 #include <string>
 
+#include "row_sweeps.cuh"
 #include "wide_cg.cuh"
 #include "wide_plan.hpp"
 
@@ -63,8 +65,9 @@ double waits(const WidePlan& plan, const std::vector<WideJob>& jobs, int threads
       const WideJob& job = jobs[static_cast<std::size_t>(plan.list[static_cast<std::size_t>(k)])];
       const int R = ctasOf(job, c.R, threads);
       const double outer = outerBound(job.NI, job.NJ, R, threads, wideEffort(false, 1, cap, 16, 3));
-      // a poll is 0.4 us at least
-      worst = std::max(worst, behind / (wideSpinLimit(outer + iterations * ahead) * 0.4e-3));
+      // a poll is 0.4 us at least, a unit of the limit 2^20 ns
+      const double limit = kWideSpinLimit * 0.4e-3 + wideWaitLimit(outer + iterations * ahead) * 1.048576;
+      worst = std::max(worst, behind / limit);
       behind += milliseconds(job, R, iterations, cap);
       ahead += outer;
     }
@@ -80,7 +83,11 @@ int main() {
     std::istringstream in(line);
     std::string what;
     in >> what;
-    if (what == "tiles") {
+    if (what == "sweeps") {
+      int NI = 0;
+      in >> NI;
+      std::printf("%d\n", rowSweepBytes(rowSweepShape(NI)));
+    } else if (what == "tiles") {
       int threads = 0, NJ = 0, first = 0, last = 0, bad = 0, where = 0;
       in >> threads >> NJ >> first >> last;
       for (int NI = first; NI <= last; ++NI) {
