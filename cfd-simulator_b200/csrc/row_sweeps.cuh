@@ -40,8 +40,10 @@ constexpr int kAhead = 3;       // rows whose old values are on their way
 
 struct RowSweepShape {
   int per, width, chunks, padded;  // cells per lane, columns per chunk, chunks, columns with padding
-  int edges;                       // rows whose chunk edges are kept
+  int edges;                       // rows whose chunk edges are kept on chip
 };
+/// Shared memory of one sweep at most: what a wide kernel has (kMaxWideSmem).
+constexpr int kMaxSweepBytes = 222032;
 __host__ __device__ inline RowSweepShape rowSweepShape(int NI) {
   RowSweepShape s;
   s.per = (NI + 255) / 256;
@@ -50,6 +52,9 @@ __host__ __device__ inline RowSweepShape rowSweepShape(int NI) {
   s.chunks = (NI + s.width - 1) / s.width;
   s.padded = s.chunks * s.width;
   s.edges = (s.chunks <= 16) ? 64 : 16;
+  // more than 816 chunks (104,448 columns): not on chip at all, a chunk's west
+  // value is then its west neighbour's message (rowSweep)
+  if (s.chunks > kMaxSweepBytes / (s.edges * 16 + 16)) s.edges = 0;
   return s;
 }
 /// Place of column i in a row of the packed layouts: lane-contiguous cells,
@@ -66,7 +71,9 @@ __host__ __device__ inline long long rowSweepMessages(int NI, int NJ) {
   return static_cast<long long>(kSweeps + 1) * rowSweepShape(NI).padded * NJ;
 }
 /// Shared memory of one sweep: the chunks' edges and progress.
-__host__ __device__ inline int rowSweepBytes(const RowSweepShape& s) { return s.chunks * (s.edges * 16 + 16); }
+__host__ __device__ inline int rowSweepBytes(const RowSweepShape& s) {
+  return (s.edges > 0) ? s.chunks * (s.edges * 16 + 16) : 0;
+}
 /// And with the coefficients of kSweepDepth rows of every chunk.
 __host__ __device__ inline int rowSweepRingBytes(const RowSweepShape& s) {
   return rowSweepBytes(s) + s.chunks * kSweepDepth * 5 * s.width * 8;
@@ -176,7 +183,8 @@ DEV void copyAsync16(double* to, const double* from) {
 /// Sweep s of one equation by the `warps` warps from this thread's slot on
 /// (warp `w` of them). kRing: a warp has one chunk, its coefficients arrive by
 /// asynchronous copies; else a warp has every warps-th chunk and loads as it goes.
-template <int PER, bool kRing>
+/// kOnChip: the chunks' edges are kept on chip (RowSweepShape::edges).
+template <int PER, bool kRing, bool kOnChip>
 __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, const RowSweepSystem& system, int s,
                                       unsigned tag, int w, int warps, char* smem) {
   WideTeam t = team;
@@ -207,11 +215,17 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
     return (exists && j < NJ) ? messageLoad(in + static_cast<long long>(j) * z.padded + place) : ulonglong2{0, 0};
   };
 
+  // Where no edges are kept, the value that enters a chunk's part of a row: its west
+  // neighbour's last message.
+  auto neighbour = [&](int chunk, int j) {
+    const ulonglong2* slot = out + static_cast<long long>(j) * z.padded + rowSweepPlace(z, chunk * z.width - 1);
+    return messageWait(t, slot, tag, kFaultChainWait);
+  };
   // What a row leaves: progress, its values, and at the last sweep the unknowns.
   auto finish = [&](int chunk, int j, unsigned exists, const double (&x)[PER]) {
     // every lane has the value from the west: its place may be used again
     __syncwarp();
-    if (lane == 0) progress[chunk] = j + 1;
+    if (kOnChip && lane == 0) progress[chunk] = j + 1;
     const long long at = static_cast<long long>(j) * z.padded + chunk * z.width + lane;
     const long long cell = static_cast<long long>(j) * NI + chunk * z.width + lane * PER;
 #pragma unroll
@@ -259,11 +273,16 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
       before = 0.0;
       scale = 1.0;
     }
-    volatile unsigned long long* mine = edges + (chunk * z.edges + j % z.edges) * 2;
-    const double x0 = (chunk > 0) ? edgeWait(t, mine - 2 * z.edges, static_cast<unsigned>(j) + 1u) : 0.0;
-    if (lane == 31 && chunk + 1 < z.chunks) {
-      if (j >= z.edges) edgeRoom(t, progress + chunk + 1, j - z.edges + 1);
-      edgeStore(mine, fma(Q, x0, P), static_cast<unsigned>(j) + 1u);  // the chunk's last value
+    double x0;
+    if constexpr (kOnChip) {
+      volatile unsigned long long* mine = edges + (chunk * z.edges + j % z.edges) * 2;
+      x0 = (chunk > 0) ? edgeWait(t, mine - 2 * z.edges, static_cast<unsigned>(j) + 1u) : 0.0;
+      if (lane == 31 && chunk + 1 < z.chunks) {
+        if (j >= z.edges) edgeRoom(t, progress + chunk + 1, j - z.edges + 1);
+        edgeStore(mine, fma(Q, x0, P), static_cast<unsigned>(j) + 1u);  // the chunk's last value
+      }
+    } else {
+      x0 = (chunk > 0) ? neighbour(chunk, j) : 0.0;
     }
     double v = fma(scale, x0, before);
     unsigned exists = 0;
@@ -288,7 +307,8 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
 #pragma unroll
     for (int e = 0; e < PER; ++e) exists |= (i0 + e < NI) ? 1u << e : 0u;
     volatile unsigned long long* mine = edges + chunk * z.edges * 2;
-    double x0 = (chunk > 0) ? edgeWait(t, mine - 2 * z.edges, 1u) : 0.0;
+    double x0 = 0.0;
+    if (chunk > 0) x0 = kOnChip ? edgeWait(t, mine - 2 * z.edges, 1u) : neighbour(chunk, 0);
     double last = 0.0;
     for (int part = 0; part < 2; ++part) {
       const int from = part ? half : 0, to = part ? NI : half;
@@ -320,7 +340,7 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
         }
       }
     }
-    if (lane == 31 && chunk + 1 < z.chunks) edgeStore(mine, last, 1u);
+    if (kOnChip && lane == 31 && chunk + 1 < z.chunks) edgeStore(mine, last, 1u);
 #pragma unroll
     for (int e = 0; e < PER; ++e) x[e] = ((exists >> e) & 1u) ? c.x[e] : 0.0;
     finish(chunk, 0, exists, x);
@@ -423,11 +443,15 @@ __device__ __noinline__ void rowSweep(const Instance& I, const WideTeam& team, c
 template <bool kRing>
 DEV void rowSweepAny(const Instance& I, const WideTeam& t, const RowSweepSystem& y, int s, unsigned tag, int w, int warps,
                      char* smem) {
-  switch (rowSweepShape(I.NI).per) {
-    case 1: rowSweep<1, kRing>(I, t, y, s, tag, w, warps, smem); break;
-    case 2: rowSweep<2, kRing>(I, t, y, s, tag, w, warps, smem); break;
-    case 3: rowSweep<3, kRing>(I, t, y, s, tag, w, warps, smem); break;
-    default: rowSweep<4, kRing>(I, t, y, s, tag, w, warps, smem); break;
+  const RowSweepShape z = rowSweepShape(I.NI);
+  switch (z.per) {
+    case 1: rowSweep<1, kRing, true>(I, t, y, s, tag, w, warps, smem); break;
+    case 2: rowSweep<2, kRing, true>(I, t, y, s, tag, w, warps, smem); break;
+    case 3: rowSweep<3, kRing, true>(I, t, y, s, tag, w, warps, smem); break;
+    default:
+      if (kRing || z.edges > 0) rowSweep<4, kRing, true>(I, t, y, s, tag, w, warps, smem);
+      else rowSweep<4, false, false>(I, t, y, s, tag, w, warps, smem);
+      break;
   }
 }
 

@@ -30,3 +30,17 @@ def test_first_iteration_matches_the_oracle(threads, grid, monkeypatch):
     s.iterate(1)
     for f, a in _fields(s).items():
         assert rel_err(a, o.read(FIELDS[f])) <= 1e-9, (f, rel_err(a, o.read(FIELDS[f])))
+
+
+@pytest.mark.parametrize("wake,normal", [(52170, 4), (52186, 4), (60000, 3)])
+def test_very_wide_blocks(wake, normal):
+    # 104,418 columns: a sweep's chunk edges just fit on chip; 104,450 and more: none
+    # are kept there
+    mesh = cb.cgrid("0012", surface_points=40, wake_points=wake, normal_points=normal, first_layer_height=1e-3)
+    o = port.OracleSolver(mesh, cb.freestream_conditions(mesh, 1.0, 3.0), _packed(), 2, port.DEVICE_ORDER)
+    o.initialise(*cb.uniform_field(mesh, 1.0, 3.0, 1.0, 1e6))
+    o.iterate(1)
+    s = _solver(mesh)
+    s.iterate(1)
+    for f, a in _fields(s).items():
+        assert rel_err(a, o.read(FIELDS[f])) <= 1e-9, (f, rel_err(a, o.read(FIELDS[f])))

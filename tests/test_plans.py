@@ -69,3 +69,9 @@ def test_every_column_tile_holds_columns(ask):
     queries = [f"tiles {threads} {nj} 1 5000" for threads in range(32, 513, 32) for nj in (1, 6, 48, 192, 400, 3000)]
     for query, (bad, where) in zip(queries, ask(queries)):
         assert bad == 0, (query, bad, where)
+
+
+def test_a_sweep_of_any_width_fits_on_chip(ask):
+    widths = list(range(1, 4000, 37)) + [104448, 104449, 104450, 130000, 355000, 10 ** 6, 10 ** 8]
+    for ni, (size,) in zip(widths, ask([f"sweeps {ni}" for ni in widths])):
+        assert 0 <= size <= 222032, (ni, size)
