@@ -378,7 +378,7 @@ struct WideCgScalars {
     } else {
       converged = final <= tolerance * initial;
       if (converged || !(fabs(gamma) > 0.0)) return false;
-      beta = sum0 * inverse;
+      beta = isfinite(inverse) ? sum0 * inverse : sum0 / gamma;  // below 5.6e-309 it has none
       dAd = fma(-beta * beta, dAd, sum1);
     }
     if (!(fabs(dAd) > 0.0) || iterations >= cap) return false;
