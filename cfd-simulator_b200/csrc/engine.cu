@@ -208,6 +208,8 @@ struct Engine {
   int statusSlots{0};
   Instance* dTable{nullptr};
   int tableSlots{0};
+  // the last plan of each form and thread count, and the solves it was made for
+  std::map<std::pair<bool, int>, std::pair<std::vector<WideJob>, WidePlan>> planned;
   char* dPlans{nullptr};  // the wide launches' plans
   std::size_t planBytes{0};
   std::vector<cudaStream_t> streams;
@@ -503,7 +505,12 @@ struct Engine {
         table[offset + static_cast<int>(m)] = I;
         jobs.push_back(s.solver->wideJob());
       }
-      Launch launch{shape.first, offset, shape.second, planWide(jobs, shape.second, wideCapacity()), plans.size()};
+      auto& [plannedJobs, plan] = planned[shape];
+      if (plan.ctas.empty() || !(plannedJobs == jobs)) {
+        plan = planWide(jobs, shape.second, wideCapacity());
+        plannedJobs = std::move(jobs);
+      }
+      Launch launch{shape.first, offset, shape.second, plan, plans.size()};
       const std::size_t ctas = launch.plan.ctas.size() * sizeof(WideCta);
       const std::size_t list = launch.plan.list.size() * sizeof(int);
       plans.resize(plans.size() + ((ctas + list + 15) & ~std::size_t{15}));

@@ -1385,6 +1385,7 @@ struct BatchGroup {
   int offset{0}, count{0};
   int threads{512};
   std::vector<int> members;  // indices into cfd_batch_t::handles
+  std::vector<cfdb::WideJob> jobs;  // what the plan was made for
   cfdb::WidePlan plan;
   cfdb::WideCta* dPlan{nullptr};
   int* dList{nullptr};
@@ -1421,8 +1422,10 @@ cfd_status refreshTable(cfd_batch b) {
   for (BatchGroup& g : b->groups) {
     std::vector<cfdb::WideJob> jobs;
     for (int k : g.members) jobs.push_back(b->handles[static_cast<std::size_t>(k)]->solver->wideJob());
+    if (!g.plan.ctas.empty() && jobs == g.jobs) continue;
     cfdb::WidePlan plan = cfdb::planWide(jobs, g.threads, cfdb::wideCapacity());
-    if (g.dList != nullptr && plan == g.plan) continue;
+    g.jobs = std::move(jobs);
+    if (plan == g.plan) continue;
     if (b->graph != nullptr) {
       cudaGraphExecDestroy(b->graph);
       b->graph = nullptr;

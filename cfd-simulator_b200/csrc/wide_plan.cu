@@ -3,8 +3,11 @@
 
 #include "wide_plan.hpp"
 
-#include <cstdlib>
+#include <functional>
+#include <map>
 #include <numeric>
+#include <queue>
+#include <utility>
 
 #include "common.hpp"
 #include "row_sweeps.cuh"
@@ -127,30 +130,63 @@ WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity) {
     return plan;
   }
   // teams of equal width, each with a list of solves: longest first to the
-  // team that is free first. The number of teams that finishes first wins; a
-  // solve's bits do not depend on it.
+  // team that is free first. The number of teams that finishes first wins (the
+  // fewest of equals); a solve's bits do not depend on it. A solve's cost follows
+  // from its kind and the width, and numbers of teams are tried in the order of
+  // what they take at least, so most are not tried at all: 512 coarse solves 0.3
+  // ms, 31 with every number tried and every solve priced for it.
   int least = 1;
-  for (const WideJob& job : jobs) {
-    if (job.mixedSmem == 0) least = std::max(least, wideLeastCtas(job.NI, job.NJ, threads));
+  std::vector<WideJob> kinds;
+  std::vector<int> kindOf(jobs.size()), members;
+  for (int k = 0; k < count; ++k) {
+    std::size_t kind = 0;
+    while (kind < kinds.size() && !(kinds[kind] == jobs[k])) ++kind;
+    if (kind == kinds.size()) {
+      kinds.push_back(jobs[k]);
+      members.push_back(0);
+      if (jobs[k].mixedSmem == 0) least = std::max(least, wideLeastCtas(jobs[k].NI, jobs[k].NJ, threads));
+    }
+    kindOf[k] = static_cast<int>(kind);
+    ++members[kind];
   }
+  std::map<int, std::vector<double>> priced;  // width -> cost of each kind
+  auto costs = [&](int width) -> const std::vector<double>& {
+    std::vector<double>& cost = priced[width];
+    if (cost.empty()) {
+      for (const WideJob& job : kinds) cost.push_back(outerMicroseconds(job, usefulCtas(job, width, threads)));
+    }
+    return cost;
+  };
+  std::vector<std::pair<double, int>> tries;  // what so many teams take at least
+  for (int teams = 1; teams <= std::min(count, capacity / least); ++teams) {
+    const std::vector<double>& cost = costs(capacity / teams);
+    double sum = 0.0;
+    for (std::size_t kind = 0; kind < kinds.size(); ++kind) sum += members[kind] * cost[kind];
+    // (less a little: sums of the same numbers in other orders)
+    tries.emplace_back(std::max(sum / teams * (1.0 - 1e-9), *std::max_element(cost.begin(), cost.end())), teams);
+  }
+  std::sort(tries.begin(), tries.end());
   double best = -1.0;
   int bestTeams = 1;
   std::vector<std::vector<int>> bestLists;
-  for (int teams = 1; teams <= std::min(count, capacity / least); ++teams) {
-    const int width = capacity / teams;
-    std::vector<double> cost(jobs.size()), load(static_cast<std::size_t>(teams), 0.0);
+  for (const auto& [atLeast, teams] : tries) {
+    if (best >= 0.0 && atLeast > best) break;
+    const std::vector<double>& cost = costs(capacity / teams);
     std::vector<int> order(jobs.size());
     std::iota(order.begin(), order.end(), 0);
-    for (int k = 0; k < count; ++k) cost[k] = outerMicroseconds(jobs[k], usefulCtas(jobs[k], width, threads));
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[kindOf[a]] > cost[kindOf[b]]; });
     std::vector<std::vector<int>> lists(static_cast<std::size_t>(teams));
+    std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> load;
+    for (int team = 0; team < teams; ++team) load.emplace(0.0, team);
+    double makespan = 0.0;
     for (int k : order) {
-      const std::size_t team = std::min_element(load.begin(), load.end()) - load.begin();
+      const auto [until, team] = load.top();
+      load.pop();
       lists[team].push_back(k);
-      load[team] += cost[k];
+      load.emplace(until + cost[kindOf[k]], team);
+      makespan = std::max(makespan, until + cost[kindOf[k]]);
     }
-    const double makespan = *std::max_element(load.begin(), load.end());
-    if (best < 0.0 || makespan < best) {
+    if (best < 0.0 || makespan < best || (makespan == best && teams < bestTeams)) {
       best = makespan;
       bestTeams = teams;
       bestLists = std::move(lists);

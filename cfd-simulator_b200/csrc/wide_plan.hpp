@@ -69,6 +69,9 @@ struct WideJob {
   int most;  // CTAs at most
   bool sst;
   int mixedSmem;  // mixed form: its dynamic shared memory; 0: plain form
+  bool operator==(const WideJob& o) const {
+    return NI == o.NI && NJ == o.NJ && most == o.most && sst == o.sst && mixedSmem == o.mixedSmem;
+  }
 };
 struct WidePlan {
   std::vector<WideCta> ctas;

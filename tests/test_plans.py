@@ -75,3 +75,13 @@ def test_a_sweep_of_any_width_fits_on_chip(ask):
     widths = list(range(1, 4000, 37)) + [104448, 104449, 104450, 130000, 355000, 10 ** 6, 10 ** 8]
     for ni, (size,) in zip(widths, ask([f"sweeps {ni}" for ni in widths])):
         assert 0 <= size <= 222032, (ni, size)
+
+
+def test_planning_many_solves_is_quick(ask):
+    # a plan is made between launches, with the GPU idle: 20 ms each with every number
+    # of teams tried and every solve priced for it, 0.5 ms now
+    import time
+    queries = [plan([(192, 48, 1)] * 512)] * 100
+    start = time.perf_counter()
+    assert all(ok == 1 for _, _, _, ok in ask(queries))
+    assert time.perf_counter() - start < 1.0
