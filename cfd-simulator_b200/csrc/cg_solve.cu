@@ -379,10 +379,15 @@ struct ThreadScratch {
 /// at least as many rows as the cluster form would use CTAs (a block of a few
 /// very long rows stays with the cluster form, which splits cells). Measured
 /// per iteration: 768x192 on 144 CTAs 3.6 us against 28 on a cluster of 16,
-/// 384x96 2.6 against 8, 192x48 2.2 against 5.5.
-int wideCtasFor(const CgView& V) {
-  const int capacity = wideCapacity();
+/// 384x96 2.6 against 8, 192x48 2.2 against 5.5. `together`: solves of other
+/// threads in flight, this one included (wideShare).
+int wideCtasFor(const CgView& V, int together) {
+  int capacity = wideCapacity();
   if (capacity < kMaxColumnTiles || V.NJ < chooseClusterSize(V.N)) return 0;
+  if (together > 1) {
+    const WideJob job{V.NI, V.NJ, wideMostCtas(V.NI, V.NJ, kWideThreads), false, 0};
+    capacity = wideShare(job, kWideThreads, together, capacity);
+  }
   return wideChooseCtas(V.NI, V.NJ, capacity);
 }
 WideScratchLayout wideLayoutFor(const CgView& V, int R) {
@@ -459,7 +464,8 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
   V.maxIt = max_iterations;
   V.tol = tolerance;
   char* scratch = nullptr;
-  if (const int R = cfdb::wideCtasFor(V); R > 0) {
+  const cfdb::WideFlight flight;
+  if (const int R = cfdb::wideCtasFor(V, flight.together()); R > 0) {
     // Scratch for this call: the messages, the report, u, and what the shared
     // memory does not hold.
     const cfdb::WideScratchLayout layout = cfdb::wideLayoutFor(V, R);
@@ -594,7 +600,7 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
   V.report = base + 9 * slot;
   // A wide team where everything else stays on chip and its messages fit in
   // the slots beside u: the array as the cluster form carves it is the limit.
-  if (int R = cfdb::wideCtasFor(V); R > 0) {
+  if (int R = cfdb::wideCtasFor(V, 1); R > 0) {
     const std::size_t room = 8 * slot * sizeof(double);
     while (R > 1 && cfdb::wideLayoutFor(V, R).bytes > room) --R;
     if (cfdb::wideLayoutFor(V, R).bytes <= room && R >= cfdb::wideCgShape(V.NI, V.NJ, R, cfdb::kWideThreads).columnTiles &&

@@ -860,11 +860,14 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
   if (n < 0) return fail(CFD_INVALID_ARGUMENT, "negative iteration count");
   if (history != nullptr) history->clear();
   int total = 0;
+  const WideFlight flight;
   while (total < n) {
-    const int chunk = std::min(n - total, historyCapacity_);
+    const int chunk = std::min(n - total, historyCapacity_), capacity = wideCapacity();
     const auto launch = (settings_.precision == 1) ? launchSimple : launchPlain;
-    const Status st = launch(dView_, planWide({wideJob()}, threads_, wideCapacity()), nullptr, nullptr, threads_, chunk,
-                             stopStage, tolerance, stream_);
+    WideJob job = wideJob();
+    if (const int together = flight.together(); together > 1) job.most = wideShare(job, threads_, together, capacity);
+    const Status st = launch(dView_, planWide({job}, threads_, capacity), nullptr, nullptr, threads_, chunk, stopStage,
+                             tolerance, stream_);
     if (st != CFD_OK) return st;
     CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
     int words[2] = {0, 0};

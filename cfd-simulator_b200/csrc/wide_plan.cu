@@ -3,6 +3,7 @@
 
 #include "wide_plan.hpp"
 
+#include <atomic>
 #include <functional>
 #include <map>
 #include <numeric>
@@ -206,6 +207,29 @@ WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity) {
     for (int r = 0; r < widest; ++r) plan.ctas.push_back(WideCta{begin, end, r, width});
   }
   return plan;
+}
+
+int wideShare(const WideJob& job, int threads, int together, int capacity) {
+  const std::vector<WideJob> all(static_cast<std::size_t>(std::min(std::max(together, 1), kMaxWideCtas)), job);
+  const WidePlan plan = planWide(all, threads, capacity);
+  return plan.ctas.empty() ? job.most : std::min(plan.ctas.front().R, job.most);
+}
+
+namespace {
+std::atomic<int> g_inFlight[64];
+}
+
+WideFlight::WideFlight() {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return;
+  device_ = device;
+  g_inFlight[device_].fetch_add(1, std::memory_order_relaxed);
+}
+WideFlight::~WideFlight() {
+  if (device_ >= 0) g_inFlight[device_].fetch_sub(1, std::memory_order_relaxed);
+}
+int WideFlight::together() const {
+  return (device_ >= 0) ? std::max(g_inFlight[device_].load(std::memory_order_relaxed), 1) : 1;
 }
 
 }  // namespace cfdb

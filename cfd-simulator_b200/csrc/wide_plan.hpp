@@ -90,4 +90,25 @@ struct WidePlan {
 /// one solve after another.
 WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity);
 
+/// CTAs of a launch of one solve beside `together - 1` others, from other host
+/// threads: as many as it would get in one launch with as many of its kind. A
+/// launch as wide as the GPU would make the others wait for all of it. Seven
+/// threads, each a lone SST solve, ms per solve and iteration: plain 384x96 0.94 as
+/// wide as it goes, 0.36 so, 768x192 1.67 and 0.82; mixed 0.42 and 0.21, 1.28 and 0.47.
+int wideShare(const WideJob& job, int threads, int together, int capacity);
+
+/// The launches of lone solves that this process has in flight on a device, this
+/// one included, while it lives.
+class WideFlight {
+ public:
+  WideFlight();
+  ~WideFlight();
+  WideFlight(const WideFlight&) = delete;
+  WideFlight& operator=(const WideFlight&) = delete;
+  int together() const;
+
+ private:
+  int device_{-1};
+};
+
 }  // namespace cfdb

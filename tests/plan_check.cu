@@ -9,6 +9,7 @@
 //                                          tile that holds no column, or more units
 //                                          than sums are kept of; the first of them
 //   sweeps NI                              shared memory of one k or omega sweep
+//   share CAPACITY THREADS TOGETHER NI NJ SST  CTAs of a lone launch beside others
 //   waits CAPACITY THREADS ITERATIONS CAP {NI NJ SST}...  of any CTA's longest wait
 //                                          for the solves before its own, as
 //                                          modelled, the permille of its limit
@@ -83,7 +84,13 @@ int main() {
     std::istringstream in(line);
     std::string what;
     in >> what;
-    if (what == "sweeps") {
+    if (what == "share") {
+      int capacity = 0, threads = 0, together = 0, NI = 0, NJ = 0, sst = 0;
+      in >> capacity >> threads >> together >> NI >> NJ >> sst;
+      const WideJob job{NI, NJ, wideMostCtas(NI, NJ, threads), sst != 0, 0};
+      const int share = wideShare(job, threads, together, capacity);
+      std::printf("%d %d %d\n", share, wideLeastCtas(NI, NJ, threads), ctasOf(job, share, threads));
+    } else if (what == "sweeps") {
       int NI = 0;
       in >> NI;
       std::printf("%d\n", rowSweepBytes(rowSweepShape(NI)));

@@ -85,3 +85,15 @@ def test_planning_many_solves_is_quick(ask):
     start = time.perf_counter()
     assert all(ok == 1 for _, _, _, ok in ask(queries))
     assert time.perf_counter() - start < 1.0
+
+
+def test_a_lone_launch_leaves_room_for_others(ask):
+    grids = [(192, 48), (384, 96), (768, 192), (234, 61), (1500, 60)]
+    queries = [f"share 148 512 {n} {ni} {nj} 1" for ni, nj in grids for n in (1, 2, 3, 7, 200)]
+    answers = ask(queries)
+    for query, (share, least, used) in zip(queries, answers):
+        assert least <= used <= share <= 148, query
+    for k, _ in enumerate(grids):
+        alone, two = answers[5 * k], answers[5 * k + 1]
+        assert alone[2] > 74 or two[2] == alone[2]  # narrower only if two do not fit
+        assert 2 * two[2] <= 148 or two[2] == alone[2]
