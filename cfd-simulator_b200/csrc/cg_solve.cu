@@ -511,10 +511,11 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
 // has reserved the whole device up front (a cudaMalloc outside that manager
 // fails or breaks its accounting), or a latency-critical loop that must not
 // block on the implicit device-wide synchronisation cudaFree performs.
-// cfd_cg_solve_noalloc serves them. Its scratch (both coefficient families,
-// the seven CG vectors, the wake map and the report) is one file-scope device
-// array of fixed size, so a call allocates nothing; the caller still provides
-// the system and x in its own device memory.
+// cfd_cg_solve_noalloc serves them. Its scratch (a team's messages and its u, or
+// for the cluster form both coefficient families, the seven CG vectors and the
+// wake map; the report) is one file-scope device array of fixed size, so a call
+// allocates nothing; the caller still provides the system and x in its own
+// device memory.
 //
 // Limits and sharing:
 //   * blocks of at most kNoAllocMaxNodes mesh nodes, (cells_i+1)*(cells_j+1)
@@ -522,12 +523,12 @@ cfd_status cfd_cg_solve(const cfd_cg_system* system, double* x, double tolerance
 //     refused with CFD_OUT_OF_RANGE. The array is 4.75 MiB, held by every GPU
 //     that loads this library until the process exits.
 //   * every call shares the one array per device and it keeps the last
-//     call's contents. Nothing in it needs clearing beforehand: each word a
-//     solve reads is written earlier in the same call (coefficients and wake
-//     map by the layout launch; the first residual, w and the zero p and s
-//     at the start of the solve; each later half of the double-buffered r, w
-//     and s in the iteration before it is read), and the error flag is
-//     cleared by the call itself. Calls whose work overlaps on the GPU (other
+//     call's contents. The caller need not clear it: a call clears the report
+//     and a team's messages itself, and each other word it reads it has
+//     written before (cluster form: coefficients and wake map by the layout
+//     launch; the first residual, w and the zero p and s at the start of the
+//     solve; each later half of the double-buffered r, w and s in the
+//     iteration before it is read). Calls whose work overlaps on the GPU (other
 //     host threads, or other streams of this one) race on the array and must
 //     be serialised by the caller.
 //   * the first call on each device resolves the array's device address with
@@ -600,10 +601,9 @@ cfd_status cfd_cg_solve_noalloc(const cfd_cg_system* system, double* x, double t
   V.report = base + 9 * slot;
   // A wide team where everything else stays on chip and its messages fit in
   // the slots beside u: the array as the cluster form carves it is the limit.
-  if (int R = cfdb::wideCtasFor(V, 1); R > 0) {
-    const std::size_t room = 8 * slot * sizeof(double);
-    while (R > 1 && cfdb::wideLayoutFor(V, R).bytes > room) --R;
-    if (cfdb::wideLayoutFor(V, R).bytes <= room && R >= cfdb::wideCgShape(V.NI, V.NJ, R, cfdb::kWideThreads).columnTiles &&
+  // (A block within the node limit needs 2.3 MB of messages at most, of 4.2.)
+  if (const int R = cfdb::wideCtasFor(V, 1); R > 0) {
+    if (cfdb::wideLayoutFor(V, R).bytes <= 8 * slot * sizeof(double) &&
         cfdb::wideCgSpill(V.NI, V.NJ, R, cfdb::kWideThreads, cfdb::kMaxWideSmem, true) == 0) {
       if (cfd_status st = cfdb::cgRunWide(system, V, R, reinterpret_cast<char*>(base), base + 8 * slot, nullptr, s);
           st != CFD_OK) {

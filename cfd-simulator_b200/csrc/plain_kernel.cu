@@ -14,7 +14,6 @@
 // Every sum is formed in an order that depends on the grid alone, so a solve
 // gives the same bits on any number of CTAs, alone or in a batch.
 
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -31,7 +31,6 @@
 // wake cut because cellsI is even on a C-grid, so partners across the cut have
 // opposite colours. It changes the iterate path but not the converged answer.
 
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>

@@ -218,7 +218,6 @@ struct WideCgTile {
   WideCgShape z;
   int ct, rt, unit0, units;
   int i0, width, j0, rows, stride;  // rows of `stride` doubles: a border column on either side
-  bool member;                      // the rest of the team only follows the sums
   bool splitWake;                   // the wake's partners may lie in another tile: border cells
   int topRows, leftCols, rightCols, sums, unitCount, set;  // offsets in a message set, its size
   int team, lt, q, g;               // this thread: its team, its place there, its first column and row group
@@ -228,12 +227,10 @@ struct WideCgTile {
     z = wideCgShape(t.NI, t.NJ, t.R, t.T);
     ct = t.rank % z.columnTiles;
     rt = t.rank / z.columnTiles;
-    member = rt < z.RT;
-    unit0 = member ? z.unitRows * rt / z.RT : 0;
-    units = member ? z.unitRows * (rt + 1) / z.RT - unit0 : 0;
+    unit0 = z.unitRows * rt / z.RT;
+    units = z.unitRows * (rt + 1) / z.RT - unit0;
     j0 = unit0 * z.B;
     rows = min((unit0 + units) * z.B, t.NJ) - j0;
-    if (!member) rows = 0;
     i0 = ct * z.width;
     width = min(z.width, t.NI - i0);
     stride = z.width + 2;
@@ -249,9 +246,9 @@ struct WideCgTile {
     lt = t.tid - team * teamThreads;
     q = lt % z.G;
     g = lt / z.G;
-    working = member && team < z.teams && g < z.groups && q < width;
+    working = team < z.teams && g < z.groups && q < width;
   }
-  DEV int border() const { return member ? 2 * width + 2 * rows : 0; }
+  DEV int border() const { return 2 * width + 2 * rows; }
   /// Border cell h: the row below (0 .. width), above, the column left, right.
   /// Its cell in the block or -1; its place among the tile's cells; the message
   /// that carries its w.
@@ -309,7 +306,7 @@ DEV bool wideCgLoadBorder(const WideTeam& t, const WideCgSystem& S, const Loader
 }
 template <typename Loader>
 DEV void wideCgLoadCoefficients(const WideTeam& t, const Loader& load, const WideCgTile& a, double* sN, double* sE) {
-  for (int m = t.tid; m < (a.rows + 1) * a.width && a.member; m += t.T) {
+  for (int m = t.tid; m < (a.rows + 1) * a.width; m += t.T) {
     const int lr = m / a.width, q = m - lr * a.width;
     sN[(lr + 1) * a.stride + q + 1] = load.north(a.i0 + q, a.j0 + lr);
   }
@@ -829,8 +826,11 @@ __device__ __noinline__ WideCgResult wideCgAnyTile(WideTeam& team, const WideCgS
 }
 
 /// The whole solve by every thread of the team, in the block's dynamic shared
-/// memory of `smemBytes`; on return x is written (no barrier after it). Needs
-/// at least as many CTAs as column tiles. `any`: the form for any shape.
+/// memory of `smemBytes`; on return x is written (no barrier after it). The team is
+/// whole rows of CTAs, one per column tile in each and no more rows than units (R is
+/// columnTiles * RT: wideUsefulCtas, wideChooseCtas). A CTA without a unit would
+/// publish nothing, so the others could overwrite the messages it waits for. `any`:
+/// the form for any shape.
 template <typename Loader>
 DEV WideCgResult wideCg(WideTeam& t, const WideCgSystem& S, const Loader& load, int smemBytes, bool any) {
   const WideCgShape z = wideCgShape(t.NI, t.NJ, t.R, t.T);

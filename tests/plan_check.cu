@@ -8,6 +8,8 @@
 //   tiles THREADS NJ NI0 NI1               blocks of NI0 .. NI1 columns with a column
 //                                          tile that holds no column, or more units
 //                                          than sums are kept of; the first of them
+//   whole CAPACITY THREADS NI NJ           1 if every team such a block can get is
+//                                          whole rows of CTAs with a unit each
 //   sweeps NI                              shared memory of one k or omega sweep
 //   share CAPACITY THREADS TOGETHER NI NJ SST  CTAs of a lone launch beside others
 //   waits CAPACITY THREADS ITERATIONS CAP {NI NJ SST}...  of any CTA's longest wait
@@ -84,7 +86,21 @@ int main() {
     std::istringstream in(line);
     std::string what;
     in >> what;
-    if (what == "share") {
+    if (what == "whole") {
+      int capacity = 0, threads = 0, NI = 0, NJ = 0;
+      in >> capacity >> threads >> NI >> NJ;
+      auto whole = [&](int R, int T) {
+        const WideCgShape s = wideCgShape(NI, NJ, R, T);
+        return s.RT >= 1 && R == s.columnTiles * s.RT;
+      };
+      bool ok = capacity < wideLeastCtas(NI, NJ, kWideThreads) ||
+                whole(wideChooseCtas(NI, NJ, capacity), kWideThreads);
+      const int most = wideMostCtas(NI, NJ, threads);
+      for (int width = wideLeastCtas(NI, NJ, threads); width <= capacity; ++width) {
+        ok = ok && whole(wideUsefulCtas(NI, NJ, std::min(width, most), threads), threads);
+      }
+      std::printf("%d\n", ok ? 1 : 0);
+    } else if (what == "share") {
       int capacity = 0, threads = 0, together = 0, NI = 0, NJ = 0, sst = 0;
       in >> capacity >> threads >> together >> NI >> NJ >> sst;
       const WideJob job{NI, NJ, wideMostCtas(NI, NJ, threads), sst != 0, 0};

@@ -97,3 +97,11 @@ def test_a_lone_launch_leaves_room_for_others(ask):
         alone, two = answers[5 * k], answers[5 * k + 1]
         assert alone[2] > 74 or two[2] == alone[2]  # narrower only if two do not fit
         assert 2 * two[2] <= 148 or two[2] == alone[2]
+
+
+def test_every_team_is_whole_rows_of_ctas(ask):
+    rng = random.Random(11)
+    queries = [f"whole {rng.randint(1, 148)} {rng.choice([32, 64, 128, 256, 512])} {rng.randint(1, 3000)} "
+               f"{rng.randint(1, 1500)}" for _ in range(3000)]
+    for query, (ok,) in zip(queries, ask(queries)):
+        assert ok == 1, query
