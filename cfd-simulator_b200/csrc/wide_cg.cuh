@@ -351,7 +351,9 @@ DEV void sumsCollect(WideTeam& t, const WideCgTile& a, const ulonglong2* set, un
 /// The CG's scalars. step() takes the sums of an exchange: the reference's stop
 /// tests, then the next alpha and beta; false when the solve is over.
 struct WideCgScalars {
-  double gamma{0.0}, dAd{0.0}, alpha{0.0}, beta{0.0}, inverse{0.0};
+  double gamma{0.0}, dAd{0.0}, alpha{0.0}, beta{0.0};
+  double inverse{0.0};  // 1 / gamma, of a subnormal gamma 1 / (2^600 gamma)
+  bool tiny{false};     // it is subnormal
   double initial{0.0}, final{0.0};
   int iterations{-1};  // updates done; -1 before the first exchange
   bool converged{false};
@@ -375,13 +377,15 @@ struct WideCgScalars {
     } else {
       converged = final <= tolerance * initial;
       if (converged || !(fabs(gamma) > 0.0)) return false;
-      beta = isfinite(inverse) ? sum0 * inverse : sum0 / gamma;  // below 5.6e-309 it has none
+      beta = sum0 * inverse;
+      if (tiny) beta *= 0x1p600;
       dAd = fma(-beta * beta, dAd, sum1);
     }
     if (!(fabs(dAd) > 0.0) || iterations >= cap) return false;
     gamma = sum0;
     alpha = gamma / dAd;
-    inverse = 1.0 / gamma;
+    tiny = fabs(gamma) < 0x1p-1022;
+    inverse = 1.0 / (tiny ? gamma * 0x1p600 : gamma);
     ++iterations;
     return true;
   }
