@@ -1,4 +1,4 @@
-"""The plain form on blocks of fewer than 512 threads: column counts that leave
+"""The plain form at the edges of its tiling, mostly on fewer than 512 threads: column counts that leave
 fewer tiles than asked for at the width they get, and ordinary grids with threads
 that do or do not fill a unit of the CG.
 
@@ -16,7 +16,8 @@ pytestmark = pytest.mark.gpu
 
 # threads, (surface, wake, normal): 2 * (surface + wake) - 2 columns
 CASES = [(32, (900, 126, 7)), (64, (1300, 238, 7)), (128, (1300, 238, 12)), (32, (20, 8, 6)), (96, (70, 30, 60)),
-         (160, (100, 29, 40)), (256, (200, 58, 30)), (288, (70, 30, 60))]
+         (160, (100, 29, 40)), (256, (200, 58, 30)), (288, (70, 30, 60)),
+         (512, (800, 227, 41))]  # 17 chunks and 40 rows: a sweep's kept edges are used again
 
 
 @pytest.mark.parametrize("threads,grid", CASES)
