@@ -522,10 +522,6 @@ struct Engine {
     if (cudaMemcpy(dTable, table.data(), n * sizeof(Instance), cudaMemcpyHostToDevice) != cudaSuccess) {
       return fail(CFD_INITIALIZATION_FAILURE, "engine table upload failed");
     }
-    // monitors, counts and fault words of the chunk
-    if (cudaMemset(dStatus, 0, n * per * sizeof(double)) != cudaSuccess) {
-      return fail(CFD_INITIALIZATION_FAILURE, "engine status reset failed");
-    }
     if (plans.size() > planBytes) {
       if (dPlans) cudaFree(dPlans);
       planBytes = 2 * plans.size();
@@ -544,6 +540,11 @@ struct Engine {
         return fail(CFD_INITIALIZATION_FAILURE, "engine stream creation failed");
       }
       streams.push_back(s);
+    }
+    // monitors, counts and fault words of the chunk, before any of its launches
+    if (!launches.empty() && (cudaMemsetAsync(dStatus, 0, n * per * sizeof(double), streams[0]) != cudaSuccess ||
+                              cudaStreamSynchronize(streams[0]) != cudaSuccess)) {
+      return fail(CFD_INITIALIZATION_FAILURE, "engine status reset failed");
     }
     inFlightStreams.clear();
     for (std::size_t g = 0; g < launches.size(); ++g) {

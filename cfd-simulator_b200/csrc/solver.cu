@@ -754,7 +754,8 @@ Status Solver::initialise(const double* u, const double* v, const double* p, con
     }
   }
   // a fault of an earlier launch that nobody has read goes with its values
-  CUDA_OR_FAIL(cudaMemset(dIterations_ + 1, 0, sizeof(int)));
+  CUDA_OR_FAIL(cudaMemsetAsync(dIterations_ + 1, 0, sizeof(int), stream_));
+  CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
   initialised_ = true;
   if (model_ == 2) {
     if ((st = sstInitialise()) != CFD_OK) return st;
@@ -875,7 +876,7 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
     int words[2] = {0, 0};
     CUDA_OR_FAIL(cudaMemcpy(words, dIterations_, sizeof(words), cudaMemcpyDeviceToHost));
     if (words[1] != 0) {
-      CUDA_OR_FAIL(cudaMemset(dIterations_ + 1, 0, sizeof(int)));
+      CUDA_OR_FAIL(cudaMemsetAsync(dIterations_ + 1, 0, sizeof(int), stream_));
       return launchFault(words[1]);
     }
     const int ran = words[0];
@@ -1603,11 +1604,14 @@ cfd_status cfd_batch_monitors(cfd_batch b, int* taken, cfd_monitor* last) {
   for (std::size_t k = 0; k < b->handles.size(); ++k) {
     int* const source = b->handles[k]->solver->deviceView().iterations;
     e = cudaMemcpy(words[k].data(), source, sizeof(words[k]), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && words[k][1] != 0) e = cudaMemset(source + 1, 0, sizeof(int));
+    if (e == cudaSuccess && words[k][1] != 0) e = cudaMemsetAsync(source + 1, 0, sizeof(int), b->stream);
     if (e != cudaSuccess) return cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
     fault |= words[k][1];
   }
-  if (fault != 0) return cfdb::launchFault(fault);
+  if (fault != 0) {
+    e = cudaStreamSynchronize(b->stream);
+    return (e == cudaSuccess) ? cfdb::launchFault(fault) : cfdb::fail(CFD_INITIALIZATION_FAILURE, cudaGetErrorString(e));
+  }
   for (std::size_t k = 0; k < b->handles.size(); ++k) {
     const cfdb::Instance& I = b->handles[k]->solver->deviceView();
     const int ran = words[k][0];
