@@ -358,13 +358,11 @@ Status Solver::build(const cfd_mesh_desc& m, const cfd_face_bc& bc) {
       I.tkC = a.take<float4>(words);
       I.twC = a.take<float4>(words);
     } else {
+      double** vectors[] = {&I.z, &I.q, &I.d0, &I.d1};
+      for (double** ptr : vectors) *ptr = a.take<double>(N);
       const std::size_t packed = static_cast<std::size_t>(rowSweepCoefficients(NI_, NJ_));
       const std::size_t values = static_cast<std::size_t>(rowSweepMessages(NI_, NJ_));
       I.kC = a.take<double>(packed); I.wC = a.take<double>(packed);
-      // the two-reduction CG's vectors (kFlagTwoReductionCg) lie where the sweeps'
-      // coefficients, 5 a cell, are not yet
-      double** vectors[] = {&I.z, &I.q, &I.d0, &I.d1};
-      for (std::size_t k = 0; k < 4; ++k) *vectors[k] = (I.kC != nullptr) ? I.kC + k * N : nullptr;
       I.kV = a.take<ulonglong2>(values); I.wV = a.take<ulonglong2>(values);
       const std::size_t spill =
           static_cast<std::size_t>(wideSpillDoubles(NI_, NJ_, I.wideMost, threads_));
