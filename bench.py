@@ -191,7 +191,7 @@ def measured_peak() -> tuple[float, str]:
 
 
 def committed_traffic(name: str) -> float | None:
-    """DRAM bytes per launch of simpleKernel on a workload, from a committed
+    """DRAM bytes per launch of the form's kernel on a workload, from a committed
     ncu summary (its `traffic_bytes_per_launch:` line)."""
     path = os.path.join(ROOT, "profiles", name)
     try:
@@ -399,7 +399,7 @@ def _roofline(solvers, cg, step_ms, mixed, profile):
     achieved = per_launch / (float(np.mean(step_ms)) / 1e3) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
-            "traffic": committed_traffic(profile), "kernel": "simpleKernel",
+            "traffic": committed_traffic(profile), "kernel": "simpleKernel" if mixed else "plainKernel",
             "bytes_per_launch_algorithmic": per_launch,
             "mean_cg_iterations": float(np.average(cg, weights=[s.mesh.cells for s in solvers]))}
 
@@ -478,7 +478,7 @@ def run_ours(args) -> None:
 
     if rank == 0:
         profile = ("simple_kernel_c2_sst_mixed.md" if mixed_only else "simple_kernel_c2_sst_fp64.md") if c2 \
-            else ("simple_kernel_polar_mixed.md" if mixed_only else "simple_kernel_polar_fp64.md")
+            else ("simple_kernel_polar_mixed.md" if mixed_only else "plain_kernel_polar.md")
         roofline = _roofline(solvers, cg, step_ms, mixed_only, profile)
         config = c2_config() if c2 else polar_config({"solves": len(solvers), "cells": cells})
         if not c2 and args.solves is not None:
