@@ -378,8 +378,8 @@ struct ThreadScratch {
 /// Whether a wide team takes the block: it splits rows over CTAs, so it needs
 /// at least as many rows as the cluster form would use CTAs (a block of a few
 /// very long rows stays with the cluster form, which splits cells). Measured
-/// per iteration: 768x192 on 144 CTAs 3.6 us against 28 on a cluster of 16,
-/// 384x96 2.6 against 8, 192x48 2.2 against 5.5. `together`: solves of other
+/// per iteration: 768x192 on 144 CTAs 4.6 us against 28 on a cluster of 16,
+/// 384x96 on 96 3.8 against 8, 192x48 on 24 2.9 against 5.5. `together`: solves of other
 /// threads in flight, this one included (wideShare).
 int wideCtasFor(const CgView& V, int together) {
   int capacity = wideCapacity();

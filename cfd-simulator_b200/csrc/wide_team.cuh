@@ -6,7 +6,8 @@
 // in one GPC, so a lone 768x192 solve keeps 132 of the 148 SMs idle and its
 // state (1.2 MB per array) in L2. Spread over ~100 SMs the state of the
 // pressure CG fits on chip, and what a step costs is one exchange through L2
-// (~1.3 us) instead of the streaming of 900 KB per SM.
+// (an iteration of the CG takes 4.6 us, of which a round trip is under 1) instead
+// of the streaming of 900 KB per SM.
 //
 // Messages are tagged: every double travels as two 64-bit words, each half of
 // it beside a 32-bit tag, so a reader that sees the tag in both words has the
@@ -16,9 +17,9 @@
 // between launches, so a stale message never carries the tag waited for.
 //
 // Every CTA of a team must be resident: the launch is cooperative, one CTA
-// per SM. All waits are bounded (kWideSpinLimit polls): one that gives up sets
-// a code in the launch's fault word, after which the CTA waits no more, so a
-// launch always ends and the host reports it.
+// per SM. All waits are bounded (kWideSpinLimit polls, then wideWaitLimit): one
+// that gives up sets a code in the solve's fault word, after which the CTA waits no
+// more, so a launch always ends and the host reports it.
 //
 // Sums are formed per chunk of 256 consecutive cells and the chunks' sums in one
 // fixed order, so their bits do not depend on how many CTAs share the cells.
@@ -50,9 +51,9 @@ __host__ __device__ inline WideEffort wideEffort(bool mixed, int corrections, in
   return WideEffort{mixed ? 0.0 : passes * (cgMax + 1.0), mixed ? passes * (mgCap + 3.0) : 0.0, sweeps};
 }
 /// Microseconds that one outer iteration of a solve takes at most on R CTAs of T
-/// threads, per cell of a thread where it streams. Measured at 768x192: a CG
-/// exchange 5.9 us on 148 CTAs (2 cells a thread), 12 on 37, 30 on 24 and 88 on 12
-/// (24 cells), bounded by 5 + 5 a cell; a V-cycle 38 us, by 200 + 20; the rows of
+/// threads, per cell of a thread where it streams. Measured at 768x192: an iteration
+/// of the CG 4.6 us on 144 CTAs (2 cells a thread), in a full GPU 12 on 36, 30 on 24
+/// and 88 on 12 (24 cells), bounded by 5 + 5 a cell; a V-cycle 38 us, by 200 + 20; the rows of
 /// the sweeps 1.1 to 3.5 us each, by 5 + 5 a cell of the row for each of the six.
 __host__ __device__ inline double outerBound(int NI, int NJ, int R, int T, const WideEffort& e) {
   const double cells = static_cast<double>(NI) * NJ / (static_cast<double>(R) * T) + 1.0;

@@ -157,7 +157,10 @@ cfd_status cfd_gpu_initialise(cfd_handle h, const double* u, const double* v, co
 
 /* n x SimpleSolver::iterate() (SimpleSolver.cpp:662-794) in one device launch.
  * last (may be NULL) gets the final iteration's monitor, history (may be
- * NULL) n monitors. Returns after the device has finished. */
+ * NULL) n monitors. Returns after the device has finished. The launch is as wide
+ * as the grid can use, up to the whole GPU; while other host threads have solves in
+ * flight it takes a share, so that they run side by side (the same bits). Any other
+ * kernel that holds an SM can delay it: all its CTAs start together. */
 cfd_status cfd_gpu_iterate(cfd_handle h, int n, cfd_monitor* last, cfd_monitor* history);
 
 /* Iterate until worst() of the residuals < tol (SolverWorker.cpp:182-185),
@@ -416,8 +419,9 @@ cfd_status cfd_batch_graph_launch(cfd_batch b, int n, void* stream);
 /* Monitors of the last launch (count entries); synchronises first. Fails with
  * CFD_INTERNAL when a wait inside any launch since the last call gave up. */
 cfd_status cfd_batch_monitors(cfd_batch b, int* taken, cfd_monitor* last);
-/* CTAs reported per solve and threads per CTA of the batch's largest
- * group of solves. */
+/* The CTAs per solve and threads per CTA that most solves of the batch report
+ * (a rule of their grids: cfd_engine_set_shape_policy; what a launch gives a solve
+ * is its plan's). */
 cfd_status cfd_batch_shape(cfd_batch b, int* cluster_size, int* threads);
 cfd_status cfd_batch_destroy(cfd_batch b);
 
