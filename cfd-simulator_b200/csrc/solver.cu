@@ -875,6 +875,7 @@ Status Solver::iterate(int n, int stopStage, double tolerance, std::vector<doubl
     CUDA_OR_FAIL(cudaMemcpy(words, dIterations_, sizeof(words), cudaMemcpyDeviceToHost));
     if (words[1] != 0) {
       CUDA_OR_FAIL(cudaMemsetAsync(dIterations_ + 1, 0, sizeof(int), stream_));
+      CUDA_OR_FAIL(cudaStreamSynchronize(stream_));
       return launchFault(words[1]);
     }
     const int ran = words[0];
