@@ -134,8 +134,8 @@ WidePlan planWide(const std::vector<WideJob>& jobs, int threads, int capacity) {
   // team that is free first. The number of teams that finishes first wins (the
   // fewest of equals); a solve's bits do not depend on it. A solve's cost follows
   // from its kind and the width, and numbers of teams are tried in the order of
-  // what they take at least, so most are not tried at all: 512 coarse solves 0.3
-  // ms, 31 with every number tried and every solve priced for it.
+  // what they take at least, so most are not tried at all: 512 coarse solves 0.5
+  // ms, 20 with every number tried and every solve priced for it.
   int least = 1;
   std::vector<WideJob> kinds;
   std::vector<int> kindOf(jobs.size()), members;
